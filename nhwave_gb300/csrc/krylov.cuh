@@ -302,8 +302,12 @@ __global__ void __launch_bounds__(256) k_bicg_init(Dev<T> S) {
       const T r = S.kr0[t];
       S.kr[t] = r;
       S.kx[t] = (T)0;
-      S.kp[t] = (T)0;
-      S.kv[t] = (T)0;
+      if (S.kq) {
+        S.kq[t] = (T)0;
+      } else {
+        S.kp[t] = (T)0;
+        S.kv[t] = (T)0;
+      }
       v[0] += (A)r * (A)r;
     }
   }
@@ -511,6 +515,7 @@ __global__ void __launch_bounds__(256) k_bicg_xr(Dev<T> S) {
       x[t] = x[t] + alpha * ph[t] + omega * sh[t];
       const T r = ss[t] - omega * tt[t];
       rr[t] = r;
+      if (S.kq) S.kq[t] = S.kp[t] - omega * S.kv[t];   // for the next p, which the smoother forms
       v[0] += (A)r0[t] * (A)r;
       v[1] += (A)r * (A)r;
     }

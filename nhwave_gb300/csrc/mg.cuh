@@ -39,6 +39,7 @@ struct MGL {
   // sp + (2 s + c) * K * N * Mh, Mh = (M + 1) / 2, and holds level k, row jj,
   // column ii of that colour at k * N * Mh + jj * Mh + ii / 2.
   const T* sp;
+  T* xp;                // colour 0 of x between the two halves of a V-cycle (mg_tile.cuh)
 };
 
 template <class T>
@@ -191,8 +192,8 @@ __device__ __forceinline__ T off_column_p(const MGL<T>& L, const T* __restrict__
 //
 // Right-hand sides of a half-sweep:
 //   MgB            b as stored;
-//   MgInP / MgInS  the BiCGSTAB vectors p = r + beta (p - omega v) and
-//                  s = r - alpha v, formed on the fine level by the sweep that
+//   MgInP / MgInS  the BiCGSTAB vectors p = r + beta q (q = p - omega v, from
+//                  k_bicg_xr) and s = r - alpha v, formed on the fine level by the sweep that
 //                  owns each column (colour 0 in the first half-sweep, colour 1
 //                  in the second) and stored -- no launch of their own.
 //
@@ -210,16 +211,15 @@ template <class T>
 struct MgInP {
   T* p;
   const T* r;
-  const T* v;
-  T beta = (T)0, omega = (T)0;   // set by bind
+  const T* q;
+  T beta = (T)0;   // set by bind
   __device__ __forceinline__ MgInP bind(const DevScal* sc) const {
-    MgInP q = *this;
-    q.beta = (T)sc->beta;
-    q.omega = (T)sc->omega;
-    return q;
+    MgInP u = *this;
+    u.beta = (T)sc->beta;
+    return u;
   }
   __device__ __forceinline__ T operator()(const DevScal*, int ic, int, int, int) const {
-    const T val = r[ic] + beta * (p[ic] - omega * v[ic]);
+    const T val = r[ic] + beta * q[ic];
     p[ic] = val;
     return val;
   }
@@ -604,7 +604,8 @@ __device__ void cta_half_sweep(const MGL<T>& L, int color, int zero_x, const Pro
 
 template <class T>
 __device__ void cta_restrict(const MGL<T>& F, const MGL<T>& C) {
-  for (int ic = threadIdx.x; ic < C.n; ic += blockDim.x) {
+  const int nt = blockDim.x * blockDim.y;
+  for (int ic = threadIdx.x + blockDim.x * threadIdx.y; ic < C.n; ic += nt) {
     int I, J, k;
     decode(ic, C.M, C.N, I, J, k);
     T acc = (T)0;
@@ -794,14 +795,13 @@ __global__ void __launch_bounds__(256) k_mg_factor(MGL<T> L, T* lcp, T* linv) {
   }
 }
 
-// p = r + beta (p - omega v)   /   s = r - alpha v   (cell kernels when MG preconditions)
+// p = r + beta q   /   s = r - alpha v   (cell kernels when MG preconditions)
 template <class T>
 __global__ void __launch_bounds__(256) k_bicg_p_cell(Dev<T> S) {
   if (S.sc->conv) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S.neq) return;
-  const T beta = (T)S.sc->beta, omega = (T)S.sc->omega;
-  S.kp[t] = S.kr[t] + beta * (S.kp[t] - omega * S.kv[t]);
+  S.kp[t] = S.kr[t] + (T)S.sc->beta * S.kq[t];
 }
 template <class T>
 __global__ void __launch_bounds__(256) k_bicg_s_cell(Dev<T> S) {

@@ -28,7 +28,7 @@
 // partials in the same fixed order -- every block gets bit-identical totals
 // and takes identical decisions, with no second barrier.
 #pragma once
-#include "mg.cuh"
+#include "mg_tile.cuh"
 
 namespace nhw {
 

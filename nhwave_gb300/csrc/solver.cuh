@@ -386,7 +386,11 @@ class Solver final : public SolverBase {
       }
     }
     std::vector<T**> mgptr;
-    if (use_mg) add(&S.sp0, sizeof(T) * 7 * 2 * (size_t)K * N * ((M + 1) / 2));
+    if (use_mg) {
+      add(&S.sp0, sizeof(T) * 7 * 2 * (size_t)K * N * ((M + 1) / 2));
+      add(&S.kq, sizeof(T) * neq);
+      add(&mg[0].xp, sizeof(T) * neq);
+    }
     if (kFP32 && !p.hllc)   // 2-D face states (scratch of one stage)
       for (T** ft : {&S.fxT, &S.fyT}) add(ft, sizeof(T) * 6 * n2);
     for (size_t l = 1; l < mg.size(); ++l) {
@@ -397,6 +401,7 @@ class Solver final : public SolverBase {
       add((T**)&mg[l].lcp, sizeof(T) * nl);
       add((T**)&mg[l].linv, sizeof(T) * nl);
       add(&mg[l].x, sizeof(T) * nl);
+      add(&mg[l].xp, sizeof(T) * nl);
       add(&mg[l].b, sizeof(T) * nl);
     }
     // persistent solve: every block resident (cooperative launch), at most
@@ -476,6 +481,22 @@ class Solver final : public SolverBase {
         NHW_CU(cudaFuncSetAttribute(k_mg_smooth_split_strided<T, false, MgInV<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
       }
       NHW_CU(cudaFuncSetAttribute(k_mg_smooth_blk<T, false, MgInV<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
+    }
+    {
+      const int shm = (int)tile_smem<TileS, T>(KMAX);
+      const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+      NHW_CU(cudaFuncSetAttribute(k_mg_down<T, true, TileS, 1, TileInP<T>>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_down<T, true, TileS, 1, TileInS<T>>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_down<T, false, TileS, 1, TileB<T>>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_up<T, true, TileS, 1>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_up<T, false, TileS, 1>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_down<T, true, TileS, 2, TileInP<T>>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_down<T, true, TileS, 2, TileInS<T>>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_down<T, false, TileS, 2, TileB<T>>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_up<T, true, TileS, 2>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_up<T, false, TileS, 2>, at, shm));
+      NHW_CU(cudaFuncSetAttribute(k_mg_cycle<T, 1>, at, (int)cycle_smem<T>(KMAX)));
+      NHW_CU(cudaFuncSetAttribute(k_mg_cycle<T, 2>, at, (int)cycle_smem<T>(KMAX)));
     }
     NHW_CU(cudaFuncSetAttribute(k_mg_cta_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(sizeof(T) * 4 * 32 * 64)));
@@ -1171,6 +1192,60 @@ class Solver final : public SolverBase {
         k_mg_smooth_blk<T, false, In><<<cdiv(nthr, 32), dim3(32, by), shm, st>>>(Lv, S.sc, color, zero_x, P, in);
     });
   }
+  // Levels whose half of the V-cycle runs as one launch of small tiles
+  // (mg_tile.cuh).  Up to 4096 columns a tile launch takes less time than the
+  // passes one by one, although it solves the tiles' borders more than once
+  // (GB300, one level of 20 sigma levels, down / up in us): FP32 64 x 8
+  // 9.3 / 8.3 -> 5.1 / 4.8, 128 x 32 10.5 / 8.8 -> 7.1 / 7.3, but 256 x 32
+  // 10.3 / 8.8 -> 12.4 / 13.2; FP64 64 x 8 15.6 / 34 -> 12.6 / 15.0, 128 x 32
+  // 16.3 / 34 -> 19.6 / 24.3.  Aggregates must fill whole tiles.
+  static bool tiled(const MGL<T>& Lv) {
+    auto pow2 = [](int r) { return r == 1 || r == 2 || r == 4; };
+    return (long long)Lv.M * Lv.N <= 4096 && pow2(Lv.rx) && pow2(Lv.ry);
+  }
+  // Levels a thread: two where one each would not fit a block, or where the
+  // blocks (2 threads a cell) are more than the 152 SMs hold at 64 registers
+  // a thread (FP32 128 x 32 x 20: 9.5 / 9.1 -> 7.1 / 7.3 us; 64 x 64 x 10
+  // 4.8 / 4.6 with one, 5.0 / 5.4 with two)
+  static int tile_lpt(const MGL<T>& Lv) { return Lv.K > 32 || 2LL * Lv.n > 152 * 1024 ? 2 : 1; }
+  template <bool kFine, class In>
+  void down(int l, In in) {
+    static const char* names[] = {"mg_down_l0", "mg_down_l1", "mg_down_l2", "mg_down_l3",
+                                  "mg_down_l4", "mg_down_l5", "mg_down_l6", "mg_down_l7+"};
+    const MGL<T> f = mg[l], c = mg[l + 1];
+    const int nx = (int)cdiv(f.M, TileS::TX);
+    const unsigned nb = (unsigned)nx * cdiv(f.N, TileS::TY);
+    L(names[l < 7 ? l : 7], [&] {
+      if (tile_lpt(f) == 1)
+        k_mg_down<T, kFine, TileS, 1, In><<<nb, dim3(32, f.K), tile_smem<TileS, T>(f.K), st>>>(f, c, nx, S.sc, in);
+      else
+        k_mg_down<T, kFine, TileS, 2, In>
+            <<<nb, dim3(32, (f.K + 1) / 2), tile_smem<TileS, T>(f.K), st>>>(f, c, nx, S.sc, in);
+    });
+  }
+  template <bool kFine>
+  void up(int l, const Prolong<T>& pr) {
+    static const char* names[] = {"mg_up_l0", "mg_up_l1", "mg_up_l2", "mg_up_l3",
+                                  "mg_up_l4", "mg_up_l5", "mg_up_l6", "mg_up_l7+"};
+    const MGL<T> f = mg[l];
+    const int nx = (int)cdiv(f.M, TileS::TX);
+    const unsigned nb = (unsigned)nx * cdiv(f.N, TileS::TY);
+    L(names[l < 7 ? l : 7], [&] {
+      if (tile_lpt(f) == 1)
+        k_mg_up<T, kFine, TileS, 1><<<nb, dim3(32, f.K), tile_smem<TileS, T>(f.K), st>>>(f, pr, nx, S.sc);
+      else
+        k_mg_up<T, kFine, TileS, 2>
+            <<<nb, dim3(32, (f.K + 1) / 2), tile_smem<TileS, T>(f.K), st>>>(f, pr, nx, S.sc);
+    });
+  }
+  // the levels from `lc` on in one block
+  template <int LPT>
+  void cycle(const MGSet<T>& set, int cnt) {
+    L("mg_coarse_cycle", [&] {
+      k_mg_cycle<T, LPT><<<1, dim3(kCycleSlots, (S.K + LPT - 1) / LPT), cycle_smem<T>(S.K), st>>>(
+          set, cnt, S.sc, mg_w, mg_coarse_sweeps);
+    });
+  }
   // fine_in: 0 b as given; 1 b = p formed on the fly; 2 b = s formed on the fly
   void vcycle(T* b, T* x, int fine_in) {
     mg[0].b = b;
@@ -1188,9 +1263,15 @@ class Solver final : public SolverBase {
     static const char* rnames[] = {"mg_restrict_l0", "mg_restrict_l1", "mg_restrict_l2", "mg_restrict_l3",
                                    "mg_restrict_l4", "mg_restrict_l5", "mg_restrict_l6", "mg_restrict_l7+"};
     for (int l = 0; l < lc; ++l) {
+      if (tiled(mg[l]) && (l > 0 || fine_in != 3)) {   // GMRES forms its basis vector in the separate passes
+        if (l > 0) down<false>(l, TileB<T>{mg[l].b});
+        else if (fine_in == 1) down<true>(0, TileInP<T>{S.kp, S.kr, S.kq});
+        else down<true>(0, TileInS<T>{S.ks, S.kr, S.kv});
+        continue;
+      }
       for (int color = 0; color < 2; ++color) {
         const int zx = color == 0 ? 1 : 0;
-        if (l == 0 && fine_in == 1) smooth(mg[0], color, zx, 0, none, MgInP<T>{S.kp, S.kr, S.kv});
+        if (l == 0 && fine_in == 1) smooth(mg[0], color, zx, 0, none, MgInP<T>{S.kp, S.kr, S.kq});
         else if (l == 0 && fine_in == 2) smooth(mg[0], color, zx, 0, none, MgInS<T>{S.ks, S.kr, S.kv});
         else if (l == 0 && fine_in == 3)
           smooth(mg[0], color, zx, 0, none, MgInV<T>{S.kt, S.kp, S.gmV, S.gmT + kGmTInv, (size_t)S.neq});
@@ -1201,12 +1282,23 @@ class Solver final : public SolverBase {
     }
     if (lc < nl) {
       MGSet<T> set{};
-      for (int l = lc; l < nl; ++l) set.L[l - lc] = mg[l];
+      int slots = 0;
+      for (int l = lc; l < nl; ++l) {
+        set.L[l - lc] = mg[l];
+        slots = std::max(slots, cycle_slots(mg[l]));
+      }
       const int cnt = nl - lc;
-      const size_t shm = sizeof(T) * 4 * 32 * S.K;
-      L("mg_coarse_cycle", [&] {
-        k_mg_cta_cycle<T><<<1, 1024, shm, st>>>(set, cnt, S.sc, mg_w, mg_coarse_sweeps);
-      });
+      // Levels of up to 32 slots a colour and 40 sigma levels take the form
+      // that keeps x and the operator on chip (32 x 2 and 8 x 2 columns, 20
+      // levels: FP32 21.9 -> 15.0 us, FP64 74.6 -> 57.7; 40 levels FP32 36.5
+      // -> 23.7, FP64 140 -> 115); with more slots the FP64 form spills and
+      // is slower (5 x 12 columns: 76.8 against 82.7 us)
+      if (slots <= kCycleSlots && S.K <= 20) cycle<1>(set, cnt);
+      else if (slots <= kCycleSlots && S.K <= 40) cycle<2>(set, cnt);
+      else
+        L("mg_coarse_cycle", [&] {
+          k_mg_cta_cycle<T><<<1, 1024, sizeof(T) * 4 * 32 * S.K, st>>>(set, cnt, S.sc, mg_w, mg_coarse_sweeps);
+        });
     }
     static const char* pnames[] = {"mg_prolong_l0", "mg_prolong_l1", "mg_prolong_l2", "mg_prolong_l3",
                                    "mg_prolong_l4", "mg_prolong_l5", "mg_prolong_l6", "mg_prolong_l7+"};
@@ -1214,6 +1306,11 @@ class Solver final : public SolverBase {
       const MGL<T>& f = mg[l];
       const MGL<T>& c = mg[l + 1];
       const Prolong<T> pr = prolong_from(f, c, mg_w);
+      if (tiled(f) && (l > 0 || fine_in != 3)) {
+        if (l > 0) up<false>(l, pr);
+        else up<true>(0, pr);
+        continue;
+      }
       // levels of 8192 columns or more: the correction in its own pass (C2:
       // 15.3 -> 14.7 ms/step FP32+IR, 63.9 -> 56.9 FP64); on smaller levels
       // one launch more costs more than the interpolations it saves

@@ -1,0 +1,40 @@
+"""GPU: grids at the edges of the multigrid cycle's tiled levels.
+
+Levels of up to 4096 columns run each half of a V-cycle as one launch of 4 x 4
+column tiles, and the last levels as one block's cycle.  Sides that are no
+multiple of the tile, a level of exactly 4096 columns and one just above, one
+sigma level, and the heights at which a thread takes a second level (33) or the
+block's cycle changes form (21, 41) must solve the pressure as the oracle
+does: eta and P within the 1e-10 that every FP64 grid is held to, and FP32+IR
+eta within 1e-6.
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from test_gpu_shapes import _case
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(64, 64, 2), (65, 64, 2), (63, 65, 3), (7, 9, 21), (13, 6, 33), (10, 9, 41), (66, 3, 1),
+          (32, 32, 20)]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_tiled_levels_step_like_the_oracle(shape, precision, oracle_mod, gpu_lib):
+    from nhwave_gb300 import fields as F, lib
+    p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
+    g = lib.Scenario(p, depth, eta)
+    po, _, _ = _case(*shape, 0, 1e-13)
+    o = oracle_mod.Oracle(po, depth.ravel(), eta.ravel())
+    for n in range(2):
+        assert g.step() == 0 and o.step() == 0
+    assert np.array_equal(g.get(F.MASK), o.get(F.MASK))
+    sl = o.shape.interior
+    r = rel_l2(g.get(F.ETA)[sl(F.ETA)], o.get(F.ETA)[sl(F.ETA)])
+    assert r < (1e-10 if precision == 0 else 1e-6), f"{shape} eta rel L2 {r:.3e}"
+    if precision == 0:
+        r = rel_l2(g.get(F.P)[sl(F.P)], o.get(F.P)[sl(F.P)])
+        assert r < 1e-10, f"{shape} P rel L2 {r:.3e}"
+    g.close()
