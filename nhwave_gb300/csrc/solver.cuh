@@ -369,15 +369,39 @@ class Solver final : public SolverBase {
       MGL<T> L0{};
       L0.M = M; L0.N = N; L0.K = K; L0.n = M * N * K;
       mg.push_back(L0);
-      while (use_mg && mg.size() < 16) {
+      double ratio = p.dy / p.dx;   // spacing ratio of the level, as far as the first levels even it out
+      int semi = 0;
+      while (use_mg && mg.size() < kPsMaxLevels) {
         MGL<T>& f = mg.back();
-        // aggregates of agg x agg columns while a direction keeps at least two
-        // aggregates; by default 2 x 2, and 4 x 4 once a level has at most
-        // 1024 columns -- one launched level fewer, the same iteration count
-        // on the submerged bar (7.3 per solve), 2 % less time per step
-        const int agg = p.mg_aggregate > 1 ? p.mg_aggregate : ((long long)f.M * f.N <= 1024 ? 4 : 2);
-        const int rx = f.M >= 2 * agg ? agg : (f.M >= 4 ? 2 : 1), ry = f.N >= 2 * agg ? agg : (f.N >= 4 ? 2 : 1);
+        // Aggregates of agg x agg columns while a direction keeps at least two
+        // aggregates; by default 2 x 2, and 4 x 4 on the last levels -- one
+        // launched level fewer.  4 x 4 starts at 1024 columns on narrow
+        // levels and at 512 where both sides are above 16: there the first
+        // 4 x 4 level costs iterations (basin 200 x 300 x 12 FP32+IR: 5.2 ->
+        // 4.2 a solve, 5.77 -> 5.10 ms/step; 64 x 64 x 10 3.51 -> 2.91; from
+        // 256 columns 320 x 320 x 15 is slower again, 8.97 -> 9.37).
+        const bool fixed = p.mg_aggregate > 1;
+        const int last = std::min(f.M, f.N) > 16 ? 512 : 1024;
+        const int agg = fixed ? p.mg_aggregate : ((long long)f.M * f.N <= last ? 4 : 2);
+        int rx = f.M >= 2 * agg ? agg : (f.M >= 4 ? 2 : 1), ry = f.N >= 2 * agg ? agg : (f.N >= 4 ? 2 : 1);
         if ((rx == 1 && ry == 1) || f.M * f.N <= 32) break;
+        // Grids whose spacings differ by 1.5 times or more: the in-level
+        // coupling along the finer spacing is (dy/dx)^2 times the other, and
+        // a red-black sweep hardly smooths across the weak one, so the first
+        // levels aggregate pairs along the finer spacing alone until the
+        // level's spacings are near each other (at most six such levels).
+        // Submerged bar 1024 x 64 x 20, dy/dx = 2: 7.3 -> 4.7 iterations a
+        // solve, 10.5 -> 8.8 ms/step; 128 x 40 x 12, dy/dx = 1/4: 12.8 ->
+        // 4.3, 6.70 -> 3.48.  Drawn at 1.5 because the further level costs
+        // as much as it saves there (dy/dx = 1.37: 4.75 -> 5.53 ms/step
+        // with it; 1.5: 7.96 -> 7.72).
+        if (!fixed && semi < 6) {
+          if (rx > 1 && ratio >= 1.5) {
+            rx = 2; ry = 1; ratio *= 0.5; ++semi;
+          } else if (ry > 1 && ratio * 1.5 <= 1.0) {
+            rx = 1; ry = 2; ratio *= 2.0; ++semi;
+          }
+        }
         f.rx = rx; f.ry = ry;
         f.Mc = (f.M + rx - 1) / rx; f.Nc = (f.N + ry - 1) / ry;
         MGL<T> c{};

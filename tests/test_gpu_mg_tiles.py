@@ -20,21 +20,42 @@ SHAPES = [(64, 64, 2), (65, 64, 2), (63, 65, 3), (7, 9, 21), (13, 6, 33), (10, 9
           (32, 32, 20)]
 
 
-@pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
-def test_tiled_levels_step_like_the_oracle(shape, precision, oracle_mod, gpu_lib):
+# spacings 4, 1/4, 1.5, 2 and 100 times apart: levels that aggregate along one side alone, to the end of a short side;
+# the last with more than 512 columns on a broad second level
+SPACINGS = [(48, 20, 4, 0.5, 2.0), (48, 20, 4, 2.0, 0.5), (33, 17, 5, 0.5, 0.75), (3, 40, 3, 0.5, 1.0),
+            (40, 6, 3, 0.5, 50.0), (60, 50, 3, 0.5, 0.5)]
+
+
+def _against_oracle(p, po, depth, eta, oracle_mod):
     from nhwave_gb300 import fields as F, lib
-    p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
     g = lib.Scenario(p, depth, eta)
-    po, _, _ = _case(*shape, 0, 1e-13)
     o = oracle_mod.Oracle(po, depth.ravel(), eta.ravel())
     for n in range(2):
         assert g.step() == 0 and o.step() == 0
     assert np.array_equal(g.get(F.MASK), o.get(F.MASK))
     sl = o.shape.interior
     r = rel_l2(g.get(F.ETA)[sl(F.ETA)], o.get(F.ETA)[sl(F.ETA)])
-    assert r < (1e-10 if precision == 0 else 1e-6), f"{shape} eta rel L2 {r:.3e}"
-    if precision == 0:
+    assert r < (1e-10 if p.precision == 0 else 1e-6), f"eta rel L2 {r:.3e}"
+    if p.precision == 0:
         r = rel_l2(g.get(F.P)[sl(F.P)], o.get(F.P)[sl(F.P)])
-        assert r < 1e-10, f"{shape} P rel L2 {r:.3e}"
+        assert r < 1e-10, f"P rel L2 {r:.3e}"
     g.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("grid", SPACINGS, ids=lambda s: "x".join(map(str, s)))
+def test_uneven_spacings_step_like_the_oracle(grid, precision, oracle_mod, gpu_lib):
+    M, N, K, dx, dy = grid
+    p, depth, eta = _case(M, N, K, precision, 1e-13 if precision == 0 else 1e-10)
+    po, _, _ = _case(M, N, K, 0, 1e-13)
+    p.dx = po.dx = dx
+    p.dy = po.dy = dy
+    _against_oracle(p, po, depth, eta, oracle_mod)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_tiled_levels_step_like_the_oracle(shape, precision, oracle_mod, gpu_lib):
+    p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
+    po, _, _ = _case(*shape, 0, 1e-13)
+    _against_oracle(p, po, depth, eta, oracle_mod)
