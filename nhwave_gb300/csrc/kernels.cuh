@@ -88,6 +88,40 @@ __device__ __forceinline__ R hllc(R sl, R sr, R ss, R fl, R fr, R ul, R uls, R u
   return fr + sr * (urs - ur);
 }
 
+// A divisor used more than once: the FP64 form divides by it, as the reference
+// does; the FP32+IR form multiplies by its FP64 reciprocal (one division of
+// some 25 FP64 instructions for all of them).
+template <class T>
+struct Quot {
+  double b, r;
+};
+template <class T>
+__device__ __forceinline__ Quot<T> over(double b) {
+  if constexpr (sizeof(T) == 4) return Quot<T>{b, 1.0 / b};
+  else return Quot<T>{b, 0.0};
+}
+template <class T>
+__device__ __forceinline__ double operator/(double a, const Quot<T>& q) {
+  if constexpr (sizeof(T) == 4) return a * q.r;
+  else return a / q.b;
+}
+
+// the same for divisors in the working precision R of a cell kernel
+template <class R>
+struct QuotR {
+  R b, r;
+};
+template <class R>
+__device__ __forceinline__ QuotR<R> over_r(R b) {
+  if constexpr (sizeof(R) == 4) return QuotR<R>{b, (R)1 / b};
+  else return QuotR<R>{b, (R)0};
+}
+template <class R>
+__device__ __forceinline__ R operator/(R a, const QuotR<R>& q) {
+  if constexpr (sizeof(R) == 4) return a * q.r;
+  else return a / q.b;
+}
+
 __device__ __forceinline__ int mirror(int i, int b, int e) {
   return i < b ? 2 * b - 1 - i : (i > e ? 2 * e + 1 - i : i);
 }
@@ -1298,6 +1332,29 @@ struct OpVelBcB {
 // sigma slopes of the last sigma_transform (zero before the first one).
 // Cmu = Visc; CmuHt per cell (Cmut_min until eval_turb).  Each bracket
 // keeps the reference's evaluation order (bit-exact in the FP64 form).
+// DelxSc / DelySc and DelxSl / DelySl of the last sigma_transform (zero
+// before the first one), which OpDiffusion reads: formed once a column and
+// level, since each of that stencil's 30 uses costs two FP64 divisions
+// (515 x 30 x 15 FP32+IR: 679 us with the slopes in place, now below 30).
+struct OpViscSlopes {
+  static constexpr const char* kName = "visc_slopes";
+  template <class T>
+  __device__ void operator()(const Dev<T>& S, int i, int j, int k) const {
+    const long long q = i2(S, i, j), o = i3(S, i, j, k);
+    T cx = (T)0, cy = (T)0, lx = (T)0, ly = (T)0;
+    if (S.sc->sig_set != 0) {
+      const Quot<T> D = over<T>(S.scD[q]);
+      const double hx = S.scHx[q], ex = S.scEx[q], hy = S.scHy[q], ey = S.scEy[q];
+      const double c = S.sigc[k], l = S.sig[k];
+      const double c1 = (1.0 - c) / D, c0 = c / D, l1 = (1.0 - l) / D, l0 = l / D;
+      cx = (T)(c1 * hx - c0 * ex);
+      cy = (T)(c1 * hy - c0 * ey);
+      lx = (T)(l1 * hx - l0 * ex);
+      ly = (T)(l1 * hy - l0 * ey);
+    }
+    S.vsx[o] = cx; S.vsy[o] = cy; S.vlx[o] = lx; S.vly[o] = ly;
+  }
+};
 struct OpDiffusion {
   static constexpr const char* kName = "diffusion";
   template <class T>
@@ -1308,21 +1365,15 @@ struct OpDiffusion {
       S.Dxx[o] = (T)0; S.Dxy[o] = (T)0; S.Dyx[o] = (T)0; S.Dyy[o] = (T)0; S.Dzx[o] = (T)0; S.Dzy[o] = (T)0;
       return;
     }
-    const bool set = S.sc->sig_set != 0;
-    // DelxSc / DelySc at level kk (sigc) and DelxSl / DelySl at face kk (sig)
-    auto slope = [&](const double* lev, const double* H, const double* E, int ii, int jj, int kk) -> R {
-      if (!set) return (R)0;
-      const long long q = i2(S, ii, jj);
-      return (R)((1.0 - lev[kk]) / S.scD[q] * H[q] - lev[kk] / S.scD[q] * E[q]);
-    };
-    auto Scx = [&](int ii, int jj, int kk) { return slope(S.sigc, S.scHx, S.scEx, ii, jj, kk); };
-    auto Scy = [&](int ii, int jj, int kk) { return slope(S.sigc, S.scHy, S.scEy, ii, jj, kk); };
+    auto Scx = [&](int ii, int jj, int kk) -> R { return S.vsx[i3(S, ii, jj, kk)]; };
+    auto Scy = [&](int ii, int jj, int kk) -> R { return S.vsy[i3(S, ii, jj, kk)]; };
     const T* DU = S.DU;
     const T* DV = S.DV;
     const T* DW = S.DW;
     auto F = [&](const T* a, int ii, int jj, int kk) -> R { return a[i3(S, ii, jj, kk)]; };
-    const R dx = (R)S.dx, dy = (R)S.dy;
-    const R cmu = (R)S.v_cmu, sch = (R)S.v_schmidt;
+    const QuotR<R> dx = over_r<R>((R)S.dx), dy = over_r<R>((R)S.dy);
+    const R cmu = (R)S.v_cmu;
+    const QuotR<R> sch = over_r<R>((R)S.v_schmidt);
     // CmuHt of a cell; face viscosity between two cells; cell viscosity
     auto H = [&](int ii, int jj, int kk) -> R { return (R)S.CmuHt[i3(S, ii, jj, kk)]; };
     auto nuF = [&](R ha, R hb) -> R { return (R)0.5 * (cmu + cmu) + (R)0.5 * (ha + hb) / sch; };
@@ -1332,14 +1383,14 @@ struct OpDiffusion {
     const R nuN = nuF(H(i, j + 1, k), h0), nuS = nuF(h0, H(i, j - 1, k));
     const R cE = nuC(i + 1, j, k), cW = nuC(i - 1, j, k), cN = nuC(i, j + 1, k), cS = nuC(i, j - 1, k);
     const R cD = nuC(i, j, k - 1), c0 = nuC(i, j, k), cU = nuC(i, j, k + 1);
-    const double* dsg = S.dsig;
-    const double L1top = dsg[k + 1] / (dsg[k] + dsg[k + 1]), L2top = dsg[k] / (dsg[k] + dsg[k + 1]);
-    const double L1bot = dsg[k] / (dsg[k] + dsg[k - 1]), L2bot = dsg[k - 1] / (dsg[k] + dsg[k - 1]);
-    const double ck = (dsg[k] + dsg[k + 1]) / 2.0, ck1 = (dsg[k - 1] + dsg[k]) / 2.0;
-    const R ac = (R)(-ck / (ck + ck1) / ck1), bc = (R)((ck - ck1) / (ck * ck1)), gc = (R)(ck1 / (ck + ck1) / ck);
+    auto lv = [&](int n) { return S.lvv[n * S.Kloc + k]; };
+    const double L1top = lv(kLvL1t), L2top = lv(kLvL2t), L1bot = lv(kLvL1b), L2bot = lv(kLvL2b);
+    const R rck = (R)lv(kLvCk), rck1 = (R)lv(kLvCk1);
+    const QuotR<R> qck = over_r<R>(rck), qck1 = over_r<R>(rck1), qcc = over_r<R>(rck + rck1);
+    const R ac = (R)lv(kLvAc), bc = (R)lv(kLvBc), gc = (R)lv(kLvGc);
     const R nuH_top = ((R)L1top * cmu + (R)L2top * cmu) + ((R)L1top * h0 + (R)L2top * H(i, j, k + 1)) / sch;
     const R nuH_bot = ((R)L1bot * cmu + (R)L2bot * cmu) + ((R)L1bot * H(i, j, k - 1) + (R)L2bot * h0) / sch;
-    const R Dc = (R)S.D[c], dsk = (R)dsg[k], rck = (R)ck, rck1 = (R)ck1;
+    const QuotR<R> Dc = over_r<R>((R)S.D[c]), dsk = over_r<R>((R)S.dsig[k]);
     auto s3 = [&](const T* a, bool y, int ii, int jj) -> R {   // a F(k-1) Sc(k-1) + b .. + c ..
       auto sc = [&](int kk) { return y ? Scy(ii, jj, kk) : Scx(ii, jj, kk); };
       return ac * F(a, ii, jj, k - 1) * sc(k - 1) + bc * F(a, ii, jj, k) * sc(k) + gc * F(a, ii, jj, k + 1) * sc(k + 1);
@@ -1356,12 +1407,12 @@ struct OpDiffusion {
              gc * (F(DW, ii, jj, k + 1) * sc(k + 1) + F(a, ii, jj, k + 1) / Dc);
     };
     auto vco = [&](bool y, R& cA, R& cB, R& cC) {   // coefficients of d/dsigma[nu Sl d/dsigma]
-      const R st = slope(S.sig, y ? S.scHy : S.scHx, y ? S.scEy : S.scEx, i, j, k + 1);
-      const R sb = slope(S.sig, y ? S.scHy : S.scHx, y ? S.scEy : S.scEx, i, j, k);
+      const T* sl = y ? S.vly : S.vlx;
+      const R st = sl[o + S.sz], sb = sl[o];
       const R Pq = nuH_top * st - nuH_bot * sb, Sq = nuH_top * st + nuH_bot * sb;
-      cA = Pq * ac / dsk + Sq / rck1 / (rck + rck1);
-      cB = Pq * bc / dsk - Sq / rck1 / rck;
-      cC = Pq * gc / dsk + Sq / rck / (rck + rck1);
+      cA = Pq * ac / dsk + Sq / qck1 / qcc;
+      cB = Pq * bc / dsk - Sq / qck1 / qck;
+      cC = Pq * gc / dsk + Sq / qck / qcc;
     };
     R xA, xB, xC, yA, yB, yC;
     vco(false, xA, xB, xC);
@@ -1572,18 +1623,19 @@ struct OpKeTop {
   }
 };
 
-// HLPA face value (src/nhwave.F:7809-7847)
+// HLPA face value (src/nhwave.F:7809-7847): the upstream value Fw and, where
+// the profile is monotone (|Fp - 2 Fw + Fww| < |Fp - Fww|), its correction,
+// whose division the other (finite) faces skip
+__device__ __forceinline__ double ke_hlpa_side(double Fww, double Fw, double Fp) {
+  const double d = Fp - Fww, c = fabs(Fp - 2.0 * Fw + Fww);
+  if (fabs(d) <= (double)1.e-16f || (c >= fabs(d) && c <= 1.0e300)) return Fw;
+  const double a = c < fabs(d) ? 1.0 : 0.0;
+  return Fw + a * (Fp - Fw) * (Fw - Fww) / d;
+}
 __device__ __forceinline__ double ke_hlpa(double Uw, double Fww, double Fw, double Fp, double Fe) {
-  double h = 0.0;
-  if (Uw >= 0.0) {
-    const double a = fabs(Fp - 2.0 * Fw + Fww) < fabs(Fp - Fww) ? 1.0 : 0.0;
-    h = fabs(Fp - Fww) <= (double)1.e-16f ? Fw : Fw + a * (Fp - Fw) * (Fw - Fww) / (Fp - Fww);
-  }
-  if (Uw < 0.0) {
-    const double a = fabs(Fw - 2.0 * Fp + Fe) < fabs(Fw - Fe) ? 1.0 : 0.0;
-    h = fabs(Fw - Fe) <= (double)1.e-16f ? Fp : Fp + a * (Fw - Fp) * (Fp - Fe) / (Fw - Fe);
-  }
-  return h;
+  if (Uw >= 0.0) return ke_hlpa_side(Fww, Fw, Fp);
+  if (Uw < 0.0) return ke_hlpa_side(Fe, Fp, Fw);
+  return 0.0;
 }
 
 // adv_scalar_hlpa with flux_scalar_bc (src/nhwave.F:7604-7806, 7850-7986) at
@@ -1622,43 +1674,72 @@ __device__ double ke_r5(const Dev<T>& S, int i, int j, int k, const T* Phi, doub
     return w * ke_hlpa(w, (double)Phi[o - 2 * z], (double)Phi[o - z], (double)Phi[o], (double)Phi[o + z]);
   };
   const double cmu = S.v_cmu;
-  auto nu = [&](double ha, double hb) { return 0.5 * (cmu + cmu) + 0.5 * (ha + hb) / SchtH; };
+  const Quot<T> Sc = over<T>(SchtH), dx2 = over<T>(S.dx * S.dx), dy2 = over<T>(S.dy * S.dy);
+  auto nu = [&](double ha, double hb) { return 0.5 * (cmu + cmu) + 0.5 * (ha + hb) / Sc; };
   auto H = [&](int ii, int jj) { return (double)S.CmuHt[i3(S, ii, jj, k)]; };
   auto Dq = [&](int ii, int jj) { return S.D[i2(S, ii, jj)]; };
   auto Ph = [&](int ii, int jj) { return (double)Phi[i3(S, ii, jj, k)]; };
   const double Sdx = 0.5 *
                      (nu(H(i + 1, j), H(i, j)) * (Dq(i + 1, j) + Dq(i, j)) * (Ph(i + 1, j) - Ph(i, j)) -
                       nu(H(i, j), H(i - 1, j)) * (Dq(i, j) + Dq(i - 1, j)) * (Ph(i, j) - Ph(i - 1, j))) /
-                     (S.dx * S.dx);
+                     dx2;
   const double Sdy = 0.5 *
                      (nu(H(i, j + 1), H(i, j)) * (Dq(i, j + 1) + Dq(i, j)) * (Ph(i, j + 1) - Ph(i, j)) -
                       nu(H(i, j), H(i, j - 1)) * (Dq(i, j) + Dq(i, j - 1)) * (Ph(i, j) - Ph(i, j - 1))) /
-                     (S.dy * S.dy);
-  return -(1.0 / S.dx * (scx(i + 1) - scx(i))) - 1.0 / S.dy * (scy(j + 1) - scy(j)) -
-         1.0 / S.dsig[k] * (scz(k + 1) - scz(k)) + Sdx + Sdy;
+                     dy2;
+  // 2 i2dx = 1/dx and lv_ds = 1/dsig, rounded alike
+  return -(2.0 * S.i2dx * (scx(i + 1) - scx(i))) - 2.0 * S.i2dy * (scy(j + 1) - scy(j)) -
+         S.lv_ds[k] * (scz(k + 1) - scz(k)) + Sdx + Sdy;
 }
 
 // shear production of the nonlinear model (ke_model = 2, src/nhwave.F:
 // 10139-10274): Reynolds stresses from the velocity gradient G, contracted
-// with G per PRODTYPE (1 vertical shear of U, V; 2 vertical shear; else 3-D)
+// with G per PRODTYPE (1 vertical shear of U, V; 2 vertical shear; else 3-D).
+// kOrdered: the reference's order of sums, term by term (FP64 form); else the
+// same sums, in FP64 too, with the traces formed once and the stresses that
+// the contraction does not read left out (a seventh of the operations).
+template <bool kOrdered>
 __device__ inline double ke_production(const double (&G)[3][3], double tk, double ep, int prod_type) {
   const double c23 = (double)(2.0f / 3.0f), c13 = (double)(1.0f / 3.0f);
+  const double tke = kOrdered ? 0.0 : tk / ep;
   double smax = 0.0;
   for (int n = 0; n < 3; ++n)
     if (fabs(G[n][n]) > smax) smax = fabs(G[n][n]);
-  smax = smax * tk / ep;
+  smax = kOrdered ? smax * tk / ep : smax * tke;
   const double c_d = c23 * (1.0 / ((double)7.4f + 2.0 * smax));
   double dmx = 0.0;
   for (int n = 0; n < 3; ++n)
     for (int m = 0; m < 3; ++m)
       if (fabs(G[n][m]) > dmx) dmx = fabs(G[n][m]);
-  dmx = dmx * tk / ep;
+  dmx = kOrdered ? dmx * tk / ep : dmx * tke;
   const double c_1 = 1.0 / ((double)185.2f + 3.0 * (dmx * dmx));
   const double c_2 = -(1.0 / (58.5 + 2.0 * (dmx * dmx)));
   const double c_3 = 1.0 / ((double)370.4f + 3.0 * (dmx * dmx));
-  const double tk2 = tk * tk, tk3 = tk * tk * tk, ep2 = ep * ep;
   const int n1 = prod_type == 1 ? 2 : 3, m0 = (prod_type == 1 || prod_type == 2) ? 2 : 0;
   double P = 0.0;
+  if constexpr (!kOrdered) {
+    const double kd = c_d * tk * tke, t3 = tk * tke * tke, k1 = c_1 * t3, k2 = c_2 * t3, k3 = c_3 * t3;
+    double gg = 0.0, gt = 0.0;   // sum G_lg G_gl, sum G_lg G_lg
+    for (int l = 0; l < 3; ++l)
+      for (int g = 0; g < 3; ++g) {
+        gg += G[l][g] * G[g][l];
+        gt += G[l][g] * G[l][g];
+      }
+    const double iso = -c23 * tk - c23 * k1 * gg - c13 * (k2 + k3) * gt;
+    for (int n = 0; n < 3; ++n)
+      for (int m = 0; m < 3; ++m) {
+        if (!(n < n1 && m >= m0)) continue;
+        double s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        for (int l = 0; l < 3; ++l) {
+          s1 += G[n][l] * G[l][m] + G[m][l] * G[l][n];
+          s2 += G[n][l] * G[m][l];
+          s3 += G[l][n] * G[l][m];
+        }
+        P += (kd * (G[n][m] + G[m][n]) + k1 * s1 + k2 * s2 + k3 * s3 + (n == m ? iso : 0.0)) * G[n][m];
+      }
+    return P;
+  }
+  const double tk2 = tk * tk, tk3 = tk * tk * tk, ep2 = ep * ep;
   for (int n = 0; n < 3; ++n)
     for (int m = 0; m < 3; ++m) {
       const double dl = n == m ? 1.0 : 0.0;
@@ -1680,7 +1761,7 @@ __device__ inline double ke_production(const double (&G)[3][3], double tk, doubl
   return P;
 }
 
-// one interior column of kepsilon_3D: production, the epsilon equation
+// kepsilon_3D over the interior columns: production, the epsilon equation
 // (HLPA advection, horizontal diffusion, source, implicit vertical
 // diffusion with the bed and surface terms), its SSP-RK combination and
 // floor, the same for tke (whose source reads the new DEps), then the bed
@@ -1688,205 +1769,257 @@ __device__ inline double ke_production(const double (&G)[3][3], double tk, doubl
 // 10858).  The column's own snapshot gives DelxSc / DelySc / DelxSl /
 // DelySl; neighbours are read only through Tke, Eps, CmuHt, D, U, V, W, Ex,
 // Ey, Omega, Mask and the surface values, which no thread writes here.
-struct OpKeColumn {
-  static constexpr const char* kName = "kepsilon_column";
-  static constexpr int kMaxK = 64;   // Kglob <= 64 (nhw_create)
-  int istep;                         // 0-based stage
-  template <class T>
-  __device__ void operator()(const Dev<T>& S, int i, int j) const {
-    const long long q = i2(S, i, j);
-    const double Dc = S.D[q];
-    const int mk = S.Mask[q];
-    const double Dmin = S.ke_dmin, dt = S.sc->dt, cmu = S.v_cmu, cmuR = 0.0;
-    const bool rng = S.ke_rng != 0;
-    const double c1e = rng ? (double)1.42f : (double)1.44f;
-    double c2e = rng ? 0.0 : (double)1.92f;
-    const double c3e = 0.0, Prod_b = 0.0;
-    const double cmiu = rng ? (double)0.085f : (double)0.09f;
-    const double Sche = rng ? (double)0.72f : (double)1.3f, Schk = rng ? (double)0.72f : 1.0;
-    const int KB = S.KB, KE = S.KE, n = KE - KB + 1;
-    const double* sigc = S.sigc;
-    const double* sig = S.sig;
-    const double* dsig = S.dsig;
-    const bool set = S.sc->sig_set != 0;
-    auto slope = [&](const double* lev, bool y, int kk) -> double {
-      if (!set) return 0.0;
-      return (1.0 - lev[kk]) / S.scD[q] * (y ? S.scHy[q] : S.scHx[q]) - lev[kk] / S.scD[q] * (y ? S.scEy[q] : S.scEx[q]);
-    };
-    auto Scx = [&](int kk) { return slope(sigc, false, kk); };
-    auto Scy = [&](int kk) { return slope(sigc, true, kk); };
-    auto Slx = [&](int kk) { return slope(sig, false, kk); };
-    auto Sly = [&](int kk) { return slope(sig, true, kk); };
-    auto at = [&](const T* a, int kk) -> double { return (double)a[i3(S, i, j, kk)]; };
-    auto ds = [&](int kk) { return sigc[kk + 1] - sigc[kk - 1]; };
-    const double dxh = S.DelxH[q], dyh = S.DelyH[q], dxe = S.DelxEta[q], dye = S.DelyEta[q];
-    // production (zero in shallow or dry columns; no negative production at the surface)
-    double prod[kMaxK];
-    for (int k = KB; k <= KE; ++k) {
+//
+// A block has 32 columns and up to 16 threads a column: every cell's
+// production and coefficients are formed side by side, and one warp solves the
+// 32 tridiagonal systems in shared memory.  (One thread a column leaves a
+// 515 x 30 grid with 15,450 threads, each with 15 levels of some 2,000 FP64
+// operations in a row: 2967 us a stage in FP32+IR, now 632 us.)  Bound by the
+// FP64 pipe, most of it divisions; the FP32+IR form shares its reciprocals
+// (Quot) and production sums.
+constexpr int kKeThreadsY = 16;
+inline size_t ke_smem(int K) { return sizeof(double) * (size_t)(5 * 32 * K); }
+template <class T>
+__global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int istep) {
+  if (gated_off(S)) return;
+  extern __shared__ double ke_sh[];
+  const int K = S.K, KB = S.KB, KE = S.KE;
+  double *prod = ke_sh, *A = prod + 32 * K, *B = A + 32 * K, *C = B + 32 * K, *X = C + 32 * K;
+  const double* sigc = S.sigc;
+  const double* sig = S.sig;
+  const double* dsig = S.dsig;
+  const int tx = threadIdx.x, ty = threadIdx.y, by = blockDim.y;
+  const int t = blockIdx.x * 32 + tx;
+  const bool valid = t < S.M * S.N;
+  const int i = S.IB + (valid ? t % S.M : 0), j = S.JB + (valid ? t / S.M : 0);
+  const long long q = i2(S, i, j);
+  const double Dc = S.D[q];
+  const int mk = S.Mask[q];
+  const double Dmin = S.ke_dmin, dt = S.sc->dt, cmu = S.v_cmu, cmuR = 0.0;
+  const bool rng = S.ke_rng != 0;
+  const double c1e = rng ? (double)1.42f : (double)1.44f;
+  const double c3e = 0.0, Prod_b = 0.0;
+  const double cmiu = rng ? (double)0.085f : (double)0.09f;
+  const double Sche = rng ? (double)0.72f : (double)1.3f, Schk = rng ? (double)0.72f : 1.0;
+  const bool set = S.sc->sig_set != 0;
+  const Quot<T> scD = over<T>(S.scD[q]), Dq = over<T>(Dc), D2 = over<T>(Dc * Dc);
+  const double shx = S.scHx[q], sex = S.scEx[q], shy = S.scHy[q], sey = S.scEy[q];
+  auto Scx = [&](int kk) { return set ? (1.0 - sigc[kk]) / scD * shx - sigc[kk] / scD * sex : 0.0; };
+  auto Scy = [&](int kk) { return set ? (1.0 - sigc[kk]) / scD * shy - sigc[kk] / scD * sey : 0.0; };
+  auto Slx = [&](int kk) { return set ? (1.0 - sig[kk]) / scD * shx - sig[kk] / scD * sex : 0.0; };
+  auto Sly = [&](int kk) { return set ? (1.0 - sig[kk]) / scD * shy - sig[kk] / scD * sey : 0.0; };
+  auto at = [&](const T* a, int kk) -> double { return (double)a[i3(S, i, j, kk)]; };
+  auto dsq = [&](int kk) { return over<T>(sigc[kk + 1] - sigc[kk - 1]); };
+  auto lv = [&](int n, int kk) { return S.lvv[n * S.Kloc + kk]; };
+  const double dxh = S.DelxH[q], dyh = S.DelyH[q], dxe = S.DelxEta[q], dye = S.DelyEta[q];
+  const bool wet = Dc >= Dmin && mk == 1;
+  const bool solve = valid && !(Dc < Dmin && mk == 0);
+  // production (zero in shallow or dry columns; no negative production at the surface)
+  if (solve)
+    for (int m = ty; m < K; m += by) {
+      const int k = KB + m;
       double P = 0.0;
-      if (Dc >= Dmin && mk == 1) {
+      if (wet) {
         double G[3][3];
+        const Quot<T> ds = dsq(k);
         const double dU = at(S.U, k + 1) - at(S.U, k - 1), dV = at(S.V, k + 1) - at(S.V, k - 1);
         const double dW = at(S.W, k + 1) - at(S.W, k - 1);
-        G[0][0] = at(S.keDxU, k) + dU / ds(k) * Scx(k);
-        G[0][1] = at(S.keDyU, k) + dU / ds(k) * Scy(k);
-        G[0][2] = 1.0 / Dc * dU / ds(k);
-        G[1][0] = at(S.keDxV, k) + dV / ds(k) * Scx(k);
-        G[1][1] = at(S.keDyV, k) + dV / ds(k) * Scy(k);
-        G[1][2] = 1.0 / Dc * dV / ds(k);
-        G[2][0] = at(S.keDxW, k) + dW / ds(k) * Scx(k);
-        G[2][1] = at(S.keDyW, k) + dW / ds(k) * Scy(k);
-        G[2][2] = 1.0 / Dc * dW / ds(k);
-        P = ke_production(G, at(S.Tke, k), at(S.Eps, k), S.ke_prod);
+        const double sx = Scx(k), sy = Scy(k);
+        G[0][0] = at(S.keDxU, k) + dU / ds * sx;
+        G[0][1] = at(S.keDyU, k) + dU / ds * sy;
+        G[0][2] = 1.0 / Dq * dU / ds;
+        G[1][0] = at(S.keDxV, k) + dV / ds * sx;
+        G[1][1] = at(S.keDyV, k) + dV / ds * sy;
+        G[1][2] = 1.0 / Dq * dV / ds;
+        G[2][0] = at(S.keDxW, k) + dW / ds * sx;
+        G[2][1] = at(S.keDyW, k) + dW / ds * sy;
+        G[2][2] = 1.0 / Dq * dW / ds;
+        P = ke_production<sizeof(T) == 8>(G, at(S.Tke, k), at(S.Eps, k), S.ke_prod);
         if (k == KE && P < 0.0) P = 0.0;
       }
-      prod[k - KB] = P;
+      prod[m * 32 + tx] = P;
     }
-    double A[kMaxK], B[kMaxK], C[kMaxK], X[kMaxK];
-    // one equation: eq = 2 epsilon, 1 tke
-    auto column = [&](int eq) {
-      const T* Old = eq == 2 ? S.Eps : S.Tke;
-      T* Dv = eq == 2 ? S.DEps : S.DTke;
-      const double zL = eq == 2 ? S.keTopE[q] : S.keTopK[q];
-      const double Sch = eq == 2 ? Sche : Schk;
-      const double DxD = (dxh + dxe) / Dc, DyD = (dyh + dye) / Dc;
-      for (int k = KB; k <= KE; ++k) {
-        const int m = k - KB;
-        const double L1top = dsig[k + 1] / (dsig[k] + dsig[k + 1]), L2top = dsig[k] / (dsig[k] + dsig[k + 1]);
-        const double L1bot = dsig[k] / (dsig[k] + dsig[k - 1]), L2bot = dsig[k - 1] / (dsig[k] + dsig[k - 1]);
-        const double dsigck = (dsig[k] + dsig[k + 1]) / 2.0, dsigck1 = (dsig[k - 1] + dsig[k]) / 2.0;
-        const double alpha_c = -dsigck / (dsigck + dsigck1) / dsigck1;
-        const double beta_c = (dsigck - dsigck1) / (dsigck * dsigck1);
-        const double gamma_c = dsigck1 / (dsigck + dsigck1) / dsigck;
+  // one equation: eq = 2 epsilon, 1 tke
+  for (int eq = 2; eq >= 1; --eq) {
+    const T* Old = eq == 2 ? S.Eps : S.Tke;
+    T* Dv = eq == 2 ? S.DEps : S.DTke;
+    const double zL = eq == 2 ? S.keTopE[q] : S.keTopK[q];
+    const double SchV = eq == 2 ? Sche : Schk;
+    const Quot<T> Sch = over<T>(SchV);
+    const double DxD = (dxh + dxe) / Dq, DyD = (dyh + dye) / Dq;
+    if (solve)
+      for (int m = ty; m < K; m += by) {
+        const int k = KB + m;
+        const double L1top = lv(kLvL1t, k), L2top = lv(kLvL2t, k);
+        const double L1bot = lv(kLvL1b, k), L2bot = lv(kLvL2b, k);
+        const double dsigck = lv(kLvCk, k), dsigck1 = lv(kLvCk1, k);
+        const double alpha_c = lv(kLvAc, k), beta_c = lv(kLvBc, k), gamma_c = lv(kLvGc, k);
+        const Quot<T> dsk{dsig[k], S.lv_ds[k]};
+        const double vt0 = at(S.CmuVt, k), vtu = at(S.CmuVt, k + 1), vtd = at(S.CmuVt, k - 1);
+        const double ht0 = at(S.CmuHt, k), htu = at(S.CmuHt, k + 1), htd = at(S.CmuHt, k - 1);
         const double nuV_top = (L1top * cmu + L2top * cmu) + (L1top * cmuR + L2top * cmuR) +
-                               (L1top * at(S.CmuVt, k) + L2top * at(S.CmuVt, k + 1)) / Sch;
+                               (L1top * vt0 + L2top * vtu) / Sch;
         const double nuH_top = (L1top * cmu + L2top * cmu) + (L1top * cmuR + L2top * cmuR) +
-                               (L1top * at(S.CmuHt, k) + L2top * at(S.CmuHt, k + 1)) / Sch;
+                               (L1top * ht0 + L2top * htu) / Sch;
         const double nuV_bot = (L1bot * cmu + L2bot * cmu) + (L1bot * cmuR + L2bot * cmuR) +
-                               (L1bot * at(S.CmuVt, k - 1) + L2bot * at(S.CmuVt, k)) / Sch;
+                               (L1bot * vtd + L2bot * vt0) / Sch;
         const double nuH_bot = (L1bot * cmu + L2bot * cmu) + (L1bot * cmuR + L2bot * cmuR) +
-                               (L1bot * at(S.CmuHt, k - 1) + L2bot * at(S.CmuHt, k)) / Sch;
-        double r = ke_r5(S, i, j, k, Old, Sch);
-        if (eq == 2) r = r + c1e * Dc * (prod[m] + c3e * Prod_b) * at(S.Eps, k) / at(S.Tke, k);
-        else r = r + Dc * (prod[m] + Prod_b) - at(S.DEps, k);
+                               (L1bot * htd + L2bot * ht0) / Sch;
+        const double tk = at(S.Tke, k), ep = at(S.Eps, k);
+        const Quot<T> tkq = over<T>(eq == 2 ? tk : 1.0);
+        double r = ke_r5(S, i, j, k, Old, SchV);
+        if (eq == 2) r = r + c1e * Dc * (prod[m * 32 + tx] + c3e * Prod_b) * ep / tkq;
+        else r = r + Dc * (prod[m * 32 + tx] + Prod_b) - at(S.DEps, k);
+        const double slx1 = Slx(k + 1), sly1 = Sly(k + 1), slx0 = Slx(k), sly0 = Sly(k);
         if (k == KB) {
-          r = r - (-(nuH_bot * (dxh * DxD + dyh * DyD) * at(Old, k))) / dsig[k] +
+          r = r - (-(nuH_bot * (dxh * DxD + dyh * DyD) * at(Old, k))) / dsk +
               (dsig[k] - dsigck) / (dsig[k] * dsig[k] / 2.0 * (dsigck + dsig[k] / 2.0)) *
-                  (nuH_top * (Slx(k + 1) * dxh + Sly(k + 1) * dyh) + nuV_top / Dc) * at(Old, k);
+                  (nuH_top * (slx1 * dxh + sly1 * dyh) + nuV_top / Dq) * at(Old, k);
         } else if (k == KE) {
-          r = r + ((nuH_top * (dxe * dxe + dye * dye) + nuV_top) / (Dc * Dc) * (at(Old, k + 1) - at(Old, k)) * Dc / dsigck -
+          r = r + ((nuH_top * (dxe * dxe + dye * dye) + nuV_top) / D2 * (at(Old, k + 1) - at(Old, k)) * Dc / dsigck -
                    nuH_top * (-(dxe * DxD) - dye * DyD) * zL) /
-                      dsig[k] +
+                      dsk +
               (dsig[k] - dsigck1) / (dsig[k] * dsig[k] / 2.0 * (dsigck1 + dsig[k] / 2.0)) *
-                  (nuH_bot * (-(Slx(k) * dxe) - Sly(k) * dye) + nuV_bot / Dc) * zL;
+                  (nuH_bot * (-(slx0 * dxe) - sly0 * dye) + nuV_bot / Dq) * zL;
         }
-        auto top = [&](int kk) { return nuH_top * (Slx(k + 1) * Scx(kk) + Sly(k + 1) * Scy(kk)) + nuV_top / (Dc * Dc); };
-        auto bot = [&](int kk) { return nuH_bot * (Slx(k) * Scx(kk) + Sly(k) * Scy(kk)) + nuV_bot / (Dc * Dc); };
-        if (k == KB) A[m] = 0.0;
-        else if (k == KE) A[m] = -dt * (3.0 / 2.0 * bot(k - 1) / (dsigck1 * (dsigck1 + dsig[k] / 2.0)));
-        else
-          A[m] = -dt * ((top(k - 1) - bot(k - 1)) * alpha_c / dsig[k] +
-                        (top(k - 1) + bot(k - 1)) / (dsigck1 * (dsigck1 + dsigck)));
-        if (k == KB) C[m] = -dt * (3.0 / 2.0 * top(k + 1) / (dsigck * (dsigck + dsig[k] / 2.0)));
-        else if (k == KE) C[m] = 0.0;
-        else
-          C[m] = -dt * ((top(k + 1) - bot(k + 1)) * gamma_c / dsig[k] +
-                        (top(k + 1) + bot(k + 1)) / (dsigck * (dsigck1 + dsigck)));
+        const double vtopD = nuV_top / D2, vbotD = nuV_bot / D2;
+        auto top = [&](double sx, double sy) { return nuH_top * (slx1 * sx + sly1 * sy) + vtopD; };
+        auto bot = [&](double sx, double sy) { return nuH_bot * (slx0 * sx + sly0 * sy) + vbotD; };
+        const double sxd = Scx(k - 1), syd = Scy(k - 1), sx0 = Scx(k), sy0 = Scy(k), sxu = Scx(k + 1), syu = Scy(k + 1);
+        double a = 0.0, c = 0.0;
+        if (k == KB) {
+        } else if (k == KE) a = -dt * (3.0 / 2.0 * bot(sxd, syd) / (dsigck1 * (dsigck1 + dsig[k] / 2.0)));
+        else {
+          const double tp = top(sxd, syd), bt = bot(sxd, syd);
+          a = -dt * ((tp - bt) * alpha_c / dsk + (tp + bt) / (dsigck1 * (dsigck1 + dsigck)));
+        }
+        if (k == KB) c = -dt * (3.0 / 2.0 * top(sxu, syu) / (dsigck * (dsigck + dsig[k] / 2.0)));
+        else if (k == KE) {
+        } else {
+          const double tp = top(sxu, syu), bt = bot(sxu, syu);
+          c = -dt * ((tp - bt) * gamma_c / dsk + (tp + bt) / (dsigck * (dsigck1 + dsigck)));
+        }
         double b0 = 1.0;
         if (eq == 2) {
+          double c2e = (double)1.92f;
           if (rng) {   // c2e of Yakhot et al. (1992) from the strain rate
-            const double dUs = (at(S.U, k + 1) - at(S.U, k - 1)) / ds(k), dVs = (at(S.V, k + 1) - at(S.V, k - 1)) / ds(k);
-            const double dWs = (at(S.W, k + 1) - at(S.W, k - 1)) / ds(k);
-            const double S11 = at(S.keDxU, k) + dUs * Scx(k);
-            const double S22 = at(S.keDyV, k) + dVs * Scy(k);
-            const double S33 = 1.0 / Dc * (at(S.W, k + 1) - at(S.W, k - 1)) / ds(k);
-            const double S12 = 0.5 * (at(S.keDyU, k) + dUs * Scy(k) + at(S.keDxV, k) + dVs * Scx(k));
-            const double S13 = 0.5 * ((at(S.U, k + 1) - at(S.U, k - 1)) / ds(k) / Dc + at(S.keDxW, k) + dWs * Scx(k));
-            const double S23 = 0.5 * ((at(S.V, k + 1) - at(S.V, k - 1)) / ds(k) / Dc + at(S.keDyW, k) + dWs * Scy(k));
-            const double lambda = at(S.Tke, k) / at(S.Eps, k) *
+            const Quot<T> ds = dsq(k);
+            const double dU = at(S.U, k + 1) - at(S.U, k - 1), dV = at(S.V, k + 1) - at(S.V, k - 1);
+            const double dW = at(S.W, k + 1) - at(S.W, k - 1);
+            const double dUs = dU / ds, dVs = dV / ds;
+            const double dWs = dW / ds;
+            const double S11 = at(S.keDxU, k) + dUs * sx0;
+            const double S22 = at(S.keDyV, k) + dVs * sy0;
+            const double S33 = 1.0 / Dq * dW / ds;
+            const double S12 = 0.5 * (at(S.keDyU, k) + dUs * sy0 + at(S.keDxV, k) + dVs * sx0);
+            const double S13 = 0.5 * (dU / ds / Dq + at(S.keDxW, k) + dWs * sx0);
+            const double S23 = 0.5 * (dV / ds / Dq + at(S.keDyW, k) + dWs * sy0);
+            const double lambda = tk / ep *
                                   sqrt(2.0 * (S11 * S11 + S22 * S22 + S33 * S33 + 2.0 * (S12 * S12 + S13 * S13 + S23 * S23)));
             const double l3 = lambda * lambda * lambda;
             c2e = (double)1.68f + cmiu * l3 * (1.0 - lambda / (double)4.38f) / (1.0 + (double)0.012f * l3);
             c2e = dmax_(0.0, dmin_(c2e, 4.0));
           }
-          b0 = 1.0 + dt * c2e * at(S.Eps, k) / at(S.Tke, k);
+          b0 = 1.0 + dt * c2e * ep / tkq;
         }
-        if (k == KB) B[m] = b0 - dt * (-(3.0 / 2.0 - dsigck / dsig[k]) * top(k) / (dsig[k] / 2.0 * dsigck));
-        else if (k == KE) B[m] = b0 - dt * (-(3.0 / 2.0 - dsigck1 / dsig[k]) * bot(k) / (dsig[k] / 2.0 * dsigck1));
-        else B[m] = b0 - dt * ((top(k) - bot(k)) * beta_c / dsig[k] - (top(k) + bot(k)) / (dsigck * dsigck1));
-        X[m] = at(Dv, k) + dt * r;
-      }
-      // trig (src/nhwave.F:13182-13224): elimination in place, then back substitution
-      for (int m = 1; m < n; ++m) {
-        const double coeff = A[m] / B[m - 1];
-        B[m] = B[m] - coeff * C[m - 1];
-        X[m] = X[m] - coeff * X[m - 1];
-      }
-      X[n - 1] = X[n - 1] / B[n - 1];
-      for (int m = n - 2; m >= 0; --m) X[m] = (X[m] - C[m] * X[m + 1]) / B[m];
-      for (int k = KB; k <= KE; ++k) Dv[i3(S, i, j, k)] = (T)X[k - KB];
-    };
-    auto rk = [&](T* Dv, const T* Dv0, double vmin) {
-      if (!(Dc >= Dmin && mk == 1)) return;
-      const double al = S.alpha[istep], be = S.beta[istep];
-      for (int k = KB; k <= KE; ++k) {
-        const long long o = i3(S, i, j, k);
-        const double v = al * (double)Dv0[o] + be * (double)Dv[o];
-        Dv[o] = (T)dmax_(v, Dc * vmin);
-      }
-    };
-    const bool solve = !(Dc < Dmin && mk == 0);
-    if (solve) column(2);
-    rk(S.DEps, S.DEps0, kEpsMin);
-    if (solve) column(1);
-    rk(S.DTke, S.DTke0, kTkeMin);
-    // bed: wall function (src/nhwave.F:10776-10831)
-    if (!(Dc < Dmin || mk == 0)) {
-      const long long ob = i3(S, i, j, KB);
-      const double Abot = sqrt(1.0 + dxh * dxh + dyh * dyh), Bbot = sqrt(1.0 + dxh * dxh);
-      const double du = (double)S.DU[ob], dv = (double)S.DV[ob], dw = (double)S.DW[ob];
-      const double DUprime = (du - dxh * dw) / Bbot;
-      const double DVprime = (-(dxh * dyh * du) + (1.0 + dxh * dxh) * dv - dyh * dw) / Abot / Bbot;
-      const double DUmag = sqrt(DUprime * DUprime + DVprime * DVprime);
-      double Tkeb = kTkeMin, Epsb = kEpsMin;
-      if (!(DUmag / Dc < (double)1.e-6f)) {
-        const double Dz1 = 0.5 * Dc * dsig[KB] / Abot;
-        double Cdrag;
-        if (S.ibot == 1) Cdrag = S.cd0;
+        double b;
+        if (k == KB) b = b0 - dt * (-(3.0 / 2.0 - dsigck / dsk) * top(sx0, sy0) / (dsig[k] / 2.0 * dsigck));
+        else if (k == KE) b = b0 - dt * (-(3.0 / 2.0 - dsigck1 / dsk) * bot(sx0, sy0) / (dsig[k] / 2.0 * dsigck1));
         else {
-          const double t = kKappa / log(Dz1 / (S.zob / 30.0));
-          Cdrag = t * t;
+          const double tp = top(sx0, sy0), bt = bot(sx0, sy0);
+          b = b0 - dt * ((tp - bt) * beta_c / dsk - (tp + bt) / (dsigck * dsigck1));
         }
-        Cdrag = dmin_(Cdrag, (cmu + cmuR + at(S.CmuVt, KB)) / Dz1 / (DUmag + kSmall) * Dc);
-        const double Ustar = sqrt(Cdrag) * DUmag / Dc;
-        Tkeb = dmax_(Ustar * Ustar / sqrt(cmiu), kTkeMin);
-        Epsb = dmax_(Ustar * Ustar * Ustar / (kKappa * Dz1), kEpsMin);
+        A[m * 32 + tx] = a; B[m * 32 + tx] = b; C[m * 32 + tx] = c;
+        X[m * 32 + tx] = at(Dv, k) + dt * r;
       }
-      const T tb = (T)(Dc * Tkeb), eb = (T)(Dc * Epsb);
-      for (int k = 0; k <= NG; ++k) {
-        S.DTke[ob - S.sz * k] = tb;
-        S.DEps[ob - S.sz * k] = eb;
+    __syncthreads();
+    // trig (src/nhwave.F:13182-13224): elimination in place, then back
+    // substitution; B ends as the pivot's divisor
+    if (solve && ty == 0) {
+      Quot<T> pb = over<T>(B[tx]);
+      if constexpr (sizeof(T) == 4) B[tx] = pb.r;
+      for (int m = 1; m < K; ++m) {
+        const int w = m * 32 + tx;
+        const double coeff = A[w] / pb;
+        pb = over<T>(B[w] - coeff * C[w - 32]);
+        B[w] = sizeof(T) == 4 ? pb.r : pb.b;
+        X[w] = X[w] - coeff * X[w - 32];
+      }
+      double x = X[(K - 1) * 32 + tx] / pb;
+      X[(K - 1) * 32 + tx] = x;
+      for (int m = K - 2; m >= 0; --m) {
+        const int w = m * 32 + tx;
+        const double e = X[w] - C[w] * x;
+        x = sizeof(T) == 4 ? e * B[w] : e / B[w];
+        X[w] = x;
       }
     }
-    // surface: gradient condition (Derakhti et al. 2015, eq. 60) with the
-    // limited slopes of the surface values
-    if (!(mk == 0 || Dc < Dmin)) {
-      auto tsl = [&](const double* top, bool y) {
-        const long long st = y ? S.sy : 1;
-        const double h = y ? S.dy : S.dx;
-        return lim_slope<double>(top[q - st], top[q], top[q + st], h, h);
-      };
-      const double gK = dxe * tsl(S.keTopK, false) + dye * tsl(S.keTopK, true);
-      const double gE = dxe * tsl(S.keTopE, false) + dye * tsl(S.keTopE, true);
-      const double Atop = sqrt(1.0 + dxe * dxe + dye * dye);
-      for (int k = 1; k <= NG; ++k) {
-        const double f = (sigc[KE + k] - sigc[KE - k + 1]) * (Dc * Dc) / (Atop * Atop);
-        S.DTke[i3(S, i, j, KE + k)] = (T)(at(S.DTke, KE - k + 1) + f * gK);
-        S.DEps[i3(S, i, j, KE + k)] = (T)(at(S.DEps, KE - k + 1) + f * gE);
+    __syncthreads();
+    // DEps / DTke of the stage, then its SSP-RK combination and floor
+    if (valid) {
+      const T* Dv0 = eq == 2 ? S.DEps0 : S.DTke0;
+      const double vmin = eq == 2 ? kEpsMin : kTkeMin;
+      const double al = S.alpha[istep], be = S.beta[istep];
+      for (int m = ty; m < K; m += by) {
+        const long long o = i3(S, i, j, KB + m);
+        T x = Dv[o];
+        if (solve) x = (T)X[m * 32 + tx];
+        if (wet) {
+          const double v = al * (double)Dv0[o] + be * (double)x;
+          x = (T)dmax_(v, Dc * vmin);
+        }
+        Dv[o] = x;
       }
     }
   }
-};
+  __syncthreads();
+  if (!valid || ty != 0) return;
+  // bed: wall function (src/nhwave.F:10776-10831)
+  if (!(Dc < Dmin || mk == 0)) {
+    const long long ob = i3(S, i, j, KB);
+    const double Abot = sqrt(1.0 + dxh * dxh + dyh * dyh), Bbot = sqrt(1.0 + dxh * dxh);
+    const double du = (double)S.DU[ob], dv = (double)S.DV[ob], dw = (double)S.DW[ob];
+    const double DUprime = (du - dxh * dw) / Bbot;
+    const double DVprime = (-(dxh * dyh * du) + (1.0 + dxh * dxh) * dv - dyh * dw) / Abot / Bbot;
+    const double DUmag = sqrt(DUprime * DUprime + DVprime * DVprime);
+    double Tkeb = kTkeMin, Epsb = kEpsMin;
+    if (!(DUmag / Dc < (double)1.e-6f)) {
+      const double Dz1 = 0.5 * Dc * dsig[KB] / Abot;
+      double Cdrag;
+      if (S.ibot == 1) Cdrag = S.cd0;
+      else {
+        const double lg = kKappa / log(Dz1 / (S.zob / 30.0));
+        Cdrag = lg * lg;
+      }
+      Cdrag = dmin_(Cdrag, (cmu + cmuR + at(S.CmuVt, KB)) / Dz1 / (DUmag + kSmall) * Dc);
+      const double Ustar = sqrt(Cdrag) * DUmag / Dc;
+      Tkeb = dmax_(Ustar * Ustar / sqrt(cmiu), kTkeMin);
+      Epsb = dmax_(Ustar * Ustar * Ustar / (kKappa * Dz1), kEpsMin);
+    }
+    const T tb = (T)(Dc * Tkeb), eb = (T)(Dc * Epsb);
+    for (int k = 0; k <= NG; ++k) {
+      S.DTke[ob - S.sz * k] = tb;
+      S.DEps[ob - S.sz * k] = eb;
+    }
+  }
+  // surface: gradient condition (Derakhti et al. 2015, eq. 60) with the
+  // limited slopes of the surface values
+  if (!(mk == 0 || Dc < Dmin)) {
+    auto tsl = [&](const double* top, bool y) {
+      const long long st = y ? S.sy : 1;
+      const double h = y ? S.dy : S.dx;
+      return lim_slope<double>(top[q - st], top[q], top[q + st], h, h);
+    };
+    const double gK = dxe * tsl(S.keTopK, false) + dye * tsl(S.keTopK, true);
+    const double gE = dxe * tsl(S.keTopE, false) + dye * tsl(S.keTopE, true);
+    const double Atop = sqrt(1.0 + dxe * dxe + dye * dye);
+    for (int k = 1; k <= NG; ++k) {
+      const double f = (sigc[KE + k] - sigc[KE - k + 1]) * (Dc * Dc) / (Atop * Atop);
+      S.DTke[i3(S, i, j, KE + k)] = (T)(at(S.DTke, KE - k + 1) + f * gK);
+      S.DEps[i3(S, i, j, KE + k)] = (T)(at(S.DEps, KE - k + 1) + f * gE);
+    }
+  }
+}
 
 // wall function of a friction wall (BC = 5) at one cell (src/nhwave.F:
 // 10870-11023): u* from the drag coefficient (Ibot 1) or the log law at
@@ -2463,92 +2596,123 @@ struct OpLdVisc {
 };
 
 // Implicit vertical viscous step of eval_duvw (src/nhwave.F:690-822 DU,
-// 850-1010 DV, 1012-1182 DW), one thread per wet interior column,
-// after the new D, Eta and eta slopes: DU/DV/DW hold the explicit update
-// DU + dt R2 on entry.  The tridiagonal systems are solved by trig's
-// elimination (src/nhwave.F:13182-13224) in FP64, with the eliminated
-// right-hand side kept in place (in T); the coefficients depend on the level
-// only, so they are recomputed rather than stored.
-struct OpVertVisc {
-  static constexpr const char* kName = "vertical_viscous";
-  static constexpr int kMaxK = 64;   // Kglob <= 64 (nhw_create)
-  template <class T>
-  __device__ void operator()(const Dev<T>& S, int i, int j) const {
-    const long long c = i2(S, i, j);
-    if (S.Mask[c] == 0) return;
-    const int KB = S.KB, KE = S.KE, n = KE - KB + 1;
-    const double dt = S.sc->dt, Dc = S.D[c];
-    // CmuVt of level k and the face viscosity between levels k1 and k2
-    auto vt = [&](int k) { return (double)S.CmuVt[i3(S, i, j, k)]; };
-    auto nuz = [&](int k1, int k2) { return 0.5 * (S.v_cmu + S.v_cmu) + 0.5 * (vt(k1) + vt(k2)) / S.v_schmidt; };
-    const double* dsg = S.dsig;
-    auto A = [&](int k) {
-      return k == KB ? 0.0 : -dt / (Dc * Dc) * nuz(k - 1, k) / (0.5 * dsg[k] * (dsg[k] + dsg[k - 1]));
-    };
-    auto C = [&](int k) {
-      return k == KE ? 0.0 : -dt / (Dc * Dc) * nuz(k, k + 1) / (0.5 * dsg[k] * (dsg[k] + dsg[k + 1]));
-    };
-    const double Wbot = -S.DeltH[c] - (double)S.U[i3(S, i, j, KB)] * S.DelxH[c] - (double)S.V[i3(S, i, j, KB)] * S.DelyH[c];
-    const double Wtop = (S.Eta[c] - S.Eta0[c]) / dt + (double)S.U[i3(S, i, j, KE)] * S.DelxEta[c] +
-                        (double)S.V[i3(S, i, j, KE)] * S.DelyEta[c];
-    double bp[kMaxK];   // eliminated diagonal; the eliminated right-hand side goes in place
-    for (int which = 0; which < 3; ++which) {
-      T* Fv = which == 0 ? S.DU : which == 1 ? S.DV : S.DW;
-      auto coefs = [&](int k, double& b, double& r) {
-        const double f = (double)Fv[i3(S, i, j, k)];
-        if (which < 2) {
-          if (k == KB && S.bc_z0 == 2)   // no-slip bed
-            b = 1.0 - C(k) + dt / (Dc * Dc) * (S.v_cmu + 0.0 + vt(k) / S.v_schmidt) / (0.5 * dsg[k] * dsg[k]);
-          else
-            b = 1.0 - A(k) - C(k);
-          if (k == KB && S.bc_z0 == 5) {   // friction law: bed stress in the first right-hand side
-            const double Dz1 = 0.5 * Dc * dsg[KB];
-            double Cdrag = S.cd0;
-            if (S.ibot != 1) {
-              const double lg = 1. / kKappa * log(30.0 * Dz1 / S.zob);
-              Cdrag = 1. / (lg * lg);
-            }
-            const double u = (double)S.U[i3(S, i, j, k)], v = (double)S.V[i3(S, i, j, k)];
-            const double Ustar2 = Cdrag * sqrt(u * u + v * v) * (which == 0 ? u : v);
-            r = f - dt * Ustar2 / dsg[k];
-          } else if (k == KE) {
-            r = f + dt * (which == 0 ? S.Wsx[c] : S.Wsy[c]) / dsg[k];
-          } else {
-            r = f;
+// 850-1010 DV, 1012-1182 DW) over the wet interior columns, after the new D,
+// Eta and eta slopes: DU/DV/DW hold the explicit update DU + dt R2 on entry.
+// The tridiagonal systems are solved by trig's elimination (src/nhwave.F:
+// 13182-13224) in FP64, with the eliminated right-hand side rounded to T.
+//
+// A block has 32 columns: all its threads form the coefficients, which DU, DV
+// and DW share, in shared memory, and one warp each then solves DU, DV and DW.
+// Bound by the chain of FP64 divisions of the elimination (515 x 30 x 15
+// FP32+IR, against one thread a column for all three: 415 -> 68 us).
+constexpr int kVvThreadsY = 8;
+inline size_t vv_smem(int K) { return sizeof(double) * (size_t)(8 * 32 * K); }
+template <class T>
+__global__ void __launch_bounds__(32 * kVvThreadsY) k_vert_visc(Dev<T> S) {
+  if (gated_off(S)) return;
+  extern __shared__ double vv_sh[];
+  const int K = S.K, KB = S.KB, KE = S.KE, nk = 32 * K;
+  double *As = vv_sh, *Cs = As + nk, *bps = Cs + nk, *rs = bps + 3 * nk;
+  const int tx = threadIdx.x, ty = threadIdx.y, by = blockDim.y;
+  const int t = blockIdx.x * 32 + tx;
+  const bool in = t < S.M * S.N;
+  const int i = S.IB + (in ? t % S.M : 0), j = S.JB + (in ? t / S.M : 0);
+  const long long c = i2(S, i, j), o = i3(S, i, j, KB);
+  const bool wet = in && S.Mask[c] != 0;
+  const double dt = S.sc->dt, Dc = S.D[c];
+  // CmuVt of level k and the face viscosity between levels k1 and k2
+  auto vt = [&](int k) { return (double)S.CmuVt[i3(S, i, j, k)]; };
+  const Quot<T> sch = over<T>(S.v_schmidt);
+  auto nuz = [&](int k1, int k2) { return 0.5 * (S.v_cmu + S.v_cmu) + 0.5 * (vt(k1) + vt(k2)) / sch; };
+  const double* dsg = S.dsig;
+  const double dtD2 = -dt / (Dc * Dc);
+  if (wet)
+    for (int m = ty; m < K; m += by) {
+      const int k = KB + m;
+      As[m * 32 + tx] = k == KB ? 0.0 : dtD2 * nuz(k - 1, k) / (0.5 * dsg[k] * (dsg[k] + dsg[k - 1]));
+      Cs[m * 32 + tx] = k == KE ? 0.0 : dtD2 * nuz(k, k + 1) / (0.5 * dsg[k] * (dsg[k] + dsg[k + 1]));
+      const long long e = o + S.sz * m;
+      rs[m * 32 + tx] = (double)S.DU[e];
+      rs[nk + m * 32 + tx] = (double)S.DV[e];
+      rs[2 * nk + m * 32 + tx] = (double)S.DW[e];
+    }
+  __syncthreads();
+  if (wet && ty < 3) {
+    const int which = ty;
+    double* bp = bps + which * nk + tx;
+    double* r = rs + which * nk + tx;
+    const double *A = As + tx, *C = Cs + tx;
+    auto coefs = [&](int k, double& b, double& rhs) {
+      const int w = (k - KB) * 32;
+      const double f = r[w];
+      if (which < 2) {
+        if (k == KB && S.bc_z0 == 2)   // no-slip bed
+          b = 1.0 - C[w] + dt / (Dc * Dc) * (S.v_cmu + 0.0 + vt(k) / sch) / (0.5 * dsg[k] * dsg[k]);
+        else
+          b = 1.0 - A[w] - C[w];
+        if (k == KB && S.bc_z0 == 5) {   // friction law: bed stress in the first right-hand side
+          const double Dz1 = 0.5 * Dc * dsg[KB];
+          double Cdrag = S.cd0;
+          if (S.ibot != 1) {
+            const double lg = 1. / kKappa * log(30.0 * Dz1 / S.zob);
+            Cdrag = 1. / (lg * lg);
           }
-        } else if (k == KB) {
-          const double q = 0.25 * dsg[k] * (dsg[k] + dsg[k - 1]);
-          b = 1.0 - C(k) + dt / (Dc * Dc) * nuz(k - 1, k) / q;
-          r = f + dt / Dc * nuz(k - 1, k) / q * Wbot;
+          const double u = (double)S.U[o], v = (double)S.V[o];
+          const double Ustar2 = Cdrag * sqrt(u * u + v * v) * (which == 0 ? u : v);
+          rhs = f - dt * Ustar2 / dsg[k];
         } else if (k == KE) {
-          const double q = 0.25 * dsg[k] * (dsg[k] + dsg[k + 1]);
-          b = 1.0 - A(k) + dt / (Dc * Dc) * nuz(k, k + 1) / q;
-          r = f + dt / Dc * nuz(k, k + 1) / q * Wtop;
+          rhs = f + dt * (which == 0 ? S.Wsx[c] : S.Wsy[c]) / dsg[k];
         } else {
-          b = 1.0 - A(k) - C(k);
-          r = f;
+          rhs = f;
         }
-      };
-      double rprev;
-      coefs(KB, bp[0], rprev);
-      Fv[i3(S, i, j, KB)] = (T)rprev;
-      for (int q = 1; q < n; ++q) {
-        double b, r;
-        coefs(KB + q, b, r);
-        const double coeff = A(KB + q) / bp[q - 1];
-        bp[q] = b - coeff * C(KB + q - 1);
-        rprev = r - coeff * rprev;
-        Fv[i3(S, i, j, KB + q)] = (T)rprev;
+      } else if (k == KB) {
+        const double Wbot = -S.DeltH[c] - (double)S.U[o] * S.DelxH[c] - (double)S.V[o] * S.DelyH[c];
+        const double q = 0.25 * dsg[k] * (dsg[k] + dsg[k - 1]);
+        b = 1.0 - C[w] + dt / (Dc * Dc) * nuz(k - 1, k) / q;
+        rhs = f + dt / Dc * nuz(k - 1, k) / q * Wbot;
+      } else if (k == KE) {
+        const long long ot = o + S.sz * (K - 1);
+        const double Wtop = (S.Eta[c] - S.Eta0[c]) / dt + (double)S.U[ot] * S.DelxEta[c] + (double)S.V[ot] * S.DelyEta[c];
+        const double q = 0.25 * dsg[k] * (dsg[k] + dsg[k + 1]);
+        b = 1.0 - A[w] + dt / (Dc * Dc) * nuz(k, k + 1) / q;
+        rhs = f + dt / Dc * nuz(k, k + 1) / q * Wtop;
+      } else {
+        b = 1.0 - A[w] - C[w];
+        rhs = f;
       }
-      double x = rprev / bp[n - 1];
-      Fv[i3(S, i, j, KE)] = (T)x;
-      for (int q = n - 2; q >= 0; --q) {
-        x = ((double)Fv[i3(S, i, j, KB + q)] - C(KB + q) * x) / bp[q];
-        Fv[i3(S, i, j, KB + q)] = (T)x;
-      }
+    };
+    // bp: the pivot's divisor (its reciprocal in the FP32+IR form)
+    double b, rprev;
+    coefs(KB, b, rprev);
+    Quot<T> pb = over<T>(b);
+    bp[0] = sizeof(T) == 4 ? pb.r : pb.b;
+    r[0] = (double)(T)rprev;
+    for (int m = 1; m < K; ++m) {
+      double rhs;
+      coefs(KB + m, b, rhs);
+      const double coeff = A[m * 32] / pb;
+      pb = over<T>(b - coeff * C[(m - 1) * 32]);
+      bp[m * 32] = sizeof(T) == 4 ? pb.r : pb.b;
+      rprev = rhs - coeff * rprev;
+      r[m * 32] = (double)(T)rprev;
+    }
+    double x = rprev / pb;
+    r[(K - 1) * 32] = x;
+    for (int m = K - 2; m >= 0; --m) {
+      const double e = r[m * 32] - C[m * 32] * x;
+      x = sizeof(T) == 4 ? e * bp[m * 32] : e / bp[m * 32];
+      r[m * 32] = x;
     }
   }
-};
+  __syncthreads();
+  if (wet)
+    for (int m = ty; m < K; m += by) {
+      const long long e = o + S.sz * m;
+      S.DU[e] = (T)rs[m * 32 + tx];
+      S.DV[e] = (T)rs[nk + m * 32 + tx];
+      S.DW[e] = (T)rs[2 * nk + m * 32 + tx];
+    }
+}
 
 // initial: DU = D*U*Mask over all cells (src/initialize.F:3160-3170)
 struct OpInitDU {

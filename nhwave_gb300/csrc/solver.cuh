@@ -333,8 +333,11 @@ class Solver final : public SolverBase {
     if (ke)   // k-epsilon state (checkpointed)
       for (T** pp : {&S.Tke, &S.Eps, &S.DTke, &S.DEps, &S.DTke0, &S.DEps0}) add(pp, sizeof(T) * n3);
     add(&S.P, sizeof(double) * n3);
-    if (p.viscous_flow)   // explicit viscous terms of the stage
-      for (T** pp : {&S.Dxx, &S.Dxy, &S.Dyx, &S.Dyy, &S.Dzx, &S.Dzy}) add(pp, sizeof(T) * n3);
+    if (p.viscous_flow) {   // explicit viscous terms of the stage, sigma slopes, level constants
+      for (T** pp : {&S.Dxx, &S.Dxy, &S.Dyx, &S.Dyy, &S.Dzx, &S.Dzy, &S.vsx, &S.vsy, &S.vlx, &S.vly})
+        add(pp, sizeof(T) * n3);
+      add((double**)&S.lvv, sizeof(double) * kLvN * S.Kloc);
+    }
     if (p.viscous_flow && p.ivturb == 30) {   // dynamic LES scratch
       S.ld_n = (long long)n3;
       add(&S.ld, sizeof(T) * n3 * 31);
@@ -522,6 +525,8 @@ class Solver final : public SolverBase {
       NHW_CU(cudaFuncSetAttribute(k_mg_cycle<T, 1>, at, (int)cycle_smem<T>(KMAX)));
       NHW_CU(cudaFuncSetAttribute(k_mg_cycle<T, 2>, at, (int)cycle_smem<T>(KMAX)));
     }
+    NHW_CU(cudaFuncSetAttribute(k_ke_column<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ke_smem(KMAX)));
+    NHW_CU(cudaFuncSetAttribute(k_vert_visc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vv_smem(KMAX)));
     NHW_CU(cudaFuncSetAttribute(k_mg_cta_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(sizeof(T) * 4 * 32 * 64)));
     NHW_CU(cudaMallocHost((void**)&h_sc, sizeof(DevScal)));
@@ -822,6 +827,16 @@ class Solver final : public SolverBase {
         lt[2 * S.Kloc + k] = (T)(0.5 * h.dsig[k]);
       }
       NHW_CU(cudaMemcpyAsync((void*)S.lvT, lt.data(), sizeof(T) * lt.size(), cudaMemcpyHostToDevice, st));
+      std::vector<double> lv(kLvN * (size_t)S.Kloc, 0.0);
+      for (int k = 1; k < S.Kloc - 1; ++k) {
+        const double d0 = h.dsig[k], du = h.dsig[k + 1], dd = h.dsig[k - 1];
+        const double ck = (d0 + du) / 2.0, ck1 = (dd + d0) / 2.0;
+        const double v[kLvN] = {du / (d0 + du), d0 / (d0 + du), d0 / (d0 + dd), dd / (d0 + dd), ck, ck1,
+                                -ck / (ck + ck1) / ck1, (ck - ck1) / (ck * ck1), ck1 / (ck + ck1) / ck};
+        for (int n = 0; n < kLvN; ++n) lv[n * (size_t)S.Kloc + k] = v[n];
+      }
+      if (S.lvv)
+        NHW_CU(cudaMemcpyAsync((void*)S.lvv, lv.data(), sizeof(double) * lv.size(), cudaMemcpyHostToDevice, st));
       NHW_CU(cudaStreamSynchronize(st));
     }
     struct Up { int f; const void* src; } ups[] = {
@@ -1352,11 +1367,17 @@ class Solver final : public SolverBase {
   // eval_duvw up to the pressure solve: explicit stage update, surface BC,
   // slopes, velocities and the Poisson system
   void stage_pre(int s) {
-    if (S.viscous) cells(OpDiffusion{});
+    if (S.viscous) {
+      box(OpViscSlopes{}, S.M + 2, S.N + 2, S.K + 2, S.IB - 1, S.JB - 1, S.KB - 1);
+      cells(OpDiffusion{});
+    }
     incols(OpExplicit{s});
     allcols(OpWlBcEta{});
     allcols(OpSlopeEta{true});
-    if (S.viscous) incols(OpVertVisc{});
+    if (S.viscous)
+      L("vertical_viscous", [&] {
+        k_vert_visc<T><<<cdiv((long long)S.M * S.N, 32), dim3(32, kVvThreadsY), vv_smem(S.K), st>>>(S);
+      });
     if (S.non_hydro) {
       get_uvw();
       poisson_setup();
@@ -1403,7 +1424,9 @@ class Solver final : public SolverBase {
     if (!S.viscous) return;
     if (S.ivturb == 10) {
       allcols(OpKeTop{});
-      incols(OpKeColumn{s});
+      L("kepsilon_column", [&] {
+        k_ke_column<T><<<cdiv((long long)S.M * S.N, 32), dim3(32, std::min(S.K, kKeThreadsY)), ke_smem(S.K), st>>>(S, s);
+      });
       box(OpKeSidesX{}, S.N * S.Kloc, 1, 1, 0, 0, 0);
       box(OpKeSidesY{}, S.Mloc * S.Kloc, 1, 1, 0, 0, 0);
       allcols(OpKeFinal{});

@@ -154,6 +154,14 @@ struct Dev {
   // DelySc (cell levels) and DelxSl / DelySl (faces) of that moment
   double *scD, *scEx, *scEy, *scHx, *scHy;
   T *CmuVt, *CmuHt;                // viscous flow: eddy viscosities per cell (ghosted 3-D), else nullptr
+  // viscous flow only, else nullptr (scratch): DelxSc / DelySc at the cell
+  // levels and DelxSl / DelySl at the faces of the last sigma_transform
+  T *vsx, *vsy, *vlx, *vly;
+  // viscous flow only: constants of a sigma level k in the vertical operators,
+  // [kLvN][Kloc]: dsig_k+1 / (dsig_k + dsig_k+1), dsig_k / (..), dsig_k /
+  // (dsig_k + dsig_k-1), dsig_k-1 / (..), the cell spacings above and below,
+  // and the three-point weights at k-1, k, k+1
+  const double* lvv;
   double *Hfx, *Hfy, *Hfx0, *Hfy0, *DelxH, *DelyH, *DeltH, *DeltHo, *Delt2H;
   double *DelxEta, *DelyEta, *SourceX, *SourceY, *SourceC, *Sponge, *R1, *Wsx, *Wsy;
   double *EtaxL, *EtaxR, *EtayL, *EtayR;
@@ -215,6 +223,8 @@ struct Dev {
   double* partials;   // reduction partials [nblocks * 8]
   DevScal* sc;
 };
+
+enum { kLvL1t, kLvL2t, kLvL1b, kLvL2b, kLvCk, kLvCk1, kLvAc, kLvBc, kLvGc, kLvN };
 
 // -------------------------------------------------------------- indexing
 template <class T>

@@ -1,0 +1,67 @@
+"""GPU: the column kernels of viscous flow at the sizes their blocks can go wrong at.
+
+k-epsilon columns and the implicit vertical step run as blocks of 32 columns
+with up to 16 (8) threads a column: column counts that are no multiple of 32,
+fewer levels than threads, a level more than threads, and the tallest column.
+FP64 is held to the oracle within 1e-13 over two hydrostatic stages (the same
+operations in the same order, but for the last bit of the source's cosine);
+FP32+IR to the FP64 form within 2e-5 of the fields' norms (single
+precision over two stages, as the FP32 parity bounds take it).
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2, seed_ke
+
+pytestmark = pytest.mark.gpu
+
+GRIDS = [(45, 3, 2), (33, 5, 9), (40, 4, 17), (37, 3, 33), (34, 2, 64)]
+KE = dict(viscous_flow=1, visc=1e-6, ivturb=10, ihturb=10, prod_type=3, bc_z0=5, ibot=1, cd0=0.006)
+RNG = dict(KE, rng=1, prod_type=2, ibot=2, zob=1e-3)
+SGS = dict(viscous_flow=1, visc=1e-6, cvs=0.2, chs=0.2, ivturb=2, ihturb=2, bc_z0=2)
+
+
+def _scene(grid, closure, precision):
+    from nhwave_gb300 import scenarios as S
+    M, N, K = grid
+    out = S.submerged_bar(M=M, N=N, K=K, dx=25.6 / M, dy=0.3, non_hydro=0, **closure)
+    out[0].precision = precision
+    x = np.arange(M)[None, :] + 0.3 * np.arange(N)[:, None]
+    return out[0], out[1], (0.01 * np.sin(0.4 * x)).ravel(), None
+
+
+def _stages(h, n):
+    assert h.estimate_dt() == 0
+    h.update_mask()
+    h.update_vars()
+    for s in range(1, n + 1):
+        h.source_terms()
+        h.fluxes()
+        h.eval_duvw(s)
+        h.sponge_damping()
+        h.eval_turb(s)
+
+
+@pytest.mark.parametrize("closure", [KE, RNG, SGS], ids=["ke", "ke_rng", "subgrid"])
+@pytest.mark.parametrize("grid", GRIDS, ids=lambda g: "x".join(map(str, g)))
+def test_viscous_columns(grid, closure, oracle_mod, gpu_lib):
+    from nhwave_gb300 import fields as F, lib
+    g, o = lib.Scenario(*_scene(grid, closure, 0)), oracle_mod.Oracle(*_scene(grid, closure, 0))
+    f = lib.Scenario(*_scene(grid, closure, 1))
+    if closure["ivturb"] == 10:
+        seed_ke(g, o)
+        for n in ("TKE", "EPS", "DTKE", "DEPS", "CMUVT", "CMUHT"):
+            f.set(getattr(F, n), g.get(getattr(F, n)))
+    for h in (g, o, f):
+        _stages(h, 2)
+    names = ["U", "V", "W", "DU", "DV", "DW", "CMUVT", "CMUHT"]
+    names += ["TKE", "EPS", "DTKE", "DEPS"] if closure["ivturb"] == 10 else []
+    for n in names:
+        fid = getattr(F, n)
+        a, b = g.get(fid), o.get(fid)
+        assert rel_l2(a, b) < 1e-13, f"{n} rel {rel_l2(a, b):.3e}"
+        if n in ("V", "DV"):
+            continue   # small beside U: held through CMUVT and the FP64 form
+        assert rel_l2(f.get(fid), a) < 2e-5, f"FP32+IR {n} rel {rel_l2(f.get(fid), a):.3e}"
+    for h in (g, f):
+        h.close()
