@@ -13,6 +13,7 @@
 // one allocates nothing and keeps no per-call state on the host.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -26,10 +27,8 @@ void set_last_error(const std::string& s);
 namespace {
 
 constexpr int kNaThreads = 256;
-constexpr int kNaCellsPerThread = 8;
-constexpr long long kNaCellsPerBlock = (long long)kNaThreads * kNaCellsPerThread;   // 2048
 constexpr int kNaMaxBlocks = 8192;                                                   // partial minima held
-constexpr long long kNaMaxCells = kNaMaxBlocks * kNaCellsPerBlock;                   // 16,777,216
+constexpr long long kNaMaxCells = 16777216;
 constexpr int kNaCounter = kNaMaxBlocks;                                             // counter slot
 
 // The scratch: one partial minimum per block, then a 256-byte line whose
@@ -45,50 +44,116 @@ static __device__ __align__(256) double g_dt_scratch[kNaMaxBlocks + 32];
 __device__ __forceinline__ double na_min(double m, double x) { return x < m ? x : m; }
 __device__ __forceinline__ double na_max(double a, double b) { return a > b ? a : b; }
 
-__device__ __forceinline__ double block_min(double m) {
-  __shared__ double sh[kNaThreads / 32];
-  for (int o = 16; o > 0; o >>= 1) m = na_min(m, __shfl_down_sync(0xffffffffu, m, o));
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) sh[warp] = m;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int w = 1; w < kNaThreads / 32; ++w) m = na_min(m, sh[w]);
-  return m;   // valid in thread 0
+// |x| of a finite or infinite x as an integer that orders as |x| does (the
+// bit patterns of non-negative doubles are ordered); -1 for NaN, which every
+// other value exceeds, so that a maximum skips it
+__device__ __forceinline__ long long abs_bits(double x) {
+  const long long b = __double_as_longlong(x) & 0x7fffffffffffffffll;
+  return b > 0x7ff0000000000000ll ? -1ll : b;
+}
+__device__ __forceinline__ long long max_ll(long long a, long long b) { return a > b ? a : b; }
+
+// a double as an integer of the same order (no NaN), and back: the minima are
+// reduced without the FP64 pipe, whose latency is most of a small grid's time
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double from_key(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
 
-// Same arithmetic as the handle's estimate_dt (src/nhwave.F:3694-3874 with
+// the block's minimum of m and, with kAll, maxima of u and v, valid in thread 0
+template <bool kAll>
+__device__ __forceinline__ void block_reduce(long long& m, long long& u, long long& v) {
+  __shared__ long long sh[3][kNaThreads / 32];
+  for (int o = 16; o > 0; o >>= 1) {
+    m = min(m, __shfl_down_sync(0xffffffffu, m, o));
+    if (kAll) {
+      u = max_ll(u, __shfl_down_sync(0xffffffffu, u, o));
+      v = max_ll(v, __shfl_down_sync(0xffffffffu, v, o));
+    }
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __syncthreads();   // sh may still be read from the call before
+  if (lane == 0) {
+    sh[0][warp] = m;
+    if (kAll) {
+      sh[1][warp] = u;
+      sh[2][warp] = v;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < kNaThreads / 32; ++w) {
+      m = min(m, sh[0][w]);
+      if (kAll) {
+        u = max_ll(u, sh[1][w]);
+        v = max_ll(v, sh[2][w]);
+      }
+    }
+}
+
+// Same values as the handle's estimate_dt (src/nhwave.F:3694-3874 with
 // viscous and slide limits off): tmp2 = min over interior cells of
 // dx/max(|U|+sqrt(g D), Small), dy/max(|V|+sqrt(g D), Small) and
 // dsig(k) D/max(|W|, Small); dt = min(1.05 dt_old, CFL tmp2, Large, DT_MAX).
 // Arrays are the reference's ghosted Fortran ones: U(Mloc,Nloc,Kloc),
 // D(Mloc,Nloc), dsig(Kloc) with Mloc = Mglob+4 (two ghost cells a side).
+//
+// A thread takes kc levels of a column.  Rounded sums and quotients are
+// monotone, so the smallest dx/(|U| + sqrt(g D)) of a block is that of the
+// column whose max |U| + sqrt(g D) is largest: one square root a thread and two
+// divisions a block instead of two and three a cell, the maxima kept in
+// integers off the FP64 pipe (1.2 TFLOP/s on GB300).  The dsig D / |W| of the
+// levels are divided only where products, with a margin far above their
+// rounding, do not show the smallest of them to be above dx/(|U| + sqrt(g D))
+// or its y counterpart.  Read once, coalesced along i: bound by the launch on
+// small grids and by HBM on large ones (GB300, a call in a graph with its
+// memset: 256 x 8 x 10 33.1 -> 10.4 us, 1024 x 64 x 20 129 -> 18.6 us,
+// 600 x 300 x 24 348 -> 30.9 us, whose bytes alone take 0.1, 5 and 15 us).
 __global__ void __launch_bounds__(kNaThreads)
 k_dt_min_noalloc(const double* __restrict__ U, const double* __restrict__ V, const double* __restrict__ W,
-                 const double* __restrict__ D, const double* __restrict__ dsig, int M, int N, int K, double dx,
-                 double dy, double cfl, double dt_old, double dt_max, double* __restrict__ dt_out,
+                 const double* __restrict__ D, const double* __restrict__ dsig, int M, int N, int K, int kc,
+                 double dx, double dy, double cfl, double dt_old, double dt_max, double* __restrict__ dt_out,
                  double* __restrict__ scratch) {
-  const long long Ml = M + 2 * NG, Nl = N + 2 * NG;
-  const long long n = (long long)M * N * K;
+  const long long Ml = M + 2 * NG, lev = Ml * (N + 2 * NG);
+  const unsigned cols = (unsigned)M * (unsigned)N;
+  const unsigned items = cols * (unsigned)((K + kc - 1) / kc);   // at most kNaMaxCells
   double m = kLarge;
-#pragma unroll
-  for (int q = 0; q < kNaCellsPerThread; ++q) {
-    const long long t = ((long long)blockIdx.x * kNaCellsPerThread + q) * kNaThreads + threadIdx.x;
-    if (t < n) {
-      const long long i = NG + t % M, r = t / M;
-      const long long j = NG + r % N, k = NG + r / N;
-      const long long c2 = i + Ml * j, c3 = c2 + Ml * Nl * k;
-      const double Dq = D[c2];
-      double tmp1 = na_max(fabs(U[c3]) + sqrt(kGrav * Dq), kSmall);
-      m = na_min(m, dx / tmp1);
-      tmp1 = na_max(fabs(V[c3]) + sqrt(kGrav * Dq), kSmall);
-      m = na_min(m, dy / tmp1);
-      tmp1 = na_max(fabs(W[c3]), kSmall);
-      m = na_min(m, dsig[k] * Dq / tmp1);
+  long long bu = -1ll, bv = -1ll;   // largest |U| + sqrt(g D), |V| + sqrt(g D) so far
+  for (unsigned t = blockIdx.x * kNaThreads + threadIdx.x; t < items; t += gridDim.x * kNaThreads) {
+    const unsigned ch = t / cols, col = t - ch * cols, jj = col / (unsigned)M;
+    const long long c2 = NG + (int)(col - jj * (unsigned)M) + Ml * (NG + (int)jj);
+    const int k0 = (int)ch * kc, k1 = min(K, k0 + kc);
+    const double Dq = D[c2];
+    long long u = -1ll, v = -1ll, w = -1ll, sg = 0x7fffffffffffffffll;
+    const long long c3 = c2 + lev * (NG + k0);
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) {
+      const long long c = c3 + lev * (k - k0);
+      u = max_ll(u, abs_bits(U[c]));
+      v = max_ll(v, abs_bits(V[c]));
+      w = max_ll(w, abs_bits(W[c]));
+      sg = min(sg, __double_as_longlong(dsig[NG + k]));   // as integers: a negative one comes first
     }
+    const double s = sqrt(kGrav * Dq);
+    const double tu = u < 0 ? kSmall : na_max(__longlong_as_double(u) + s, kSmall);
+    const double tv = v < 0 ? kSmall : na_max(__longlong_as_double(v) + s, kSmall);
+    bu = max_ll(bu, __double_as_longlong(tu));
+    bv = max_ll(bv, __double_as_longlong(tv));
+    const double a = __longlong_as_double(sg) * Dq, wm = w < 0 ? kSmall : na_max(__longlong_as_double(w), kSmall);
+    const double wf = wm * 1.0000001;
+    if (!(a * tu >= dx * wf || a * tv >= dy * wf))
+      for (int k = k0; k < k1; ++k) m = na_min(m, dsig[NG + k] * Dq / na_max(fabs(W[c3 + lev * (k - k0)]), kSmall));
   }
-  m = block_min(m);
+  long long key = order_key(m);
+  block_reduce<true>(key, bu, bv);
   __shared__ bool last;
   if (threadIdx.x == 0) {
+    m = from_key(key);
+    if (bu >= 0) m = na_min(m, dx / __longlong_as_double(bu));
+    if (bv >= 0) m = na_min(m, dy / __longlong_as_double(bv));
     scratch[blockIdx.x] = m;
     __threadfence();
     const unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(scratch + kNaCounter), 1u);
@@ -97,13 +162,13 @@ k_dt_min_noalloc(const double* __restrict__ U, const double* __restrict__ V, con
   __syncthreads();
   if (!last) return;
   __threadfence();
-  m = kLarge;
+  key = order_key(kLarge);
   for (unsigned b = threadIdx.x; b < gridDim.x; b += kNaThreads)
-    m = na_min(m, reinterpret_cast<volatile double*>(scratch)[b]);
-  m = block_min(m);
+    key = min(key, order_key(reinterpret_cast<volatile double*>(scratch)[b]));
+  block_reduce<false>(key, bu, bv);
   if (threadIdx.x == 0) {
     const double dt_growth = (double)1.05f * dt_old;
-    dt_out[0] = na_min(na_min(na_min(dt_growth, cfl * m), kLarge), dt_max);
+    dt_out[0] = na_min(na_min(na_min(dt_growth, cfl * from_key(key)), kLarge), dt_max);
   }
 }
 
@@ -194,8 +259,14 @@ extern "C" int nhw_estimate_dt_noalloc(const double* U, const double* V, const d
     set_last_error(std::string("nhw_estimate_dt_noalloc: cudaMemsetAsync: ") + cudaGetErrorString(e));
     return NHW_ERR_CUDA;
   }
-  const unsigned nb = (unsigned)((n + kNaCellsPerBlock - 1) / kNaCellsPerBlock);
-  k_dt_min_noalloc<<<nb, kNaThreads, 0, s>>>(U, V, W, D, dsig, Mglob, Nglob, Kglob, dx, dy, cfl, dt_old, dt_max,
+  // whole columns where there are enough of them to fill the GPU's 152 SMs
+  // (one square root a column), else as many chunks of levels as fill it
+  const long long cols = (long long)Mglob * Nglob, fill = 152 * 512;
+  const long long chunks = std::min<long long>(Kglob, (fill + cols - 1) / cols);
+  const int kc = (int)((Kglob + chunks - 1) / chunks);
+  const long long items = (long long)Mglob * Nglob * ((Kglob + kc - 1) / kc);
+  const unsigned nb = (unsigned)std::min<long long>(kNaMaxBlocks, (items + kNaThreads - 1) / kNaThreads);
+  k_dt_min_noalloc<<<nb, kNaThreads, 0, s>>>(U, V, W, D, dsig, Mglob, Nglob, Kglob, kc, dx, dy, cfl, dt_old, dt_max,
                                              dt_out, scratch);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
