@@ -69,15 +69,15 @@ class SolverBase {
   virtual int load_state(const void* host, size_t bytes) = 0;
 };
 
+// a field of the device layout as the caller's dense array (32-bit decode, as
+// k_box)
 template <class T>
-__global__ void k_pack(const void* src, int kind, double* dd, int* di, int nx, int ny, int nz, int sy,
-                       long long sz) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nx * ny * nz) return;
-  const int i = (int)(t % nx);
-  const long long r = t / nx;
-  const int j = (int)(r % ny), k = (int)(r / ny);
-  const long long s = i + (long long)sy * j + sz * k;
+__global__ void __launch_bounds__(256) k_pack(const void* src, int kind, double* dd, int* di, int nx, int ny, int nz,
+                                              int sy, long long sz) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (unsigned)nx * (unsigned)ny * (unsigned)nz) return;
+  const unsigned r = t / (unsigned)nx, k = r / (unsigned)ny;
+  const long long s = (int)(t - r * (unsigned)nx) + (long long)sy * (int)(r - k * (unsigned)ny) + sz * (int)k;
   if (kind == 0) dd[t] = (double)((const T*)src)[s];
   else if (kind == 1) dd[t] = ((const double*)src)[s];
   else di[t] = ((const int*)src)[s];
@@ -653,13 +653,34 @@ class Solver final : public SolverBase {
     *eb = d.kind == 2 ? 4 : 8;
     return NHW_OK;
   }
+  // the device address of `bytes` of page-locked host memory, nullptr for
+  // other memory
+  static void* mapped(void* host, size_t bytes) {
+    cudaPointerAttributes a{}, e{};
+    char* h = static_cast<char*>(host);
+    if (cudaPointerGetAttributes(&a, h) != cudaSuccess || cudaPointerGetAttributes(&e, h + bytes - 1) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (a.type != cudaMemoryTypeHost || e.type != cudaMemoryTypeHost || !a.devicePointer || !e.devicePointer ||
+        (char*)e.devicePointer - (char*)a.devicePointer != (ptrdiff_t)(bytes - 1))
+      return nullptr;
+    return a.devicePointer;
+  }
+  // Into page-locked memory the packing kernel writes directly, which spares
+  // the staging pass and the copy's start (GB300, one field read with its
+  // call: 0.6 MB 25 -> 21 us, 3 MB 37 -> 32 us, 13 MB 104 -> 87 us); other host
+  // memory goes through the staging buffer and the copy engine.
   int get_field(int f, void* host) override {
     FieldDesc d = desc(f);
     if (!d.ptr || !host) return NHW_ERR_ARG;
     const long long n = (long long)d.nx * d.ny * d.nz;
-    k_pack<T><<<cdiv(n, 256), 256, 0, st>>>(d.ptr, d.kind, d_stage, (int*)d_stage, d.nx, d.ny, d.nz, S.sy, S.sz);
+    const size_t bytes = (size_t)n * (d.kind == 2 ? 4 : 8);
+    void* direct = mapped(host, bytes);
+    double* out = direct ? (double*)direct : d_stage;
+    k_pack<T><<<cdiv(n, 256), 256, 0, st>>>(d.ptr, d.kind, out, (int*)out, d.nx, d.ny, d.nz, S.sy, S.sz);
     NHW_CU(cudaGetLastError());
-    NHW_CU(cudaMemcpyAsync(host, d_stage, n * (d.kind == 2 ? 4 : 8), cudaMemcpyDeviceToHost, st));
+    if (!direct) NHW_CU(cudaMemcpyAsync(host, d_stage, bytes, cudaMemcpyDeviceToHost, st));
     NHW_CU(cudaStreamSynchronize(st));
     return NHW_OK;
   }
