@@ -3170,14 +3170,35 @@ struct OpSponge {
 // =========================================================================
 //                 estimate_dt (src/nhwave.F:3694-3874)
 // =========================================================================
+// largest |x| so far, NaN skipped: bit patterns of non-negative numbers order
+// as they do
+template <class T>
+struct AbsMax {
+  long long m = -1ll;
+  __device__ __forceinline__ void take(T x) {
+    if constexpr (sizeof(T) == 4) {
+      const int b = __float_as_int(x) & 0x7fffffff;
+      m = max(m, b > 0x7f800000 ? -1ll : (long long)b);
+    } else {
+      const long long b = __double_as_longlong(x) & 0x7fffffffffffffffll;
+      m = max(m, b > 0x7ff0000000000000ll ? -1ll : b);
+    }
+  }
+  __device__ __forceinline__ bool any() const { return m >= 0; }
+  __device__ __forceinline__ double value() const {
+    if constexpr (sizeof(T) == 4) return (double)__int_as_float((int)m);
+    else return __longlong_as_double(m);
+  }
+};
 template <class T>
 __global__ void __launch_bounds__(256) k_dt_min(Dev<T> S) {
   // One thread per water column.  D, hence sqrt(g D), is the column's, and
   // division is monotonic in the denominator, so the smallest dx/tmp1 of a
   // column is dx over its largest tmp1 -- the same value, bit for bit, with
-  // two divisions and one square root per column instead of per cell.  The
-  // vertical candidate dsig(k) D / max(|W|, Small) keeps one division per
-  // cell.  A candidate replaces m only if it is smaller, as the reference's
+  // two divisions and one square root per column instead of per cell, the
+  // maxima kept as integers off the FP64 pipe.  The vertical candidates
+  // dsig(k) D / max(|W|, Small) are divided only in columns where they can be
+  // below those.  A candidate replaces m only if it is smaller, as the reference's
   // `if(dxonu<tmp2) tmp2=dxonu` (src/nhwave.F:3730-3746): a NaN candidate
   // leaves m unchanged (tmp1 = max(NaN, Small) is Small, whose quotient is
   // never the minimum).  Viscous flow: the limit dx^2 / (|CmuHt| + 1e-16)
@@ -3201,21 +3222,32 @@ __global__ void __launch_bounds__(256) k_dt_min(Dev<T> S) {
   }
   if (t < S.M * S.N) {
     const int i = S.IB + t % S.M, j = S.JB + t / S.M;
-    const long long q = i2(S, i, j);
-    const double Dq = S.D[q];
+    const double Dq = S.D[i2(S, i, j)];
     const double c = sqrt(kGrav * Dq);
-    double ux = kSmall, vy = kSmall;
-    for (int k = S.KB; k <= S.KE; ++k) {
-      const long long o = i3(S, i, j, k);
-      ux = dmax_(ux, dmax_(fabs((double)S.U[o]) + c, kSmall));
-      vy = dmax_(vy, dmax_(fabs((double)S.V[o]) + c, kSmall));
-      const double x = S.dsig[k] * Dq / dmax_(fabs((double)S.W[o]), kSmall);
-      if (x < m) m = x;
+    AbsMax<T> u, v, w;
+    long long sg = 0x7fffffffffffffffll;
+    const long long o0 = i3(S, i, j, S.KB);
+#pragma unroll 4
+    for (int k = 0; k < S.K; ++k) {
+      const long long o = o0 + S.sz * k;
+      u.take(S.U[o]);
+      v.take(S.V[o]);
+      w.take(S.W[o]);
+      sg = min(sg, __double_as_longlong(S.dsig[S.KB + k]));
     }
+    const double ux = u.any() ? dmax_(u.value() + c, kSmall) : kSmall, vy = v.any() ? dmax_(v.value() + c, kSmall) : kSmall;
     double x = S.dx / ux;
     if (x < m) m = x;
     x = S.dy / vy;
     if (x < m) m = x;
+    // the column's dsig D / |W| lie above m where the smallest dsig over the
+    // largest |W| does, by a margin far above the products' rounding
+    const double a = __longlong_as_double(sg) * Dq, wm = w.any() ? dmax_(w.value(), kSmall) : kSmall;
+    if (!(a >= m * wm * 1.0000001))
+      for (int k = 0; k < S.K; ++k) {
+        x = S.dsig[S.KB + k] * Dq / dmax_(fabs((double)S.W[o0 + S.sz * k]), kSmall);
+        if (x < m) m = x;
+      }
   }
   for (int o = 16; o > 0; o >>= 1) {
     m = dmin_(m, __shfl_down_sync(0xffffffffu, m, o));

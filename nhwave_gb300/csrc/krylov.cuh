@@ -20,6 +20,8 @@
 // (sc->conv != 0), so iterations can be queued without host round trips.  Dot
 // products are deterministic block reductions finished by the last block.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "kernels.cuh"
 
 namespace nhw {
@@ -84,14 +86,13 @@ template <class V>
 struct Xcol {
   V c, e, w, nn, s;
 };
+// levels [k0, k1) of column col
 template <class C, class V, class F>
-__device__ __forceinline__ void spmv_column(const C* __restrict__ cf, const V* __restrict__ x, size_t n, int t,
-                                            int kc, int M, int N, int K, V cxx, V cyy, F f) {
+__device__ __forceinline__ void spmv_levels(const C* __restrict__ cf, const V* __restrict__ x, size_t n, int col,
+                                            int k0, int k1, int M, int N, int K, V cxx, V cyy, F f) {
   const int MN = M * N;
-  const int col = t % MN, chunk = t / MN;
   const int ii = col % M, jj = col / M;
-  const int k0 = chunk * kc, k1 = min(K, k0 + kc);
-  if (k0 >= K) return;
+  if (k0 >= k1) return;
   const bool im = ii > 0, ip = ii < M - 1, jm = jj > 0, jp = jj < N - 1;
   auto load = [&](int k) {
     const int ic = col + MN * k;
@@ -140,6 +141,14 @@ __device__ __forceinline__ void spmv_column(const C* __restrict__ cf, const V* _
   }
 }
 
+template <class C, class V, class F>
+__device__ __forceinline__ void spmv_column(const C* __restrict__ cf, const V* __restrict__ x, size_t n, int t,
+                                            int kc, int M, int N, int K, V cxx, V cyy, F f) {
+  const int MN = M * N;
+  const int col = t % MN, chunk = t / MN;
+  const int k0 = chunk * kc, k1 = min(K, k0 + kc);
+  spmv_levels(cf, x, n, col, k0, k1, M, N, K, cxx, cyy, f);
+}
 // block-wide sum of NV accumulators (A = float or double), result in lane 0 of warp 0
 template <int NV, class A>
 __device__ __forceinline__ void block_sum_t(A (&v)[NV], double (&out)[NV]) {
@@ -164,13 +173,12 @@ __device__ __forceinline__ void block_sum_t(A (&v)[NV], double (&out)[NV]) {
 // partials + last-block finalisation (fixed order); `part` holds `stride`
 // doubles per block
 template <int NV, class T, class Fin>
-__device__ __forceinline__ void finish_reduce_at(const Dev<T>& S, double* part, int stride, double (&v)[NV],
-                                                 Fin fin) {
+__device__ __forceinline__ void finish_reduce_of(const Dev<T>& S, double* part, int stride, int bid, int nb,
+                                                 double (&v)[NV], Fin fin) {
   __shared__ bool last;
   __shared__ double sh2[NV * 32];
-  const int nb = gridDim.x;
   if (threadIdx.x == 0) {
-    for (int q = 0; q < NV; ++q) part[(size_t)blockIdx.x * stride + q] = v[q];
+    for (int q = 0; q < NV; ++q) part[(size_t)bid * stride + q] = v[q];
     __threadfence();
     const unsigned prev = atomicAdd(&S.sc->counter[0], 1u);
     last = (prev == (unsigned)nb - 1);
@@ -199,6 +207,11 @@ __device__ __forceinline__ void finish_reduce_at(const Dev<T>& S, double* part, 
   }
 }
 template <int NV, class T, class Fin>
+__device__ __forceinline__ void finish_reduce_at(const Dev<T>& S, double* part, int stride, double (&v)[NV],
+                                                 Fin fin) {
+  finish_reduce_of<NV>(S, part, stride, (int)blockIdx.x, (int)gridDim.x, v, fin);
+}
+template <int NV, class T, class Fin>
 __device__ __forceinline__ void finish_reduce(const Dev<T>& S, double (&v)[NV], Fin fin) {
   finish_reduce_at<NV>(S, S.partials, 8, v, fin);
 }
@@ -221,38 +234,10 @@ __device__ __forceinline__ void set_cond(const Dev<T>& S, unsigned long long h, 
 // Status codes of the C interface that the device writes.
 constexpr int kStKrylovNoconv = 6, kStNaN = 7, kStTimeout = 8;
 
-// r64 = b - A64 x64; inner right-hand side rT = (T) r64; ||r64||, ||b||.
-// The last block then makes the refinement decision of the outer loop (the
-// HYPRE stopping test ||r||/||b|| <= TOL, src/pressure.F:225-258 calls the
-// solver with TOL and ITMAX): stop on convergence, on b = 0 (the solution is
-// then x = 0), on a non-finite residual or an inner breakdown flagged as NaN,
-// or when ITMAX inner iterations or the sweep cap are used up; otherwise it
-// sets the next inner tolerance and iteration budget.  kFirst opens a solve.
+// What the last block of each reducing kernel does with the totals a.
 template <class T, bool kFirst>
-__global__ void __launch_bounds__(256) k_res64(Dev<T> S) {
-  // a step held back by k_dt_finalize: the loop conditions keep their
-  // launch default (0), so no sweep runs
-  if (gated_off(S)) return;
-  const int M = S.M, N = S.N, K = S.K;
-  const size_t n = (size_t)S.neq;
-  double v[2] = {0.0, 0.0};
-#pragma unroll
-  for (int q = 0; q < kCPT; ++q) {
-    const int ic = (blockIdx.x * kCPT + q) * blockDim.x + threadIdx.x;
-    if (ic < S.neq) {
-      int ii, jj, kk;
-      decode(ic, M, N, ii, jj, kk);
-      const double b = S.rhs64[ic];
-      const double r = b - spmv_c<double, double>(S.coef64, S.xsol64, n, ic, ii, jj, kk, M, N, K, S.cxx, S.cyy);
-      S.res64[ic] = r;
-      S.kr0[ic] = (T)r;
-      v[0] += r * r;
-      v[1] += b * b;
-    }
-  }
-  double out[2];
-  block_sum_t<2, double>(v, out);
-  finish_reduce<2>(S, out, [] __device__(const Dev<T>& S2, double* a) {
+struct FinRes {
+  __device__ void operator()(const Dev<T>& S2, double* a) const {
     DevScal* sc = S2.sc;
     if (kFirst) {
       sc->ir_count = 0;
@@ -286,7 +271,95 @@ __global__ void __launch_bounds__(256) k_res64(Dev<T> S) {
     }
     sc->ir_go = go;
     set_cond(S2, S2.h_ir, go != 0);
-  });
+  }
+};
+template <class T>
+struct FinInit {
+  __device__ void operator()(const Dev<T>& S2, double* a) const {
+    DevScal* sc = S2.sc;
+    sc->rho = a[0];
+    sc->red[0] = sqrt(a[0]);
+    sc->alpha = 1.0;
+    sc->omega = 1.0;
+    sc->beta = 0.0;
+    sc->it = 0;
+    sc->relres = 1.0;
+    sc->conv = (a[0] == 0.0) ? 1 : 0;
+    set_cond(S2, S2.h_inner, sc->conv == 0);
+  }
+};
+template <class T>
+struct FinV {
+  __device__ void operator()(const Dev<T>& S2, double* a) const {
+    DevScal* sc = S2.sc;
+    if (a[0] == 0.0 || !(a[0] == a[0])) { sc->conv = 2; return; }
+    sc->alpha = sc->rho / a[0];
+  }
+};
+template <class T>
+struct FinT {
+  __device__ void operator()(const Dev<T>& S2, double* a) const {
+    DevScal* sc = S2.sc;
+    sc->omega = a[1] > 0.0 ? a[0] / a[1] : 0.0;
+  }
+};
+template <class T>
+struct FinXr {
+  __device__ void operator()(const Dev<T>& S2, double* a) const {
+    DevScal* sc = S2.sc;
+    const double tol_in = sc->tol_in;
+    const int itmax_in = sc->itmax_in;
+    sc->it = sc->it + 1;
+    sc->total_it = sc->total_it + 1;
+    sc->inner_total = sc->inner_total + 1;
+    const double rel = sc->red[0] > 0.0 ? sqrt(a[1]) / sc->red[0] : 0.0;
+    sc->relres = rel;
+    int conv = 0;
+    if (!(rel == rel)) conv = 5;
+    else if (rel <= tol_in) conv = 1;
+    else if (sc->it >= itmax_in) conv = 4;
+    else if (a[0] == 0.0 || sc->omega == 0.0) conv = 2;
+    else {
+      sc->beta = (a[0] / sc->rho) * (sc->alpha / sc->omega);
+      sc->rho = a[0];
+    }
+    sc->conv = conv;
+    set_cond(S2, S2.h_inner, conv == 0);
+  }
+};
+
+// r64 = b - A64 x64; inner right-hand side rT = (T) r64; ||r64||, ||b||.
+// The last block then makes the refinement decision of the outer loop (the
+// HYPRE stopping test ||r||/||b|| <= TOL, src/pressure.F:225-258 calls the
+// solver with TOL and ITMAX): stop on convergence, on b = 0 (the solution is
+// then x = 0), on a non-finite residual or an inner breakdown flagged as NaN,
+// or when ITMAX inner iterations or the sweep cap are used up; otherwise it
+// sets the next inner tolerance and iteration budget.  kFirst opens a solve.
+template <class T, bool kFirst>
+__global__ void __launch_bounds__(256) k_res64(Dev<T> S) {
+  // a step held back by k_dt_finalize: the loop conditions keep their
+  // launch default (0), so no sweep runs
+  if (gated_off(S)) return;
+  const int M = S.M, N = S.N, K = S.K;
+  const size_t n = (size_t)S.neq;
+  double v[2] = {0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < kCPT; ++q) {
+    const int ic = (blockIdx.x * kCPT + q) * blockDim.x + threadIdx.x;
+    if (ic < S.neq) {
+      int ii, jj, kk;
+      decode(ic, M, N, ii, jj, kk);
+      const double b = S.rhs64[ic];
+      const double r = b - spmv_c<double, double>(S.coef64, S.xsol64, n, ic, ii, jj, kk, M, N, K, S.cxx, S.cyy);
+      S.res64[ic] = r;
+      S.kr0[ic] = (T)r;
+      v[0] += r * r;
+      v[1] += b * b;
+    }
+  }
+  double out[2];
+  block_sum_t<2, double>(v, out);
+  finish_reduce<2>(S, out, FinRes<T, kFirst>{});
 }
 
 // start of an inner solve from c = 0: r = r0 = rT, p = v = 0, rho = (r, r)
@@ -313,18 +386,7 @@ __global__ void __launch_bounds__(256) k_bicg_init(Dev<T> S) {
   }
   double out[1];
   block_sum_t<1, A>(v, out);
-  finish_reduce<1>(S, out, [] __device__(const Dev<T>& S2, double* a) {
-    DevScal* sc = S2.sc;
-    sc->rho = a[0];
-    sc->red[0] = sqrt(a[0]);
-    sc->alpha = 1.0;
-    sc->omega = 1.0;
-    sc->beta = 0.0;
-    sc->it = 0;
-    sc->relres = 1.0;
-    sc->conv = (a[0] == 0.0) ? 1 : 0;
-    set_cond(S2, S2.h_inner, sc->conv == 0);
-  });
+  finish_reduce<1>(S, out, FinInit<T>{});
 }
 
 // Thomas sweeps of one column held in registers: dp forward then back-substitution.
@@ -442,11 +504,7 @@ __global__ void __launch_bounds__(256) k_bicg_v(Dev<T> S) {
   }
   double out[1];
   block_sum_t<1, A>(v, out);
-  finish_reduce<1>(S, out, [] __device__(const Dev<T>& S2, double* a) {
-    DevScal* sc = S2.sc;
-    if (a[0] == 0.0 || !(a[0] == a[0])) { sc->conv = 2; return; }
-    sc->alpha = sc->rho / a[0];
-  });
+  finish_reduce<1>(S, out, FinV<T>{});
 }
 
 // t = A sh; omega = (t, s) / (t, t)
@@ -483,10 +541,7 @@ __global__ void __launch_bounds__(256) k_bicg_t(Dev<T> S) {
   }
   double out[2];
   block_sum_t<2, A>(v, out);
-  finish_reduce<2>(S, out, [] __device__(const Dev<T>& S2, double* a) {
-    DevScal* sc = S2.sc;
-    sc->omega = a[1] > 0.0 ? a[0] / a[1] : 0.0;
-  });
+  finish_reduce<2>(S, out, FinT<T>{});
 }
 
 // x += alpha ph + omega sh; r = s - omega t; convergence test.  Ends the
@@ -522,27 +577,7 @@ __global__ void __launch_bounds__(256) k_bicg_xr(Dev<T> S) {
   }
   double out[2];
   block_sum_t<2, A>(v, out);
-  finish_reduce<2>(S, out, [] __device__(const Dev<T>& S2, double* a) {
-    DevScal* sc = S2.sc;
-    const double tol_in = sc->tol_in;
-    const int itmax_in = sc->itmax_in;
-    sc->it = sc->it + 1;
-    sc->total_it = sc->total_it + 1;
-    sc->inner_total = sc->inner_total + 1;
-    const double rel = sc->red[0] > 0.0 ? sqrt(a[1]) / sc->red[0] : 0.0;
-    sc->relres = rel;
-    int conv = 0;
-    if (!(rel == rel)) conv = 5;
-    else if (rel <= tol_in) conv = 1;
-    else if (sc->it >= itmax_in) conv = 4;
-    else if (a[0] == 0.0 || sc->omega == 0.0) conv = 2;
-    else {
-      sc->beta = (a[0] / sc->rho) * (sc->alpha / sc->omega);
-      sc->rho = a[0];
-    }
-    sc->conv = conv;
-    set_cond(S2, S2.h_inner, conv == 0);
-  });
+  finish_reduce<2>(S, out, FinXr<T>{});
 }
 
 // x64 += c
@@ -550,6 +585,170 @@ template <class T>
 __global__ void __launch_bounds__(256) k_xupd(Dev<T> S) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < S.neq) S.xsol64[t] = S.xsol64[t] + (double)S.kx[t];
+}
+
+// ------------------------------------------------ the same on small grids
+// On a grid of few blocks -- 256 x 8 x 10 cells are 10 blocks of 256 threads
+// and kCPT cells a thread -- the reducing kernels above use as many of the 152
+// SMs and take their cells one after the other.  Here a cluster of kSlices
+// blocks does one such block's work: each takes a slice of every thread's
+// cells, keeps the values that the sums need in shared memory, and the
+// cluster's first block adds them from there in the order of the kernel above,
+// so that vectors and sums are the same bit for bit.  Used up to kSlicedBlocks
+// blocks: beyond, the kernels above fill the SMs by themselves.
+constexpr int kSlices = kCPT;        // a portable cluster; kCPT cells a thread, one a slice
+constexpr int kSlicedBlocks = 152;
+constexpr int kSliceLevels = (64 + kSlices - 1) / kSlices;   // levels of a column chunk a slice (K <= 64)
+
+// Sum of what `add(q, tid)` accumulates, q = 0 .. n-1 in order, by the
+// cluster's first block; the others leave after it has read their values.
+template <int NV, class A, class T, class Add, class Fin>
+__device__ __forceinline__ void sliced_reduce(const Dev<T>& S, int blk, int nblk, int n, Add add, Fin fin) {
+  auto cl = cooperative_groups::this_cluster();
+  cl.sync();
+  A v[NV];
+  for (int q = 0; q < NV; ++q) v[q] = (A)0;
+  const bool first = cl.block_rank() == 0;
+  if (first)
+    for (int q = 0; q < n; ++q) add(q, v);
+  cl.sync();
+  if (!first) return;
+  double out[NV];
+  block_sum_t<NV, A>(v, out);
+  finish_reduce_of<NV>(S, S.partials, 8, blk, nblk, out, fin);
+}
+
+template <class T, bool kFirst>
+__global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_res64_sl(Dev<T> S) {
+  if (gated_off(S)) return;
+  __shared__ double sr[256], sb[256];
+  auto cl = cooperative_groups::this_cluster();
+  const int blk = blockIdx.x / kSlices, q0 = (int)cl.block_rank(), tid = threadIdx.x;
+  const int base = blk * kCPT * 256 + tid, ic = base + q0 * 256;
+  if (ic < S.neq) {
+    int ii, jj, kk;
+    decode(ic, S.M, S.N, ii, jj, kk);
+    const double b = S.rhs64[ic];
+    const double r = b - spmv_c<double, double>(S.coef64, S.xsol64, (size_t)S.neq, ic, ii, jj, kk, S.M, S.N, S.K,
+                                                S.cxx, S.cyy);
+    S.res64[ic] = r;
+    S.kr0[ic] = (T)r;
+    sr[tid] = r;
+    sb[tid] = b;
+  }
+  sliced_reduce<2, double>(S, blk, gridDim.x / kSlices, kCPT, [&](int q, double (&v)[2]) {
+    if (base + q * 256 < S.neq) {
+      const double r = cl.map_shared_rank(sr, q)[tid], b = cl.map_shared_rank(sb, q)[tid];
+      v[0] += r * r;
+      v[1] += b * b;
+    }
+  }, FinRes<T, kFirst>{});
+}
+
+template <class T>
+__global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_init_sl(Dev<T> S) {
+  using A = typename Acc<T>::type;
+  auto cl = cooperative_groups::this_cluster();
+  const int blk = blockIdx.x / kSlices, tid = threadIdx.x;
+  const int base = blk * kCPT * 256 + tid, ic = base + (int)cl.block_rank() * 256;
+  if (ic < S.neq) {
+    S.kr[ic] = S.kr0[ic];
+    S.kx[ic] = (T)0;
+    if (S.kq) {
+      S.kq[ic] = (T)0;
+    } else {
+      S.kp[ic] = (T)0;
+      S.kv[ic] = (T)0;
+    }
+  }
+  sliced_reduce<1, A>(S, blk, gridDim.x / kSlices, kCPT, [&](int q, A (&v)[1]) {
+    if (base + q * 256 < S.neq) {
+      const T r = S.kr0[base + q * 256];
+      v[0] += (A)r * (A)r;
+    }
+  }, FinInit<T>{});
+}
+
+// y = A x over a block's cells, in slices: y of this thread's cells goes to
+// out and to ys; sum(ic, y, v) then adds them in the order of the kernel above
+template <int NV, class T, class Sum, class Fin>
+__device__ __forceinline__ void sliced_matvec(const Dev<T>& S, const T* __restrict__ x, T* __restrict__ out, Sum sum,
+                                              Fin fin) {
+  using A = typename Acc<T>::type;
+  __shared__ T ys[kColumnWalk<T> ? kSliceLevels : 1][256];
+  auto cl = cooperative_groups::this_cluster();
+  const int blk = blockIdx.x / kSlices, nblk = gridDim.x / kSlices, rank = (int)cl.block_rank(), tid = threadIdx.x;
+  const size_t n = (size_t)S.neq;
+  if constexpr (kColumnWalk<T>) {
+    const int MN = S.M * S.N, t = blk * 256 + tid;
+    const bool in = t < MN * S.col_chunks;
+    const int col = t % MN, k0 = (t / MN) * S.col_kc, k1 = in ? min(S.K, k0 + S.col_kc) : k0;
+    const int per = (S.col_kc + kSlices - 1) / kSlices, ka = k0 + rank * per, kb = min(k1, ka + per);
+    spmv_levels<T, T>(S.coefT, x, n, col, ka, kb, S.M, S.N, S.K, (T)S.cxx, (T)S.cyy, [&](int ic, T y) {
+      out[ic] = y;
+      ys[(ic - col) / MN - ka][tid] = y;
+    });
+    sliced_reduce<NV, A>(S, blk, nblk, max(k1 - k0, 0), [&](int l, A (&v)[NV]) {
+      sum(col + MN * (k0 + l), cl.map_shared_rank(&ys[l % per][0], l / per)[tid], v);
+    }, fin);
+  } else {
+    const int base = blk * kCPT * 256 + tid, ic = base + rank * 256;
+    if (ic < S.neq) {
+      int ii, jj, kk;
+      decode(ic, S.M, S.N, ii, jj, kk);
+      const T y = spmv_c<T, T>(S.coefT, x, n, ic, ii, jj, kk, S.M, S.N, S.K, (T)S.cxx, (T)S.cyy);
+      out[ic] = y;
+      ys[0][tid] = y;
+    }
+    sliced_reduce<NV, A>(S, blk, nblk, kCPT, [&](int q, A (&v)[NV]) {
+      if (base + q * 256 < S.neq) sum(base + q * 256, cl.map_shared_rank(&ys[0][0], q)[tid], v);
+    }, fin);
+  }
+}
+template <class T>
+__global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_v_sl(Dev<T> S) {
+  if (S.sc->conv) return;
+  using A = typename Acc<T>::type;
+  const T* __restrict__ r0 = S.kr0;
+  sliced_matvec<1>(S, S.kph, S.kv, [&](int ic, T y, A (&v)[1]) { v[0] += (A)r0[ic] * (A)y; }, FinV<T>{});
+}
+template <class T>
+__global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_t_sl(Dev<T> S) {
+  if (S.sc->conv) return;
+  using A = typename Acc<T>::type;
+  const T* __restrict__ ss = S.ks;
+  sliced_matvec<2>(S, S.ksh, S.kt, [&](int ic, T y, A (&v)[2]) {
+    v[0] += (A)y * (A)ss[ic];
+    v[1] += (A)y * (A)y;
+  }, FinT<T>{});
+}
+template <class T>
+__global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_xr_sl(Dev<T> S) {
+  if (S.sc->conv) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) set_cond(S, S.h_inner, false);
+    return;
+  }
+  using A = typename Acc<T>::type;
+  __shared__ T sr[256];
+  auto cl = cooperative_groups::this_cluster();
+  const int blk = blockIdx.x / kSlices, tid = threadIdx.x;
+  const int base = blk * kCPT * 256 + tid, ic = base + (int)cl.block_rank() * 256;
+  const T alpha = (T)S.sc->alpha, omega = (T)S.sc->omega;
+  if (ic < S.neq) {
+    S.kx[ic] = S.kx[ic] + alpha * S.kph[ic] + omega * S.ksh[ic];
+    const T r = S.ks[ic] - omega * S.kt[ic];
+    S.kr[ic] = r;
+    if (S.kq) S.kq[ic] = S.kp[ic] - omega * S.kv[ic];
+    sr[tid] = r;
+  }
+  const T* __restrict__ r0 = S.kr0;
+  sliced_reduce<2, A>(S, blk, gridDim.x / kSlices, kCPT, [&](int q, A (&v)[2]) {
+    if (base + q * 256 < S.neq) {
+      const T r = cl.map_shared_rank(sr, q)[tid];
+      v[0] += (A)r0[base + q * 256] * (A)r;
+      v[1] += (A)r * (A)r;
+    }
+  }, FinXr<T>{});
 }
 
 // ------------------------------------------------------------------ GMRES

@@ -542,16 +542,34 @@ class Solver final : public SolverBase {
   static long long dbits(double x) { long long b; std::memcpy(&b, &x, 8); return b; }
 
   // ---------------------------------------------------------------- launchers
+  // Threads of a block of independent items: 256, and fewer on small grids so
+  // that their blocks reach all 152 SMs -- 2048 columns in blocks of 256 run
+  // on 8 of them, each with one SM's FP64 pipe for all its columns (GB300,
+  // 256 x 8 x 10 FP64, by block: vel_bc_b 52 -> @V us with 32)
+  static int block_of(long long n) {
+    int b = 256;
+    while (b > 32 && n < 152LL * 2 * b) b /= 2;
+    return b;
+  }
   template <class Op> void allcols(Op op) {
-    L(Op::kName, [&] { k_allcols<T, Op><<<cdiv((long long)S.Mloc * S.Nloc, 256), 256, 0, st>>>(S, op); });
+    const long long n = (long long)S.Mloc * S.Nloc;
+    const int b = block_of(n);
+    L(Op::kName, [&] { k_allcols<T, Op><<<cdiv(n, b), b, 0, st>>>(S, op); });
   }
   template <class Op> void incols(Op op) {
-    L(Op::kName, [&] { k_incols<T, Op><<<cdiv((long long)S.M * S.N, 256), 256, 0, st>>>(S, op); });
+    const long long n = (long long)S.M * S.N;
+    const int b = block_of(n);
+    L(Op::kName, [&] { k_incols<T, Op><<<cdiv(n, b), b, 0, st>>>(S, op); });
   }
   template <class Op> void box(Op op, int nx, int ny, int nz, int ox, int oy, int oz) {
-    L(Op::kName, [&] {
-      k_box<T, Op><<<cdiv((long long)nx * ny * nz, 256), 256, 0, st>>>(S, op, nx, ny, nz, ox, oy, oz);
-    });
+    const long long n = (long long)nx * ny * nz;
+    const int b = block_of(n);
+    L(Op::kName, [&] { k_box<T, Op><<<cdiv(n, b), b, 0, st>>>(S, op, nx, ny, nz, ox, oy, oz); });
+  }
+  void dt_min() {
+    const long long n = (long long)S.M * S.N;
+    const int b = block_of(n);
+    L("dt_min", [&] { k_dt_min<T><<<cdiv(n, b), b, 0, st>>>(S); });
   }
   template <class Op> void cells(Op op) { box(op, S.M, S.N, S.K, S.IB, S.JB, S.KB); }
   unsigned red_blocks() const { return cdiv(S.neq, 256 * kCPT); }
@@ -759,7 +777,7 @@ class Solver final : public SolverBase {
     return NHW_OK;
   }
   void ens_prefix() {   // estimate_dt (gated), bathymetry, mask, update_vars
-    L("dt_min", [&] { k_dt_min<T><<<cdiv((long long)S.M * S.N, 256), 256, 0, st>>>(S); });
+    dt_min();
     L("dt_finalize", [&] { k_dt_finalize<T><<<1, 1, 0, st>>>(S, 1); });
     if (S.slide) update_bathymetry();
     update_wave_bc();
@@ -935,7 +953,7 @@ class Solver final : public SolverBase {
 
   // -------------------------------------------------- reference subroutines
   int estimate_dt() override {
-    L("dt_min", [&] { k_dt_min<T><<<cdiv((long long)S.M * S.N, 256), 256, 0, st>>>(S); });
+    dt_min();
     L("dt_finalize", [&] { k_dt_finalize<T><<<1, 1, 0, st>>>(S, 0); });
     int rc = pull_scalars();
     if (rc) return rc;
@@ -1066,10 +1084,11 @@ class Solver final : public SolverBase {
       for (size_t l = 1; l < mg.size(); ++l) {
         MGL<T> f = mg[l - 1];
         MGL<T>& c = mg[l];
+        const int bg = block_of(c.n), bf = block_of((long long)c.M * c.N);
         L("mg_galerkin", [&] {
-          k_mg_galerkin<T><<<cdiv(c.n, 256), 256, 0, st>>>(f, (T*)c.coef, (T*)c.cxr, (T*)c.cyr, c.M, c.N);
+          k_mg_galerkin<T><<<cdiv(c.n, bg), bg, 0, st>>>(f, (T*)c.coef, (T*)c.cxr, (T*)c.cyr, c.M, c.N);
         });
-        L("mg_factor", [&] { k_mg_factor<T><<<cdiv((long long)c.M * c.N, 256), 256, 0, st>>>(c, (T*)c.lcp, (T*)c.linv); });
+        L("mg_factor", [&] { k_mg_factor<T><<<cdiv((long long)c.M * c.N, bf), bf, 0, st>>>(c, (T*)c.lcp, (T*)c.linv); });
       }
       cudaEventRecord(ev_join, st);
       st = main_st;
@@ -1119,18 +1138,18 @@ class Solver final : public SolverBase {
       // device-side loops: refinement sweeps around BiCGSTAB iterations
       S.h_ir = new_handle();      // before the kernels that set them are captured
       S.h_inner = new_handle();
-      L("res64", [&] { k_res64<T, true><<<red_blocks(), 256, 0, st>>>(S); });
+      residual<true>();
       join_mg();
       cond_node(S.h_ir, cudaGraphCondTypeWhile, [&] {
         inner_init();
         cond_node(S.h_inner, cudaGraphCondTypeWhile, [&] { one_iteration(); }, 2);
         inner_finish();
-        L("res64", [&] { k_res64<T, false><<<red_blocks(), 256, 0, st>>>(S); });
+        residual<false>();
       }, 1);
       return NHW_OK;
     }
     // host-driven loops over the same device-side decisions
-    L("res64", [&] { k_res64<T, true><<<red_blocks(), 256, 0, st>>>(S); });
+    residual<true>();
     join_mg();
     int rc = pull_scalars();
     if (rc) return rc;
@@ -1146,17 +1165,30 @@ class Solver final : public SolverBase {
         if (chunk < 16) chunk *= 2;
       }
       inner_finish();
-      L("res64", [&] { k_res64<T, false><<<red_blocks(), 256, 0, st>>>(S); });
+      residual<false>();
       rc = pull_scalars();
       if (rc) return rc;
     }
     rc = check();
     return rc ? rc : h_sc->pstat;
   }
+  // the reducing Krylov kernels in slices (krylov.cuh) while their blocks are
+  // fewer than the SMs
+  bool sliced() const { return red_blocks() <= (unsigned)kSlicedBlocks; }
+  template <bool kFirst>
+  void residual() {
+    L("res64", [&] {
+      if (sliced()) k_res64_sl<T, kFirst><<<red_blocks() * kSlices, 256, 0, st>>>(S);
+      else k_res64<T, kFirst><<<red_blocks(), 256, 0, st>>>(S);
+    });
+  }
   // start and end of one inner solve (one refinement sweep)
   void inner_init() {
     if (use_gmres) L("gm_init", [&] { k_gm_init<T><<<red_blocks(), 256, 0, st>>>(S); });
-    else L("bicg_init", [&] { k_bicg_init<T><<<red_blocks(), 256, 0, st>>>(S); });
+    else L("bicg_init", [&] {
+      if (sliced()) k_bicg_init_sl<T><<<red_blocks() * kSlices, 256, 0, st>>>(S);
+      else k_bicg_init<T><<<red_blocks(), 256, 0, st>>>(S);
+    });
   }
   void inner_finish() {
     if (use_gmres) L("x_update", [&] { k_gm_xupd<T><<<cdiv(S.neq, 256), 256, 0, st>>>(S); });
@@ -1205,14 +1237,23 @@ class Solver final : public SolverBase {
     } else {
       L("bicg_p", [&] { k_bicg_p<T><<<cb, 128, 0, st>>>(S); });
     }
-    L("bicg_v", [&] { k_bicg_v<T><<<matvec_blocks(), 256, 0, st>>>(S); });
+    L("bicg_v", [&] {
+      if (sliced()) k_bicg_v_sl<T><<<matvec_blocks() * kSlices, 256, 0, st>>>(S);
+      else k_bicg_v<T><<<matvec_blocks(), 256, 0, st>>>(S);
+    });
     if (use_mg) {
       vcycle(S.ks, S.ksh, 2);   // s likewise
     } else {
       L("bicg_s", [&] { k_bicg_s<T><<<cb, 128, 0, st>>>(S); });
     }
-    L("bicg_t", [&] { k_bicg_t<T><<<matvec_blocks(), 256, 0, st>>>(S); });
-    L("bicg_xr", [&] { k_bicg_xr<T><<<red_blocks(), 256, 0, st>>>(S); });
+    L("bicg_t", [&] {
+      if (sliced()) k_bicg_t_sl<T><<<matvec_blocks() * kSlices, 256, 0, st>>>(S);
+      else k_bicg_t<T><<<matvec_blocks(), 256, 0, st>>>(S);
+    });
+    L("bicg_xr", [&] {
+      if (sliced()) k_bicg_xr_sl<T><<<red_blocks() * kSlices, 256, 0, st>>>(S);
+      else k_bicg_xr<T><<<red_blocks(), 256, 0, st>>>(S);
+    });
   }
   // multigrid V-cycle: x ~= A^-1 b on level 0
   int cta_columns = 64;    // levels up to this many columns run in one block (mg_cta_columns)
@@ -1610,7 +1651,7 @@ class Solver final : public SolverBase {
     S.h_go = use_persistent ? 0 : new_handle();
     if (cap_ok(cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
                "step capture")) {
-      L("dt_min", [&] { k_dt_min<T><<<cdiv((long long)S.M * S.N, 256), 256, 0, st>>>(S); });
+      dt_min();
       L("dt_finalize", [&] { k_dt_finalize<T><<<1, 1, 0, st>>>(S, gated); });
       if (use_persistent)
         step_body();   // every kernel checks sc->step_go; no loops left on the host side
