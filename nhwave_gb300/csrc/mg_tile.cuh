@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(1024) k_mg_up(MGL<T> L, Prolong<T> P, int ntil
 // load latencies (three visits, one restriction through global memory) and by
 // the chains of its nine line solves, 2 x 20 dependent levels each.
 // Slots are numbered over the level's own columns, q = jj * Mh + ii / 2.
-constexpr int kCycleSlots = 32;   // one warp a level
+constexpr int kCycleSlots = 32;
 constexpr int kCycleColumns = 2 * kCycleSlots;
 template <class T>
 __host__ __device__ inline int cycle_slots(const MGL<T>& L) { return ((L.M + 1) >> 1) * L.N; }
@@ -461,39 +461,45 @@ __host__ __device__ constexpr size_t cycle_smem(int K) {
   return sizeof(T) * ((size_t)kCycleSlots * (2 * (K + 2) + 3 * K) + (size_t)kCycleColumns * K);
 }
 
-// a thread's columns of one level, LPT levels each, with their operator
+// A thread's cells of one level (LPT of each colour) with their operator.  The
+// cells of a colour are dealt to the threads densely, cell = level * slots +
+// slot: the coarsest level of 8 slots fills 3 warps of 20 levels, not 20, and
+// an FP64 instruction holds the SM's pipe for 16 cycles whatever its lanes do.
 template <class T, int LPT>
 struct CycleLevel {
   T g[2][LPT][8], b[2][LPT], a[2][LPT], v[2][LPT], p[2][LPT];
-  int w[2], e[2], s[2], n[2], ii[2], jj, col[2];
-  bool in[2];
-  __device__ __forceinline__ void load(const MGL<T>& L, int q, int ty, int by) {
+  int w[2][LPT], e[2][LPT], s[2][LPT], n[2][LPT], ii[2][LPT], jj[LPT], col[2][LPT], q[LPT], k[LPT], ns;
+  bool in[2][LPT];
+  __device__ __forceinline__ void load(const MGL<T>& L, int tid, int nt) {
     const int K = L.K, M = L.M, N = L.N, MN = M * N, Mh = (M + 1) >> 1;
     const size_t n0 = (size_t)L.n;
-    jj = q / Mh;
+    ns = Mh * N;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int o = (c + jj) & 1;
-      ii[c] = 2 * (q - jj * Mh) + o;
-      in[c] = jj < N && ii[c] < M;
-      col[c] = ii[c] + M * jj;
-      // offsets of the neighbours' slots; 0, with a zero coupling, where there is none
-      const bool im = ii[c] > 0, ip = ii[c] < M - 1, jm = jj > 0, jp = jj < N - 1;
-      w[c] = in[c] && im ? o - 1 : 0;
-      e[c] = in[c] && ip ? o : 0;
-      s[c] = in[c] && jm ? -Mh : 0;
-      n[c] = in[c] && jp ? Mh : 0;
+    for (int t = 0; t < LPT; ++t) {
+      const int cell = tid + t * nt;
+      k[t] = cell / ns;
+      q[t] = cell - k[t] * ns;
+      jj[t] = q[t] / Mh;
 #pragma unroll
-      for (int t = 0; t < LPT; ++t) {
-        const int k = ty + t * by;
+      for (int c = 0; c < 2; ++c) {
+        const int o = (c + jj[t]) & 1;
+        ii[c][t] = 2 * (q[t] - jj[t] * Mh) + o;
+        in[c][t] = k[t] < K && ii[c][t] < M;
+        col[c][t] = ii[c][t] + M * jj[t];
+        // offsets of the neighbours' slots; 0, with a zero coupling, where there is none
+        const bool im = ii[c][t] > 0, ip = ii[c][t] < M - 1, jm = jj[t] > 0, jp = jj[t] < N - 1;
+        w[c][t] = in[c][t] && im ? o - 1 : 0;
+        e[c][t] = in[c][t] && ip ? o : 0;
+        s[c][t] = in[c][t] && jm ? -Mh : 0;
+        n[c][t] = in[c][t] && jp ? Mh : 0;
         b[c][t] = a[c][t] = v[c][t] = p[c][t] = (T)0;
 #pragma unroll
         for (int m = 0; m < 8; ++m) g[c][t][m] = (T)0;
-        if (in[c] && k < K) {
-          const int ic = col[c] + MN * k;
+        if (in[c][t]) {
+          const int ic = col[c][t] + MN * k[t];
           const T* cf = L.coef + ic;
           b[c][t] = L.b[ic];
-          a[c][t] = k > 0 ? cf[2 * n0] : (T)0;
+          a[c][t] = k[t] > 0 ? cf[2 * n0] : (T)0;
           v[c][t] = L.linv[ic];
           p[c][t] = L.lcp[ic];
           if (ip) { g[c][t][0] = cx_p(L, ic); g[c][t][4] = cf[5 * n0]; }
@@ -512,26 +518,39 @@ struct CycleBlock {
   T* x[2];    // [K + 2][NS] of each colour
   T* f;       // line factors of the colour being solved, [3][K][NS]
   T* xc;      // solution of the level below, [K][columns]
-  int K, q, ty, by;
-  // one half-sweep; x of the other colour as it stands
+  int K, tid, nt;
+  // one half-sweep; x of the other colour as it stands, or zero
   template <bool kByColumn>
-  __device__ __forceinline__ void sweep(const CycleLevel<T, LPT>& V, int c) {
+  __device__ __forceinline__ void sweep(const CycleLevel<T, LPT>& V, const MGL<T>& L, int c, bool zero = false) {
 #pragma unroll
-    for (int t = 0; t < LPT; ++t) {
-      const int k = ty + t * by;
-      if (V.in[c] && k < K) {
-        const T* y = x[1 - c] + (k + 1) * NS + q;
-        x[c][(k + 1) * NS + q] = V.b[c][t] - tile_off<kByColumn>(V.g[c][t], y, y + NS, y - NS, V.w[c], V.e[c], V.s[c], V.n[c]);
-        f[k * NS + q] = V.a[c][t]; f[(K + k) * NS + q] = V.v[c][t]; f[(2 * K + k) * NS + q] = V.p[c][t];
+    for (int t = 0; t < LPT; ++t)
+      if (V.in[c][t]) {
+        const int r = V.k[t] * NS + V.q[t];
+        const T* y = x[1 - c] + r + NS;
+        T off = (T)0;
+        if (!zero) off = tile_off<kByColumn>(V.g[c][t], y, y + NS, y - NS, V.w[c][t], V.e[c][t], V.s[c][t], V.n[c][t]);
+        x[c][r + NS] = V.b[c][t] - off;
+        f[r] = V.a[c][t]; f[K * NS + r] = V.v[c][t]; f[2 * K * NS + r] = V.p[c][t];
       }
-    }
     __syncthreads();
-    if (ty == 0 && V.in[c]) line_solve_smem<NS>(x[c] + NS + q, f + q, f + K * NS + q, f + 2 * K * NS + q, K);
+    if (tid < V.ns) {   // a slot without a column (an odd row's end) solves zeros
+      const int Mh = (L.M + 1) >> 1, jj = tid / Mh;
+      if (2 * (tid - jj * Mh) + ((c + jj) & 1) < L.M)
+        line_solve_smem<NS>(x[c] + NS + tid, f + tid, f + K * NS + tid, f + 2 * K * NS + tid, K);
+    }
     __syncthreads();
   }
   // x = 0 at the slots of both colours
   __device__ __forceinline__ void clear() {
-    for (int k = ty; k < K + 2; k += by) x[0][k * NS + q] = x[1][k * NS + q] = (T)0;
+    for (int r = tid; r < (K + 2) * NS; r += nt) x[0][r] = x[1][r] = (T)0;
+  }
+  // x of the level, in the natural layout
+  __device__ __forceinline__ void store(const CycleLevel<T, LPT>& V, T* out, int MN) const {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int t = 0; t < LPT; ++t)
+        if (V.in[c][t]) out[V.col[c][t] + MN * V.k[t]] = x[c][(V.k[t] + 1) * NS + V.q[t]];
   }
 };
 
@@ -542,70 +561,51 @@ __global__ void __launch_bounds__(640, 1) k_mg_cycle(MGSet<T> set, int nl, const
   const int stopped = sc->conv;
   CycleBlock<T, LPT> B;
   const int K = B.K = set.L[0].K;
-  B.q = threadIdx.x; B.ty = threadIdx.y; B.by = blockDim.y;
+  const int tid = B.tid = threadIdx.x, nt = B.nt = blockDim.x;
   B.x[0] = reinterpret_cast<T*>(smem_raw);
   B.x[1] = B.x[0] + (K + 2) * NS;
   B.f = B.x[1] + (K + 2) * NS;
   B.xc = B.f + 3 * K * NS;
-  const int q = B.q, ty = B.ty, by = B.by;
   CycleLevel<T, LPT> V;
-  V.load(set.L[0], q, ty, by);
+  V.load(set.L[0], tid, nt);
   if (stopped) return;
   for (int l = 0; l < nl - 1; ++l) {
     const MGL<T>& F = set.L[l];
-    const MGL<T>& C = set.L[l + 1];
-    const int MN = F.M * F.N;
-    if (l > 0) V.load(F, q, ty, by);
+    if (l > 0) V.load(F, tid, nt);
     B.clear();
     __syncthreads();
-    B.template sweep<false>(V, 0);
-    B.template sweep<false>(V, 1);
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-      for (int t = 0; t < LPT; ++t) {
-        const int k = ty + t * by;
-        if (V.in[c] && k < K) F.x[V.col[c] + MN * k] = B.x[c][(k + 1) * NS + q];
-      }
+    B.template sweep<false>(V, F, 0, true);
+    B.template sweep<false>(V, F, 1);
+    B.store(V, F.x, F.M * F.N);
     __syncthreads();
-    cta_restrict(F, C);
+    cta_restrict(F, set.L[l + 1]);
   }
-  if (nl > 1) V.load(set.L[nl - 1], q, ty, by);
+  if (nl > 1) V.load(set.L[nl - 1], tid, nt);
   B.clear();
   __syncthreads();
   for (int s = 0; s < coarse_sweeps; ++s) {
-    B.template sweep<false>(V, 0);
-    B.template sweep<false>(V, 1);
+    B.template sweep<false>(V, set.L[nl - 1], 0, s == 0);
+    B.template sweep<false>(V, set.L[nl - 1], 1);
   }
   for (int l = nl - 2;; --l) {
     // level l + 1 is done: its x to the level above, or out
-    const int MN = set.L[l + 1].M * set.L[l + 1].N;
-    T* out = l < 0 ? set.L[0].x : B.xc;
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-      for (int t = 0; t < LPT; ++t) {
-        const int k = ty + t * by;
-        if (V.in[c] && k < K) out[V.col[c] + MN * k] = B.x[c][(k + 1) * NS + q];
-      }
+    B.store(V, l < 0 ? set.L[0].x : B.xc, set.L[l + 1].M * set.L[l + 1].N);
     if (l < 0) break;
     const MGL<T>& F = set.L[l];
-    V.load(F, q, ty, by);
+    V.load(F, tid, nt);
     __syncthreads();
     B.clear();
     __syncthreads();
     Prolong<T> P = prolong_from(F, set.L[l + 1], w);
     P.xc = B.xc;
-    typename Prolong<T>::Stencil st{};
-    if (V.in[0]) st = P.stencil(V.ii[0], V.jj);
 #pragma unroll
-    for (int t = 0; t < LPT; ++t) {
-      const int k = ty + t * by;
-      if (V.in[0] && k < K) B.x[0][(k + 1) * NS + q] = P.at(F.x, V.col[0] + F.M * F.N * k, st, k);
-    }
+    for (int t = 0; t < LPT; ++t)
+      if (V.in[0][t])
+        B.x[0][(V.k[t] + 1) * NS + V.q[t]] =
+            P.at(F.x, V.col[0][t] + F.M * F.N * V.k[t], P.stencil(V.ii[0][t], V.jj[t]), V.k[t]);
     __syncthreads();
-    B.template sweep<true>(V, 1);
-    B.template sweep<false>(V, 0);
+    B.template sweep<true>(V, F, 1);
+    B.template sweep<false>(V, F, 0);
   }
 }
 

@@ -545,7 +545,7 @@ class Solver final : public SolverBase {
   // Threads of a block of independent items: 256, and fewer on small grids so
   // that their blocks reach all 152 SMs -- 2048 columns in blocks of 256 run
   // on 8 of them, each with one SM's FP64 pipe for all its columns (GB300,
-  // 256 x 8 x 10 FP64, by block: vel_bc_b 52 -> @V us with 32)
+  // 256 x 8 x 10 FP64, by block: vel_bc_b 52 -> 34 us with 32)
   static int block_of(long long n) {
     int b = 256;
     while (b > 32 && n < 152LL * 2 * b) b /= 2;
@@ -1343,8 +1343,8 @@ class Solver final : public SolverBase {
   template <int LPT>
   void cycle(const MGSet<T>& set, int cnt) {
     L("mg_coarse_cycle", [&] {
-      k_mg_cycle<T, LPT><<<1, dim3(kCycleSlots, (S.K + LPT - 1) / LPT), cycle_smem<T>(S.K), st>>>(
-          set, cnt, S.sc, mg_w, mg_coarse_sweeps);
+      k_mg_cycle<T, LPT><<<1, kCycleSlots * ((S.K + LPT - 1) / LPT), cycle_smem<T>(S.K), st>>>(set, cnt, S.sc, mg_w,
+                                                                                           mg_coarse_sweeps);
     });
   }
   // fine_in: 0 b as given; 1 b = p formed on the fly; 2 b = s formed on the fly
@@ -1391,8 +1391,8 @@ class Solver final : public SolverBase {
       const int cnt = nl - lc;
       // Levels of up to 32 slots a colour and 40 sigma levels take the form
       // that keeps x and the operator on chip (32 x 2 and 8 x 2 columns, 20
-      // levels: FP32 21.9 -> 15.0 us, FP64 74.6 -> 57.7; 40 levels FP32 36.5
-      // -> 23.7, FP64 140 -> 115); with more slots the FP64 form spills and
+      // levels: FP32 21.9 -> 15.2 us, FP64 74.7 -> 50.2; 40 levels FP32 36.6
+      // -> 25.6, FP64 140 -> 103); with more slots the FP64 form spills and
       // is slower (5 x 12 columns: 76.8 against 82.7 us)
       if (slots <= kCycleSlots && S.K <= 20) cycle<1>(set, cnt);
       else if (slots <= kCycleSlots && S.K <= 40) cycle<2>(set, cnt);
