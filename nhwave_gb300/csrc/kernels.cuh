@@ -720,32 +720,29 @@ struct OpSource {
 //    fluxes: delxyzFun + construction + wave_speed + HLL + flux_bc
 //    (src/nhwave.F:1686-2351, 2354-2552, 2673-2738, 2813-2886)
 // =========================================================================
-// x faces: face f between cells f-1 and f, row j, level k (all interior)
-struct OpFluxX {
+// x faces: face f between cells f-1 and f, row j, over its levels.  load()
+// forms what the levels share, the 2-D state of the face with the wet/dry
+// front fix (src/nhwave.F:1745-1788); level() takes the reconstructed U, V, W,
+// DU, DV, DW on both sides to the HLL / HLLC fluxes with flux_bc.  `low`: this
+// thread's levels hold the lowest one (2-D results are written once).
+template <class T>
+struct FluxXFace {
+  static constexpr int kDir = 0, NF = 6;
   static constexpr const char* kName = "flux_x";
-  template <class T>
-  __device__ void operator()(const Dev<T>& S, int f, int j, int k) const {
-    using R = T;
-    const int c0 = f - 1, c1 = f;
-    const long long e0 = i3(S, c0, j, k), e1 = e0 + 1;
+  using R = T;
+  int f, j, c0, mL, mR;
+  R reL, reR, rh0, rdL, rdR, rdd;
+  double dL, dR, h0;   // FP64 face depths (HLLC) and bed height
+  bool zl, zr;
+  __device__ __forceinline__ static const T* field(const Dev<T>& S, int m) {
+    return m == 0 ? S.U : m == 1 ? S.V : m == 2 ? S.W : m == 3 ? S.DU : m == 4 ? S.DV : S.DW;
+  }
+  __device__ __forceinline__ void load(const Dev<T>& S, int f_, int j_, bool low) {
+    f = f_; j = j_; c0 = f - 1;
     const long long q0 = i2(S, c0, j), q1 = q0 + 1;
-    const int mL = S.Mask[q0], mR = S.Mask[q1];
-    const R hdx = S.hdxT, rdx = S.dxT, irdx = S.idxT;
-    // limited x slopes of the two cells (zero in dry cells)
-    auto sl = [&](const T* A, long long e, int m) -> R {
-      return m == 0 ? (R)0 : lim_slope_u<R>(A[e - 1], A[e], A[e + 1], rdx, irdx);
-    };
-    R uL = S.U[e0] + hdx * sl(S.U, e0, mL), uR = S.U[e1] - hdx * sl(S.U, e1, mR);
-    R vL = S.V[e0] + hdx * sl(S.V, e0, mL), vR = S.V[e1] - hdx * sl(S.V, e1, mR);
-    R wL = S.W[e0] + hdx * sl(S.W, e0, mL), wR = S.W[e1] - hdx * sl(S.W, e1, mR);
-    R duL = S.DU[e0] + hdx * sl(S.DU, e0, mL), duR = S.DU[e1] - hdx * sl(S.DU, e1, mR);
-    R dvL = S.DV[e0] + hdx * sl(S.DV, e0, mL), dvR = S.DV[e1] - hdx * sl(S.DV, e1, mR);
-    R dwL = S.DW[e0] + hdx * sl(S.DW, e0, mL), dwR = S.DW[e1] - hdx * sl(S.DW, e1, mR);
-    // 2-D face state with the wet/dry front fix (src/nhwave.F:1745-1788)
-    R reL, reR, rh0, rdL, rdR, rdd;
-    double dL = 0.0, dR = 0.0, h0;   // FP64 face depths (HLLC) and bed height
-    bool zl, zr;
-    const bool inL = c0 >= S.IB && c0 <= S.IE, inR = c1 >= S.IB && c1 <= S.IE;
+    mL = S.Mask[q0]; mR = S.Mask[q1];
+    dL = dR = 0.0;
+    const bool inL = c0 >= S.IB && c0 <= S.IE, inR = f >= S.IB && f <= S.IE;
     if (face_table<R>(S)) {
       const long long n2 = face_slot(S);
       const T* ft = S.fxT + q1;
@@ -754,10 +751,14 @@ struct OpFluxX {
       face_flags(S, q0, 1, inL, inR, zl, zr);
     } else {
       const Face2D F = face_2d(S, q0, 1, inL, inR, 0.5 * S.dx, S.DelxEta, S.Hfx, S.Hfx0);
-      if (F.wrote_h0 && k == S.KB) S.Hfx0[q1] = F.h0;
+      if (F.wrote_h0 && low) S.Hfx0[q1] = F.h0;
       dL = F.dL; dR = F.dR; h0 = F.h0; zl = F.zl; zr = F.zr;
       reL = (R)F.etaL; reR = (R)F.etaR; rh0 = (R)F.h0; rdL = (R)F.dL; rdR = (R)F.dR; rdd = (R)(F.dR - F.dL);
     }
+  }
+  __device__ __forceinline__ void level(const Dev<T>& S, int k, const R (&l)[6], const R (&r)[6]) const {
+    R uL = l[0], vL = l[1], wL = l[2], duL = l[3], dvL = l[4], dwL = l[5];
+    R uR = r[0], vR = r[1], wR = r[2], duR = r[3], dvR = r[4], dwR = r[5];
     if (zl) uL = vL = wL = duL = dvL = dwL = (R)0;
     if (zr) uR = vR = wR = duR = dvR = dwR = (R)0;
     // physical fluxes at the faces
@@ -838,32 +839,48 @@ struct OpFluxX {
     S.Ex[o] = Ex; S.Fx[o] = Fx; S.Gx[o] = Gx; S.Hx[o] = Hx;
   }
 };
-
-// y faces: face g between cells g-1 and g in column i
-struct OpFluxY {
-  static constexpr const char* kName = "flux_y";
+struct OpFluxX {
+  static constexpr const char* kName = "flux_x";
   template <class T>
-  __device__ void operator()(const Dev<T>& S, int i, int g, int k) const {
+  __device__ void operator()(const Dev<T>& S, int f, int j, int k) const {
     using R = T;
-    const int c0 = g - 1, c1 = g;
-    const long long sy = S.sy;
-    const long long e0 = i3(S, i, c0, k), e1 = e0 + sy;
-    const long long q0 = i2(S, i, c0), q1 = q0 + sy;
-    const int mL = S.Mask[q0], mR = S.Mask[q1];
-    const R hdy = S.hdyT, rdy = S.dyT, irdy = S.idyT;
+    const long long e0 = i3(S, f - 1, j, k), e1 = e0 + 1;
+    const int mL = S.Mask[i2(S, f - 1, j)], mR = S.Mask[i2(S, f, j)];
+    const R hdx = S.hdxT, rdx = S.dxT, irdx = S.idxT;
+    // limited x slopes of the two cells (zero in dry cells)
     auto sl = [&](const T* A, long long e, int m) -> R {
-      return m == 0 ? (R)0 : lim_slope_u<R>(A[e - sy], A[e], A[e + sy], rdy, irdy);
+      return m == 0 ? (R)0 : lim_slope_u<R>(A[e - 1], A[e], A[e + 1], rdx, irdx);
     };
-    R uL = S.U[e0] + hdy * sl(S.U, e0, mL), uR = S.U[e1] - hdy * sl(S.U, e1, mR);
-    R vL = S.V[e0] + hdy * sl(S.V, e0, mL), vR = S.V[e1] - hdy * sl(S.V, e1, mR);
-    R wL = S.W[e0] + hdy * sl(S.W, e0, mL), wR = S.W[e1] - hdy * sl(S.W, e1, mR);
-    R duL = S.DU[e0] + hdy * sl(S.DU, e0, mL), duR = S.DU[e1] - hdy * sl(S.DU, e1, mR);
-    R dvL = S.DV[e0] + hdy * sl(S.DV, e0, mL), dvR = S.DV[e1] - hdy * sl(S.DV, e1, mR);
-    R dwL = S.DW[e0] + hdy * sl(S.DW, e0, mL), dwR = S.DW[e1] - hdy * sl(S.DW, e1, mR);
-    R reL, reR, rh0, rdL, rdR, rdd;
-    double dL = 0.0, dR = 0.0;   // FP64 face depths (HLLC)
-    bool zl, zr;
-    const bool inL = c0 >= S.JB && c0 <= S.JE, inR = c1 >= S.JB && c1 <= S.JE;
+    R l[6], r[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const T* A = FluxXFace<T>::field(S, m);
+      l[m] = A[e0] + hdx * sl(A, e0, mL);
+      r[m] = A[e1] - hdx * sl(A, e1, mR);
+    }
+    FluxXFace<T> F;
+    F.load(S, f, j, k == S.KB);
+    F.level(S, k, l, r);
+  }
+};
+
+// y faces: face g between cells g-1 and g in column i, as FluxXFace
+template <class T>
+struct FluxYFace {
+  static constexpr int kDir = 1, NF = 6;
+  static constexpr const char* kName = "flux_y";
+  using R = T;
+  int i, g, c0, mL, mR;
+  R reL, reR, rh0, rdL, rdR, rdd;
+  double dL, dR;   // FP64 face depths (HLLC)
+  bool zl, zr;
+  __device__ __forceinline__ static const T* field(const Dev<T>& S, int m) { return FluxXFace<T>::field(S, m); }
+  __device__ __forceinline__ void load(const Dev<T>& S, int i_, int g_, bool low) {
+    i = i_; g = g_; c0 = g - 1;
+    const long long sy = S.sy, q0 = i2(S, i, c0), q1 = q0 + sy;
+    mL = S.Mask[q0]; mR = S.Mask[q1];
+    dL = dR = 0.0;
+    const bool inL = c0 >= S.JB && c0 <= S.JE, inR = g >= S.JB && g <= S.JE;
     if (face_table<R>(S)) {
       const long long n2 = face_slot(S);
       const T* ft = S.fyT + q1;
@@ -871,10 +888,14 @@ struct OpFluxY {
       face_flags(S, q0, sy, inL, inR, zl, zr);
     } else {
       const Face2D F = face_2d(S, q0, sy, inL, inR, 0.5 * S.dy, S.DelyEta, S.Hfy, S.Hfy0);
-      if (F.wrote_h0 && k == S.KB) S.Hfy0[q1] = F.h0;
+      if (F.wrote_h0 && low) S.Hfy0[q1] = F.h0;
       dL = F.dL; dR = F.dR; zl = F.zl; zr = F.zr;
       reL = (R)F.etaL; reR = (R)F.etaR; rh0 = (R)F.h0; rdL = (R)F.dL; rdR = (R)F.dR; rdd = (R)(F.dR - F.dL);
     }
+  }
+  __device__ __forceinline__ void level(const Dev<T>& S, int k, const R (&l)[6], const R (&r)[6]) const {
+    R uL = l[0], vL = l[1], wL = l[2], duL = l[3], dvL = l[4], dwL = l[5];
+    R uR = r[0], vR = r[1], wR = r[2], duR = r[3], dvR = r[4], dwR = r[5];
     if (zl) uL = vL = wL = duL = dvL = dwL = (R)0;
     if (zr) uR = vR = wR = duR = dvR = dwR = (R)0;
     const R FyL = rdL * uL * vL, FyR = rdR * uR * vR;
@@ -931,6 +952,30 @@ struct OpFluxY {
     S.Ey[o] = Ey; S.Fy[o] = Fy; S.Gy[o] = Gy; S.Hy[o] = Hy;
   }
 };
+struct OpFluxY {
+  static constexpr const char* kName = "flux_y";
+  template <class T>
+  __device__ void operator()(const Dev<T>& S, int i, int g, int k) const {
+    using R = T;
+    const long long sy = S.sy;
+    const long long e0 = i3(S, i, g - 1, k), e1 = e0 + sy;
+    const int mL = S.Mask[i2(S, i, g - 1)], mR = S.Mask[i2(S, i, g)];
+    const R hdy = S.hdyT, rdy = S.dyT, irdy = S.idyT;
+    auto sl = [&](const T* A, long long e, int m) -> R {
+      return m == 0 ? (R)0 : lim_slope_u<R>(A[e - sy], A[e], A[e + sy], rdy, irdy);
+    };
+    R l[6], r[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const T* A = FluxXFace<T>::field(S, m);
+      l[m] = A[e0] + hdy * sl(A, e0, mL);
+      r[m] = A[e1] - hdy * sl(A, e1, mR);
+    }
+    FluxYFace<T> F;
+    F.load(S, i, g, k == S.KB);
+    F.level(S, k, l, r);
+  }
+};
 
 // z faces k in [KB, KE+1] of an interior column (src/nhwave.F:1998-2023, 2719-2730)
 struct OpFluxZ {
@@ -958,6 +1003,114 @@ struct OpFluxZ {
     S.Hz[o] = (R)0.5 * (om * (wL + wR) - ao * (wR - wL));
   }
 };
+
+// The z fluxes of the FP64 form, a thread walking a chunk of kc faces up a
+// column: each difference quotient serves the two cells it lies between and
+// each limited slope the two faces of its cell, 2 divisions a field and level
+// instead of 6 (the same operands, so the same values bit for bit).
+template <class T>
+__global__ void __launch_bounds__(128) k_flux_z_walk(Dev<T> S, int kc) {
+  if (gated_off(S)) return;
+  using R = T;
+  const int cols = S.M * S.N, t = blockIdx.x * blockDim.x + threadIdx.x, ch = t / cols, col = t - ch * cols;
+  const int k0 = S.KB + ch * kc, k1 = min(S.KE + 1, k0 + kc - 1);
+  if (k0 > S.KE + 1) return;
+  const long long sz = S.sz, o0 = i3(S, S.IB + col % S.M, S.JB + col / S.M, 0);
+  const T* dsc = S.lvT + S.Kloc;       // sigc_k - sigc_k-1
+  const T* hds = S.lvT + 2 * S.Kloc;   // dsig_k / 2
+  // of face k: value, quotient above and left state of the cell below
+  R a[3], q[3], left[3];
+  auto lim = [](R t1, R t2) -> R { return (fabs(t1) + fabs(t2)) < (R)kSmall ? (R)0 : limiter(t1, t2); };
+  const int kb = max(k0, S.KB + 1);   // the bed's and the surface's fluxes are zero
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const T* A = FluxXFace<T>::field(S, m) + o0;
+    const R am = A[sz * (kb - 2)], a0 = A[sz * (kb - 1)];
+    a[m] = A[sz * kb];
+    q[m] = (a[m] - a0) / dsc[kb];
+    left[m] = a0 + hds[kb - 1] * lim(q[m], (a0 - am) / dsc[kb - 1]);
+  }
+  if (k0 == S.KB) { S.Fz[o0 + sz * k0] = (R)0; S.Gz[o0 + sz * k0] = (R)0; S.Hz[o0 + sz * k0] = (R)0; }
+  for (int k = kb; k <= k1; ++k) {
+    const long long o = o0 + sz * k;
+    if (k == S.KE + 1) { S.Fz[o] = (R)0; S.Gz[o] = (R)0; S.Hz[o] = (R)0; break; }
+    const R om = S.Omega[o], ao = fabs(om);
+    R fl[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const R an = FluxXFace<T>::field(S, m)[o + sz], qn = (an - a[m]) / dsc[k + 1];
+      const R half = hds[k] * lim(qn, q[m]), right = a[m] - half;
+      fl[m] = (R)0.5 * (om * (left[m] + right) - ao * (right - left[m]));
+      left[m] = a[m] + half;
+      a[m] = an;
+      q[m] = qn;
+    }
+    S.Fz[o] = fl[0]; S.Gz[o] = fl[1]; S.Hz[o] = fl[2];
+  }
+}
+
+// Faces across x (y) of the FP64 form.  A block has 256 cells of a row (16 rows
+// of 32 cells) and walks kc levels: each cell forms its difference quotients
+// once, takes the lower neighbour's from shared memory for its limited slopes,
+// and hands its upper face's left states to the next cell.  Face by face the
+// same values cost 36 FP64 divisions a face instead of 12, and the face's 2-D
+// state and its square roots are formed once for all levels.  Bound by the
+// FP64 pipe (1024 x 64 x 20: flux_x 1478 -> 874 us, flux_y 1387 -> 832,
+// omega_x 536 -> 309, omega_y 501 -> 293; flux_z, walked, 469 -> 306).
+constexpr int kFaceX = 256, kFaceYx = 32, kFaceYy = 16;
+template <class T, class Face>
+__global__ void __launch_bounds__(Face::kDir == 0 ? kFaceX : kFaceYx * kFaceYy)
+k_faces(Dev<T> S, int kc, int ntile, int nrow) {
+  if (gated_off(S)) return;
+  using R = T;
+  constexpr bool kX = Face::kDir == 0;
+  constexpr int NF = Face::NF, NP = kX ? kFaceX : kFaceYy, NT = kX ? kFaceX : kFaceYx * kFaceYy;
+  __shared__ R sq[NF][NT], sl[NF][NT];
+  const int pos = kX ? threadIdx.x : threadIdx.y;        // along the direction of the faces
+  const int me = threadIdx.x + blockDim.x * threadIdx.y, before = me - (kX ? 1 : kFaceYx);
+  const int b = blockIdx.x, tile = b % ntile, r = b / ntile, row = r % nrow, ch = r / nrow;
+  const int k0 = S.KB + ch * kc, k1 = min(S.KE, k0 + kc - 1);
+  // this thread's cell (its lower face is the thread's face) and cross index
+  const int c = (kX ? S.IB : S.JB) + tile * (NP - 2) - 2 + pos, last = kX ? S.IE + 1 : S.JE + 1;
+  const int x = kX ? S.JB + row : S.IB + row * kFaceYx + threadIdx.x;
+  const bool cell = c <= last && (kX || x <= S.IE), face = cell && pos >= 2;
+  const int i = kX ? c : x, j = kX ? x : c;
+  const long long step = kX ? 1 : S.sy, o0 = i3(S, i, j, 0);
+  const R h = kX ? S.dxT : S.dyT, hd = kX ? S.hdxT : S.hdyT;
+  const bool wet = cell && S.Mask[i2(S, i, j)] != 0;
+  Face F;
+  if (face) F.load(S, i, j, k0 == S.KB);
+  for (int k = k0; k <= k1; ++k) {
+    R a[NF], q[NF], l[NF];
+    if (cell) {
+#pragma unroll
+      for (int m = 0; m < NF; ++m) {
+        const T* A = Face::field(S, m) + o0 + S.sz * k;
+        a[m] = A[0];
+        q[m] = (A[step] - a[m]) / h;
+        sq[m][me] = q[m];
+      }
+    }
+    __syncthreads();
+    if (cell && pos >= 1) {
+#pragma unroll
+      for (int m = 0; m < NF; ++m) {
+        const R t2 = sq[m][before];
+        R s = (R)0;
+        if (wet && !((fabs(q[m]) + fabs(t2)) < (R)kSmall)) s = limiter(q[m], t2);
+        s = hd * s;
+        sl[m][me] = a[m] + s;
+        a[m] = a[m] - s;
+      }
+    }
+    __syncthreads();
+    if (face) {
+#pragma unroll
+      for (int m = 0; m < NF; ++m) l[m] = sl[m][before];
+      F.level(S, k, l, a);
+    }
+  }
+}
 
 // =========================================================================
 //   eval_duvw, explicit part: R1, D, R2-R4, DU/DV/DW (src/nhwave.F:611-1182)
@@ -2999,24 +3152,22 @@ struct OpSSP {
 // =========================================================================
 //               get_Omega (src/nhwave.F:1411-1648)
 // =========================================================================
-struct OpOmegaX {
-  static constexpr const char* kName = "omega_x";  // Ex on x faces from the new state; EtaxL/EtaxR kept for source_terms
-  template <class T>
-  __device__ void operator()(const Dev<T>& S, int f, int j, int k) const {
-    using R = T;
-    const int c0 = f - 1, c1 = f;
-    const long long e0 = i3(S, c0, j, k), e1 = e0 + 1;
+// Ex on x faces from the new state; EtaxL/EtaxR kept for source_terms
+template <class T>
+struct OmegaXFace {
+  static constexpr int kDir = 0, NF = 2;
+  static constexpr const char* kName = "omega_x";
+  using R = T;
+  int f, j, mL, mR;
+  R rdL, rdR, rdd;
+  bool zl, zr;
+  __device__ __forceinline__ static const T* field(const Dev<T>& S, int m) { return m == 0 ? S.U : S.DU; }
+  __device__ __forceinline__ void load(const Dev<T>& S, int f_, int j_, bool low) {
+    f = f_; j = j_;
+    const int c0 = f - 1;
     const long long q0 = i2(S, c0, j), q1 = q0 + 1;
-    const int mL = S.Mask[q0], mR = S.Mask[q1];
-    const R hdx = S.hdxT, rdx = S.dxT, irdx = S.idxT;
-    auto sl = [&](const T* A, long long e, int m) -> R {
-      return m == 0 ? (R)0 : lim_slope_u<R>(A[e - 1], A[e], A[e + 1], rdx, irdx);
-    };
-    const R uL = S.U[e0] + hdx * sl(S.U, e0, mL), uR = S.U[e1] - hdx * sl(S.U, e1, mR);
-    R duL = S.DU[e0] + hdx * sl(S.DU, e0, mL), duR = S.DU[e1] - hdx * sl(S.DU, e1, mR);
-    R rdL, rdR, rdd;
-    bool zl, zr;
-    const bool inL = c0 >= S.IB && c0 <= S.IE, inR = c1 >= S.IB && c1 <= S.IE;
+    mL = S.Mask[q0]; mR = S.Mask[q1];
+    const bool inL = c0 >= S.IB && c0 <= S.IE, inR = f >= S.IB && f <= S.IE;
     if (face_table<R>(S)) {
       const long long n2 = face_slot(S);
       const T* ft = S.fxT + q1;
@@ -3024,9 +3175,13 @@ struct OpOmegaX {
       face_flags(S, q0, 1, inL, inR, zl, zr);
     } else {
       const Face2D F = face_2d(S, q0, 1, inL, inR, 0.5 * S.dx, S.DelxEta, S.Hfx, S.Hfx0);
-      if (k == S.KB) { S.EtaxL[q1] = F.etaL; S.EtaxR[q1] = F.etaR; }
+      if (low) { S.EtaxL[q1] = F.etaL; S.EtaxR[q1] = F.etaR; }
       rdL = (R)F.dL; rdR = (R)F.dR; rdd = (R)(F.dR - F.dL); zl = F.zl; zr = F.zr;
     }
+  }
+  __device__ __forceinline__ void level(const Dev<T>& S, int k, const R (&l)[2], const R (&r)[2]) const {
+    const R uL = l[0], uR = r[0];
+    R duL = l[1], duR = r[1];
     if (zl) duL = (R)0;
     if (zr) duR = (R)0;
     R SL = (R)0, SR = (R)0;
@@ -3052,25 +3207,39 @@ struct OpOmegaX {
     S.Ex[i3(S, f, j, k)] = Ex;
   }
 };
-struct OpOmegaY {
-  static constexpr const char* kName = "omega_y";
+struct OpOmegaX {
+  static constexpr const char* kName = "omega_x";
   template <class T>
-  __device__ void operator()(const Dev<T>& S, int i, int g, int k) const {
+  __device__ void operator()(const Dev<T>& S, int f, int j, int k) const {
     using R = T;
-    const int c0 = g - 1, c1 = g;
-    const long long sy = S.sy;
-    const long long e0 = i3(S, i, c0, k), e1 = e0 + sy;
-    const long long q0 = i2(S, i, c0), q1 = q0 + sy;
-    const int mL = S.Mask[q0], mR = S.Mask[q1];
-    const R hdy = S.hdyT, rdy = S.dyT, irdy = S.idyT;
+    const long long e0 = i3(S, f - 1, j, k), e1 = e0 + 1;
+    const int mL = S.Mask[i2(S, f - 1, j)], mR = S.Mask[i2(S, f, j)];
+    const R hdx = S.hdxT, rdx = S.dxT, irdx = S.idxT;
     auto sl = [&](const T* A, long long e, int m) -> R {
-      return m == 0 ? (R)0 : lim_slope_u<R>(A[e - sy], A[e], A[e + sy], rdy, irdy);
+      return m == 0 ? (R)0 : lim_slope_u<R>(A[e - 1], A[e], A[e + 1], rdx, irdx);
     };
-    const R vL = S.V[e0] + hdy * sl(S.V, e0, mL), vR = S.V[e1] - hdy * sl(S.V, e1, mR);
-    R dvL = S.DV[e0] + hdy * sl(S.DV, e0, mL), dvR = S.DV[e1] - hdy * sl(S.DV, e1, mR);
-    R rdL, rdR, rdd;
-    bool zl, zr;
-    const bool inL = c0 >= S.JB && c0 <= S.JE, inR = c1 >= S.JB && c1 <= S.JE;
+    const R l[2] = {S.U[e0] + hdx * sl(S.U, e0, mL), S.DU[e0] + hdx * sl(S.DU, e0, mL)};
+    const R r[2] = {S.U[e1] - hdx * sl(S.U, e1, mR), S.DU[e1] - hdx * sl(S.DU, e1, mR)};
+    OmegaXFace<T> F;
+    F.load(S, f, j, k == S.KB);
+    F.level(S, k, l, r);
+  }
+};
+template <class T>
+struct OmegaYFace {
+  static constexpr int kDir = 1, NF = 2;
+  static constexpr const char* kName = "omega_y";
+  using R = T;
+  int i, g, mL, mR;
+  R rdL, rdR, rdd;
+  bool zl, zr;
+  __device__ __forceinline__ static const T* field(const Dev<T>& S, int m) { return m == 0 ? S.V : S.DV; }
+  __device__ __forceinline__ void load(const Dev<T>& S, int i_, int g_, bool low) {
+    i = i_; g = g_;
+    const int c0 = g - 1;
+    const long long sy = S.sy, q0 = i2(S, i, c0), q1 = q0 + sy;
+    mL = S.Mask[q0]; mR = S.Mask[q1];
+    const bool inL = c0 >= S.JB && c0 <= S.JE, inR = g >= S.JB && g <= S.JE;
     if (face_table<R>(S)) {
       const long long n2 = face_slot(S);
       const T* ft = S.fyT + q1;
@@ -3078,9 +3247,13 @@ struct OpOmegaY {
       face_flags(S, q0, sy, inL, inR, zl, zr);
     } else {
       const Face2D F = face_2d(S, q0, sy, inL, inR, 0.5 * S.dy, S.DelyEta, S.Hfy, S.Hfy0);
-      if (k == S.KB) { S.EtayL[q1] = F.etaL; S.EtayR[q1] = F.etaR; }
+      if (low) { S.EtayL[q1] = F.etaL; S.EtayR[q1] = F.etaR; }
       rdL = (R)F.dL; rdR = (R)F.dR; rdd = (R)(F.dR - F.dL); zl = F.zl; zr = F.zr;
     }
+  }
+  __device__ __forceinline__ void level(const Dev<T>& S, int k, const R (&l)[2], const R (&r)[2]) const {
+    const R vL = l[0], vR = r[0];
+    R dvL = l[1], dvR = r[1];
     if (zl) dvL = (R)0;
     if (zr) dvR = (R)0;
     R SL = (R)0, SR = (R)0;
@@ -3102,6 +3275,25 @@ struct OpOmegaY {
     R Ey = hll_d<R>(SL, SR, dvL, dvR, rdd);
     if (g == S.JB || g == S.JE + 1) Ey = (R)0;
     S.Ey[i3(S, i, g, k)] = Ey;
+  }
+};
+struct OpOmegaY {
+  static constexpr const char* kName = "omega_y";
+  template <class T>
+  __device__ void operator()(const Dev<T>& S, int i, int g, int k) const {
+    using R = T;
+    const long long sy = S.sy;
+    const long long e0 = i3(S, i, g - 1, k), e1 = e0 + sy;
+    const int mL = S.Mask[i2(S, i, g - 1)], mR = S.Mask[i2(S, i, g)];
+    const R hdy = S.hdyT, rdy = S.dyT, irdy = S.idyT;
+    auto sl = [&](const T* A, long long e, int m) -> R {
+      return m == 0 ? (R)0 : lim_slope_u<R>(A[e - sy], A[e], A[e + sy], rdy, irdy);
+    };
+    const R l[2] = {S.V[e0] + hdy * sl(S.V, e0, mL), S.DV[e0] + hdy * sl(S.DV, e0, mL)};
+    const R r[2] = {S.V[e1] - hdy * sl(S.V, e1, mR), S.DV[e1] - hdy * sl(S.DV, e1, mR)};
+    OmegaYFace<T> F;
+    F.load(S, i, g, k == S.KB);
+    F.level(S, k, l, r);
   }
 };
 // Omega column scan (src/nhwave.F:1617-1628)

@@ -1041,12 +1041,42 @@ class Solver final : public SolverBase {
     incols(OpSource{});
     return check();
   }
+  // The FP64 form's face kernels share quotients and slopes between faces in
+  // blocks; below about 2^16 cells the FP64 pipes are not full and a face a
+  // thread has the shorter chain (256 x 8 x 10, all five: 156 against 169 us).
+  // FP32+IR multiplies by reciprocals and keeps a face a thread.
+  bool face_blocks() const { return !kFP32 && S.neq >= 65536; }
+  // as few chunks of levels as leave about 8 blocks an SM
+  template <class Face>
+  void faces() {
+    constexpr bool x = Face::kDir == 0;
+    const int ntile = x ? (int)cdiv(S.M + 1, kFaceX - 2) : (int)cdiv(S.N + 1, kFaceYy - 2);
+    const int nrow = x ? S.N : (int)cdiv(S.M, kFaceYx);
+    const int chunks = (int)std::min<long long>(S.K, std::max<long long>(1, 152LL * 8 / ((long long)ntile * nrow)));
+    const int kc = (S.K + chunks - 1) / chunks;
+    const unsigned nb = (unsigned)ntile * nrow * cdiv(S.K, kc);
+    L(Face::kName, [&] {
+      k_faces<T, Face><<<nb, x ? dim3(kFaceX) : dim3(kFaceYx, kFaceYy), 0, st>>>(S, kc, ntile, nrow);
+    });
+  }
+  void flux_z_walk() {
+    const long long cols = (long long)S.M * S.N;
+    const int chunks = (int)std::min<long long>(S.K + 1, std::max<long long>(1, 152LL * 512 / cols));
+    const int kc = (S.K + 1 + chunks - 1) / chunks;
+    L("flux_z", [&] { k_flux_z_walk<T><<<cdiv(cols * cdiv(S.K + 1, kc), 128), 128, 0, st>>>(S, kc); });
+  }
   int fluxes() override {
     allcols(OpSlopeEta{});
     if (S.fxT) box(OpFacePrep{0}, S.M + 1, S.N + 1, 1, S.IB, S.JB, 0);
-    box(OpFluxX{}, S.M + 1, S.N, S.K, S.IB, S.JB, S.KB);
-    box(OpFluxY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
-    box(OpFluxZ{}, S.M, S.N, S.K + 1, S.IB, S.JB, S.KB);
+    if (!face_blocks()) {
+      box(OpFluxX{}, S.M + 1, S.N, S.K, S.IB, S.JB, S.KB);
+      box(OpFluxY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
+      box(OpFluxZ{}, S.M, S.N, S.K + 1, S.IB, S.JB, S.KB);
+    } else if constexpr (!kFP32) {
+      faces<FluxXFace<T>>();
+      faces<FluxYFace<T>>();
+      flux_z_walk();
+    }
     if (S.keDxW) cells(OpKeSlopes{0});   // delxyzFun's DelxW / DelyW, read by the 3-D k-epsilon
     return check();
   }
@@ -1456,8 +1486,13 @@ class Solver final : public SolverBase {
     cells(OpSSP{s});
     get_uvw();
     if (S.fxT) box(OpFacePrep{1}, S.M + 1, S.N + 1, 1, S.IB, S.JB, 0);
-    box(OpOmegaX{}, S.M + 1, S.N, S.K, S.IB, S.JB, S.KB);
-    box(OpOmegaY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
+    if (!face_blocks()) {
+      box(OpOmegaX{}, S.M + 1, S.N, S.K, S.IB, S.JB, S.KB);
+      box(OpOmegaY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
+    } else if constexpr (!kFP32) {
+      faces<OmegaXFace<T>>();
+      faces<OmegaYFace<T>>();
+    }
     incols(OpOmegaScan{});
     if (S.keDxU) cells(OpKeSlopes{1});   // get_Omega's DelxU .. DelyV, before sponge_damping
   }
