@@ -2910,95 +2910,132 @@ struct OpColFactors {
   }
 };
 
-struct OpPoissonCoef {
-  static constexpr const char* kName = "poisson_coef";
-  template <class T>
-  __device__ void operator()(const Dev<T>& S, int i, int j, int k) const {
-    const int ic = ic_of(S, i, j, k);
-    const long long sy = S.sy, sz = S.sz;
-    auto inside = [&](int x, int y) { return x >= S.IB && x <= S.IE && y >= S.JB && y <= S.JE; };
+// The Poisson operator and right-hand side.  A block has 30 x 8 columns with a
+// ring of halo threads and walks kc levels up: DelxS / DelyS and the
+// velocities at the level's faces, which up to five cells read, are formed
+// once a cell and passed through shared memory (the halo columns form only
+// theirs), and a level's velocities are converted once.  Bound by the FP64
+// pipe: a cell at a time it takes about 80 FP64 operations a cell, so about 45
+// (GB300 FP32+IR, 1024 x 64 x 20: @P1 -> @P2 us; 768 x 768 x 20: 1860 -> @P4
+// us, coefT included, whose copy of its own was 200).
+constexpr int kPcX = 32, kPcY = 10;
+// a b + c as the two forms are built: fused in FP32+IR, rounded twice in FP64
+template <class T>
+__device__ __forceinline__ double mad_as(double a, double b, double c) {
+  if constexpr (sizeof(T) == 4) return fma(a, b, c);
+  else return a * b + c;
+}
+template <class T>
+__global__ void __launch_bounds__(kPcX * kPcY) k_poisson_coef(Dev<T> S, int kc, int ntile_x, int ntile_y) {
+  if (gated_off(S)) return;
+  __shared__ double sh[2][4][kPcY][kPcX];   // [level parity]: DelxS, DelyS, U and V at the level's face
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int b = blockIdx.x, tile = b % ntile_x, r = b / ntile_x, trow = r % ntile_y, ch = r / ntile_y;
+  const int i = S.IB + tile * (kPcX - 2) + tx - 1, j = S.JB + trow * (kPcY - 2) + ty - 1;
+  const int k0 = S.KB + ch * kc, k1 = min(S.KE, k0 + kc - 1);
+  const bool inx = i >= S.IB && i <= S.IE, iny = j >= S.JB && j <= S.JE, in = inx && iny;
+  const bool own = in && tx > 0 && tx < kPcX - 1 && ty > 0 && ty < kPcY - 1;
+  // which of a column's values its neighbours or itself read
+  const bool needx = iny && i >= S.IB - 1 && i <= S.IE + 1 && ty > 0 && ty < kPcY - 1;
+  const bool needy = inx && j >= S.JB - 1 && j <= S.JE + 1 && tx > 0 && tx < kPcX - 1;
+  const long long sy = S.sy, sz = S.sz;
+  const long long q = (needx || needy) ? i2(S, i, j) : 0, o2 = q;
+  double hx = 0.0, ex = 0.0, hy = 0.0, ey = 0.0;   // zero outside (src/pressure.F:494-505)
+  if (in) { hx = S.cf_hx[q]; ex = S.cf_ex[q]; hy = S.cf_hy[q]; ey = S.cf_ey[q]; }
+  const double DelzS = own ? S.cf_invD[q] : 0.0, src = own ? S.SourceC[q] : 0.0;
+  const double cxx = S.cxx, cyy = S.cyy, i2dx = S.i2dx, i2dy = S.i2dy, rho_dt = S.sc->rho_dt;
+  const size_t n = (size_t)S.neq;
+  // U, V, W of the level below, converted
+  double ud = 0.0, vd = 0.0, wd = 0.0;
+  {
+    const long long o = o2 + sz * (k0 - 1);
+    if (needx || own) ud = (double)S.U[o];
+    if (needy || own) vd = (double)S.V[o];
+    if (own) wd = (double)S.W[o];
+  }
+  for (int k = k0; k <= k1; ++k) {
+    double(*s)[kPcY][kPcX] = sh[k & 1];
+    const long long o = o2 + sz * k;
     const double sgk = S.sig[k], omk = 1. - sgk;
-    // DelxS/DelyS at level sig(k) of interior columns, zero outside (src/pressure.F:494-505)
-    auto dxs = [&](int x, int y) -> double {
-      if (!inside(x, y)) return 0.0;
-      const long long q = i2(S, x, y);
-      return omk * S.cf_hx[q] - sgk * S.cf_ex[q];
-    };
-    auto dys = [&](int x, int y) -> double {
-      if (!inside(x, y)) return 0.0;
-      const long long q = i2(S, x, y);
-      return omk * S.cf_hy[q] - sgk * S.cf_ey[q];
-    };
-    const long long q = i2(S, i, j);
-    const double DelxS = dxs(i, j), DelyS = dys(i, j), DelzS = S.cf_invD[q];
-    const double A1 = DelxS * DelxS + DelyS * DelyS + DelzS * DelzS;
-    const double lx = S.lv_x[k], ly = S.lv_y[k], ih = S.lv_h[k];
-    // Rhs (src/pressure.F:521-525); Uf/Vf: linear interpolation to sig(k) (src/nhwave.F:1346-1355)
-    const double dsk = S.dsig[k], dskm = S.dsig[k - 1];
+    // Uf/Vf: linear interpolation to sig(k) (src/nhwave.F:1346-1355)
     const double fint = S.lv_fint[k];   // dsk / (dsk + dskm)
-    const long long o = i3(S, i, j, k);
-    auto uf = [&](const T* A, long long e) -> double {
-      return (1.0 - fint) * (double)A[e] + fint * (double)A[e - sz];
-    };
-    const double i2dx = S.i2dx, i2dy = S.i2dy;
-    double rhs = -((uf(S.U, o + 1) - uf(S.U, o - 1)) * i2dx + ((double)S.U[o] - (double)S.U[o - sz]) * ih * DelxS +
-                   (uf(S.V, o + sy) - uf(S.V, o - sy)) * i2dy + ((double)S.V[o] - (double)S.V[o - sz]) * ih * DelyS +
-                   ((double)S.W[o] - (double)S.W[o - sz]) * ih * DelzS - S.SourceC[q]) *
-                 S.sc->rho_dt;
-    double C[NCOEF + 1];
-    const double cxx = S.cxx, cyy = S.cyy;
-    C[1] = -2. * cxx - 2. * cyy + A1 * S.lv_up[k] + A1 * S.lv_dn[k];
-    C[2] = cxx;
-    C[3] = cyy;
-    C[4] = (dys(i, j - 1) + DelyS) * ly;
-    C[5] = (dxs(i - 1, j) + DelxS) * lx;
-    C[6] = -A1 * S.lv_up[k];
-    C[7] = -(dxs(i + 1, j) + DelxS) * lx;
-    C[8] = -(dys(i, j + 1) + DelyS) * ly;
-    C[9] = cxx;
-    C[10] = cyy;
-    C[11] = -C[8];
-    C[12] = -C[7];
-    C[13] = -A1 * S.lv_dn[k];
-    C[14] = -C[5];
-    C[15] = -C[4];
-    // boundary folds in the reference's order (src/pressure.F:649-814)
-    if (i == S.IB) { C[1] = C[1] + C[9]; C[6] = C[6] + C[5]; C[13] = C[13] + C[14]; C[9] = C[5] = C[14] = 0.0; }
-    if (i == S.IE) { C[1] = C[1] + C[2]; C[6] = C[6] + C[7]; C[13] = C[13] + C[12]; C[2] = C[7] = C[12] = 0.0; }
-    if (j == S.JB) { C[1] = C[1] + C[10]; C[6] = C[6] + C[4]; C[13] = C[13] + C[15]; C[10] = C[4] = C[15] = 0.0; }
-    if (j == S.JE) { C[1] = C[1] + C[3]; C[6] = C[6] + C[8]; C[13] = C[13] + C[11]; C[3] = C[8] = C[11] = 0.0; }
-    if (k == S.KB) {
-      if (S.slide) {
-        const double* D = S.D;
-        const double* H2 = S.Delt2H;
-        rhs = rhs + kRho0 * (dsk + dskm) *
-                        (C[13] * D[q] * H2[q] + C[12] * D[q + 1] * H2[q + 1] + C[11] * D[q + sy] * H2[q + sy] +
-                         C[14] * D[q - 1] * H2[q - 1] + C[15] * D[q - sy] * H2[q - sy]);
-      }
-      C[6] = C[6] + C[13]; C[7] = C[7] + C[12]; C[8] = C[8] + C[11]; C[5] = C[5] + C[14]; C[4] = C[4] + C[15];
-      C[13] = C[12] = C[11] = C[14] = C[15] = 0.0;
+    double u = 0.0, v = 0.0, DelxS = 0.0, DelyS = 0.0;
+    if (needx) {
+      u = (double)S.U[o];
+      if (in) DelxS = omk * hx - sgk * ex;
+      s[0][ty][tx] = DelxS;
+      s[2][ty][tx] = mad_as<T>(1.0 - fint, u, fint * ud);
     }
-    // compact form: C1, C6, C13 after every fold; the k+1 cross terms before
-    // the top row's zeroing (their negatives are the k-1 terms of this cell)
-    const size_t n = (size_t)S.neq;
-    double* o7 = S.coef64 + ic;
-    o7[3 * n] = C[4]; o7[4 * n] = C[5]; o7[5 * n] = C[7]; o7[6 * n] = C[8];
-    if (k == S.KE) { C[4] = C[5] = C[6] = C[7] = C[8] = 0.0; }
-    o7[0] = C[1]; o7[n] = C[6]; o7[2 * n] = C[13];
-    S.rhs64[ic] = rhs;
+    if (needy) {
+      v = (double)S.V[o];
+      if (in) DelyS = omk * hy - sgk * ey;
+      s[1][ty][tx] = DelyS;
+      s[3][ty][tx] = mad_as<T>(1.0 - fint, v, fint * vd);
+    }
+    __syncthreads();
+    if (own) {
+      const int ic = ic_of(S, i, j, k);
+      const double w = (double)S.W[o];
+      const double A1 = DelxS * DelxS + DelyS * DelyS + DelzS * DelzS;
+      const double lx = S.lv_x[k], ly = S.lv_y[k], ih = S.lv_h[k];
+      // Rhs (src/pressure.F:521-525)
+      double sum = mad_as<T>(s[2][ty][tx + 1] - s[2][ty][tx - 1], i2dx, (u - ud) * ih * DelxS);
+      sum = mad_as<T>(s[3][ty + 1][tx] - s[3][ty - 1][tx], i2dy, sum);
+      sum = mad_as<T>((v - vd) * ih, DelyS, sum);
+      sum = mad_as<T>((w - wd) * ih, DelzS, sum);
+      double rhs = -(sum - src) * rho_dt;
+      double C[NCOEF + 1];
+      C[1] = -2. * cxx - 2. * cyy + A1 * S.lv_up[k] + A1 * S.lv_dn[k];
+      C[2] = cxx;
+      C[3] = cyy;
+      C[4] = (s[1][ty - 1][tx] + DelyS) * ly;
+      C[5] = (s[0][ty][tx - 1] + DelxS) * lx;
+      C[6] = -A1 * S.lv_up[k];
+      C[7] = -(s[0][ty][tx + 1] + DelxS) * lx;
+      C[8] = -(s[1][ty + 1][tx] + DelyS) * ly;
+      C[9] = cxx;
+      C[10] = cyy;
+      C[11] = -C[8];
+      C[12] = -C[7];
+      C[13] = -A1 * S.lv_dn[k];
+      C[14] = -C[5];
+      C[15] = -C[4];
+      // boundary folds in the reference's order (src/pressure.F:649-814), a
+      // branch of their own: as selects they would cost every cell 17 FP64 sums
+      if (i == S.IB || i == S.IE || j == S.JB || j == S.JE || k == S.KB) {
+        if (i == S.IB) { C[1] = C[1] + C[9]; C[6] = C[6] + C[5]; C[13] = C[13] + C[14]; C[9] = C[5] = C[14] = 0.0; }
+        if (i == S.IE) { C[1] = C[1] + C[2]; C[6] = C[6] + C[7]; C[13] = C[13] + C[12]; C[2] = C[7] = C[12] = 0.0; }
+        if (j == S.JB) { C[1] = C[1] + C[10]; C[6] = C[6] + C[4]; C[13] = C[13] + C[15]; C[10] = C[4] = C[15] = 0.0; }
+        if (j == S.JE) { C[1] = C[1] + C[3]; C[6] = C[6] + C[8]; C[13] = C[13] + C[11]; C[3] = C[8] = C[11] = 0.0; }
+        if (k == S.KB) {
+          if (S.slide) {
+            const double* D = S.D;
+            const double* H2 = S.Delt2H;
+            rhs = rhs + kRho0 * (S.dsig[k] + S.dsig[k - 1]) *
+                            (C[13] * D[q] * H2[q] + C[12] * D[q + 1] * H2[q + 1] + C[11] * D[q + sy] * H2[q + sy] +
+                             C[14] * D[q - 1] * H2[q - 1] + C[15] * D[q - sy] * H2[q - sy]);
+          }
+          C[6] = C[6] + C[13]; C[7] = C[7] + C[12]; C[8] = C[8] + C[11]; C[5] = C[5] + C[14]; C[4] = C[4] + C[15];
+          C[13] = C[12] = C[11] = C[14] = C[15] = 0.0;
+        }
+      }
+      // compact form: C1, C6, C13 after every fold; the k+1 cross terms before
+      // the top row's zeroing (their negatives are the k-1 terms of this cell)
+      // FP32+IR: the same in the inner precision
+      auto put = [&](int m, double v) {
+        S.coef64[m * n + ic] = v;
+        if constexpr (sizeof(T) == 4) S.coefT[m * n + ic] = (T)v;
+      };
+      put(3, C[4]); put(4, C[5]); put(5, C[7]); put(6, C[8]);
+      if (k == S.KE) { C[4] = C[5] = C[6] = C[7] = C[8] = 0.0; }
+      put(0, C[1]); put(1, C[6]); put(2, C[13]);
+      S.rhs64[ic] = rhs;
+      wd = w;
+    }
+    ud = u;
+    vd = v;
   }
-};
-
-// copy of the FP64 operator into the inner precision (FP32 form only)
-struct OpCoefToT {
-  static constexpr const char* kName = "coef_to_inner";
-  template <class T>
-  __device__ void operator()(const Dev<T>& S, int i, int j, int k) const {
-    const int ic = ic_of(S, i, j, k);
-    const size_t n = (size_t)S.neq;
-    for (int m = 0; m < 7; ++m) S.coefT[m * n + ic] = (T)S.coef64[m * n + ic];
-  }
-};
+}
 
 // vertical-line preconditioner factors: tridiagonal (C13, C1, C6) per column
 struct OpLineFactor {

@@ -1104,8 +1104,13 @@ class Solver final : public SolverBase {
   }
   void poisson_setup() {
     incols(OpColFactors{});
-    cells(OpPoissonCoef{});
-    if (kFP32) cells(OpCoefToT{});
+    {
+      const int nx = (int)cdiv(S.M, kPcX - 2), ny = (int)cdiv(S.N, kPcY - 2);
+      const int chunks = (int)std::min<long long>(S.K, std::max<long long>(1, 152LL * 8 / ((long long)nx * ny)));
+      const int kc = (S.K + chunks - 1) / chunks;
+      const unsigned nb = (unsigned)nx * ny * cdiv(S.K, kc);
+      L("poisson_coef", [&] { k_poisson_coef<T><<<nb, dim3(kPcX, kPcY), 0, st>>>(S, kc, nx, ny); });
+    }
     if (use_mg && mg.size() > 1) {
       cudaEventRecord(ev_fork, st);
       cudaStreamWaitEvent(mg_st, ev_fork, 0);
