@@ -88,6 +88,33 @@ __device__ __forceinline__ R hllc(R sl, R sr, R ss, R fl, R fr, R ul, R uls, R u
   return fr + sr * (urs - ur);
 }
 
+// float <-> double on the integer pipes.  A conversion takes the FP64 pipe,
+// which issues one warp's instruction in 16 cycles; a few integer operations on
+// the bit patterns take a quarter of that.  Exact (widen) and rounded to
+// nearest even (narrow), so the values are the conversions'; zeros are common
+// and handled, subnormal results, infinities and NaN go to the instruction.
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), t = b & 0x7fffffffu;
+  if (t - 0x00800000u >= 0x7f000000u && t != 0u) return (double)x;
+  const unsigned hi = t == 0u ? 0u : (t >> 3) + 0x38000000u;
+  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(b << 29));
+}
+template <class T>
+__device__ __forceinline__ T narrow(double x) {
+  if constexpr (sizeof(T) == 8) return x;
+  else {
+    const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x), t = h & 0x7fffffffu;
+    // normal floats whose rounding up stays finite: exponents 2^-126 .. 2^126
+    if (t - 0x38100000u >= 0x47d00000u - 0x38100000u && (t | l) != 0u) return (T)x;
+    if ((t | l) == 0u) return __uint_as_float(h);
+    // 20 + 3 bits of the mantissa, then round half to even on the other 29
+    const unsigned m = ((t - 0x38000000u) << 3) | (l >> 29), rest = l & 0x1fffffffu;
+    const unsigned up = (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) ? 1u : 0u;
+    return __uint_as_float((h & 0x80000000u) | (m + up));
+  }
+}
+
 // A divisor used more than once: the FP64 form divides by it, as the reference
 // does; the FP32+IR form multiplies by its FP64 reciprocal (one division of
 // some 25 FP64 instructions for all of them).
@@ -1125,20 +1152,22 @@ struct OpExplicit {
     const double dt = S.sc->dt;
     double r1 = 0.0;
     if (S.Mask[c] != 0) {
+#pragma unroll 4
       for (int k = S.KB; k <= S.KE; ++k) {
         const long long o = i3(S, i, j, k);
-        const double dEx = (double)S.Ex[o + 1] - (double)S.Ex[o];
-        const double dEy = (double)S.Ey[o + S.sy] - (double)S.Ey[o];
+        const double dEx = widen(S.Ex[o + 1]) - widen(S.Ex[o]);
+        const double dEy = widen(S.Ey[o + S.sy]) - widen(S.Ey[o]);
         r1 = r1 - 1.0 / S.dx * dEx * S.dsig[k] - 1.0 / S.dy * dEy * S.dsig[k];
       }
       r1 = r1 + S.D[c] * S.SourceC[c];
       S.D[c] = S.alpha[istep] * S.D0[c] + S.beta[istep] * (S.D[c] + dt * r1);
       const R rdx = S.idxT, rdy = S.idyT, rdt = (R)dt, fc = (R)S.fcor;
       const R sx = (R)S.SourceX[c], syy = (R)S.SourceY[c];
-      for (int k = S.KB; k <= S.KE; ++k) {
+      // two levels' loads before the first of their stores
+      auto update = [&](int k, R& du, R& dv, R& dw) {
         const long long o = i3(S, i, j, k);
         const R rds = S.lvT[k];   // (R)(1.0 / dsig_k)
-        const R du = S.DU[o], dv = S.DV[o], dw = S.DW[o];
+        du = S.DU[o]; dv = S.DV[o]; dw = S.DW[o];
         R R2 = -rdx * (S.Fx[o + 1] - S.Fx[o]) - rdy * (S.Fy[o + S.sy] - S.Fy[o]) -
                rds * (S.Fz[o + S.sz] - S.Fz[o]) + fc * dv + sx;
         R R3 = -rdx * (S.Gx[o + 1] - S.Gx[o]) - rdy * (S.Gy[o + S.sy] - S.Gy[o]) -
@@ -1150,10 +1179,27 @@ struct OpExplicit {
           R3 = R3 + S.Dyx[o] + S.Dyy[o];
           R4 = R4 + S.Dzx[o] + S.Dzy[o];
         }
-        // viscous flow: DU + dt R2 is the right-hand side of OpVertVisc
-        S.DU[o] = du + rdt * R2;
-        S.DV[o] = dv + rdt * R3;
-        S.DW[o] = dw + rdt * R4;
+        // viscous flow: DU + dt R2 is the right-hand side of k_vert_visc
+        du = du + rdt * R2;
+        dv = dv + rdt * R3;
+        dw = dw + rdt * R4;
+      };
+      auto store = [&](int k, R du, R dv, R dw) {
+        const long long o = i3(S, i, j, k);
+        S.DU[o] = du; S.DV[o] = dv; S.DW[o] = dw;
+      };
+      int k = S.KB;
+      for (; k < S.KE; k += 2) {
+        R u0, v0, w0, u1, v1, w1;
+        update(k, u0, v0, w0);
+        update(k + 1, u1, v1, w1);
+        store(k, u0, v0, w0);
+        store(k + 1, u1, v1, w1);
+      }
+      if (k == S.KE) {
+        R u0, v0, w0;
+        update(k, u0, v0, w0);
+        store(k, u0, v0, w0);
       }
     } else {
       for (int k = S.KB; k <= S.KE; ++k) {
@@ -2916,7 +2962,7 @@ struct OpColFactors {
 // once a cell and passed through shared memory (the halo columns form only
 // theirs), and a level's velocities are converted once.  Bound by the FP64
 // pipe: a cell at a time it takes about 80 FP64 operations a cell, so about 45
-// (GB300 FP32+IR, 1024 x 64 x 20: @P1 -> @P2 us; 768 x 768 x 20: 1860 -> @P4
+// (GB300 FP32+IR, 1024 x 64 x 20: 215 -> 179 us; 768 x 768 x 20: 1860 -> 1420
 // us, coefT included, whose copy of its own was 200).
 constexpr int kPcX = 32, kPcY = 10;
 // a b + c as the two forms are built: fused in FP32+IR, rounded twice in FP64
@@ -2949,9 +2995,9 @@ __global__ void __launch_bounds__(kPcX * kPcY) k_poisson_coef(Dev<T> S, int kc, 
   double ud = 0.0, vd = 0.0, wd = 0.0;
   {
     const long long o = o2 + sz * (k0 - 1);
-    if (needx || own) ud = (double)S.U[o];
-    if (needy || own) vd = (double)S.V[o];
-    if (own) wd = (double)S.W[o];
+    if (needx || own) ud = widen(S.U[o]);
+    if (needy || own) vd = widen(S.V[o]);
+    if (own) wd = widen(S.W[o]);
   }
   for (int k = k0; k <= k1; ++k) {
     double(*s)[kPcY][kPcX] = sh[k & 1];
@@ -2961,13 +3007,13 @@ __global__ void __launch_bounds__(kPcX * kPcY) k_poisson_coef(Dev<T> S, int kc, 
     const double fint = S.lv_fint[k];   // dsk / (dsk + dskm)
     double u = 0.0, v = 0.0, DelxS = 0.0, DelyS = 0.0;
     if (needx) {
-      u = (double)S.U[o];
+      u = widen(S.U[o]);
       if (in) DelxS = omk * hx - sgk * ex;
       s[0][ty][tx] = DelxS;
       s[2][ty][tx] = mad_as<T>(1.0 - fint, u, fint * ud);
     }
     if (needy) {
-      v = (double)S.V[o];
+      v = widen(S.V[o]);
       if (in) DelyS = omk * hy - sgk * ey;
       s[1][ty][tx] = DelyS;
       s[3][ty][tx] = mad_as<T>(1.0 - fint, v, fint * vd);
@@ -2975,7 +3021,7 @@ __global__ void __launch_bounds__(kPcX * kPcY) k_poisson_coef(Dev<T> S, int kc, 
     __syncthreads();
     if (own) {
       const int ic = ic_of(S, i, j, k);
-      const double w = (double)S.W[o];
+      const double w = widen(S.W[o]);
       const double A1 = DelxS * DelxS + DelyS * DelyS + DelzS * DelzS;
       const double lx = S.lv_x[k], ly = S.lv_y[k], ih = S.lv_h[k];
       // Rhs (src/pressure.F:521-525)
@@ -3024,12 +3070,13 @@ __global__ void __launch_bounds__(kPcX * kPcY) k_poisson_coef(Dev<T> S, int kc, 
       // FP32+IR: the same in the inner precision
       auto put = [&](int m, double v) {
         S.coef64[m * n + ic] = v;
-        if constexpr (sizeof(T) == 4) S.coefT[m * n + ic] = (T)v;
+        if constexpr (sizeof(T) == 4) S.coefT[m * n + ic] = narrow<T>(v);
       };
       put(3, C[4]); put(4, C[5]); put(5, C[7]); put(6, C[8]);
       if (k == S.KE) { C[4] = C[5] = C[6] = C[7] = C[8] = 0.0; }
       put(0, C[1]); put(1, C[6]); put(2, C[13]);
       S.rhs64[ic] = rhs;
+      S.xsol64[ic] = S.P[o];   // initial guess: the previous pressure
       wd = w;
     }
     ud = u;
@@ -3083,13 +3130,6 @@ struct OpPFromX {
     S.P[i3(S, i, j, k)] = S.xsol64[ic];
   }
 };
-struct OpXFromP {
-  static constexpr const char* kName = "x_from_p";
-  template <class T>
-  __device__ void operator()(const Dev<T>& S, int i, int j, int k) const {
-    S.xsol64[ic_of(S, i, j, k)] = S.P[i3(S, i, j, k)];
-  }
-};
 struct OpPGhost {
   static constexpr const char* kName = "p_ghost";
   template <class T>
@@ -3125,30 +3165,44 @@ struct OpProjection {
 };
 // The same in the FP32+IR form: the pressure differences in FP64 (P is FP64),
 // each rounded once, and the rest in FP32
-struct OpProjection32 {
-  static constexpr const char* kName = "projection";
-  template <class T>
-  __device__ void operator()(const Dev<T>& S, int i, int j, int k) const {
-    const long long q = i2(S, i, j);
-    if (S.Mask[q] == 0) return;
-    const long long o = i3(S, i, j, k), sy = S.sy, sz = S.sz;
-    const double* P = S.P;
-    const T hx = (T)S.i2dx, hy = (T)S.i2dy;
-    const T dx0 = (T)(P[o + 1] - P[o - 1]), dx1 = (T)(P[o + 1 + sz] - P[o - 1 + sz]);
-    const T dy0 = (T)(P[o + sy] - P[o - sy]), dy1 = (T)(P[o + sy + sz] - P[o - sy + sz]);
+// The same in the FP32+IR form, a thread walking kc levels of a column: the
+// column's factors are rounded to FP32 once, a level's horizontal pressure
+// differences serve the level below and above, 3 FP64 differences a cell
+// instead of 5, 7 conversions less (768 x 768 x 20: 398 -> @J us).
+template <class T>
+__global__ void __launch_bounds__(128) k_projection32(Dev<T> S, int kc) {
+  if (gated_off(S)) return;
+  const int cols = S.M * S.N, t = blockIdx.x * blockDim.x + threadIdx.x, ch = t / cols, col = t - ch * cols;
+  const int k0 = S.KB + ch * kc, k1 = min(S.KE, k0 + kc - 1);
+  if (k0 > S.KE) return;
+  const int i = S.IB + col % S.M, j = S.JB + col / S.M;
+  const long long q = i2(S, i, j), sy = S.sy, sz = S.sz;
+  if (S.Mask[q] == 0) return;
+  const double* P = S.P;
+  const T hx = (T)S.i2dx, hy = (T)S.i2dy;
+  const T chx = (T)S.cf_hx[q], cex = (T)S.cf_ex[q], chy = (T)S.cf_hy[q], cey = (T)S.cf_ey[q];
+  const T g = (T)S.sc->dt_rho, f = (T)S.D[q] * g;
+  long long o = i3(S, i, j, k0);
+  double p0 = P[o];
+  T dx0 = narrow<T>(P[o + 1] - P[o - 1]), dy0 = narrow<T>(P[o + sy] - P[o - sy]);
+#pragma unroll 2
+  for (int k = k0; k <= k1; ++k, o += sz) {
+    const double p1 = P[o + sz];
+    const T dx1 = narrow<T>(P[o + 1 + sz] - P[o - 1 + sz]), dy1 = narrow<T>(P[o + sy + sz] - P[o - sy + sz]);
     const T DelxP = (T)0.5 * (dx0 * hx + dx1 * hx), DelyP = (T)0.5 * (dy0 * hy + dy1 * hy);
-    const T DelzP = (T)(P[o + sz] - P[o]) * S.lvT[k];
+    const T DelzP = narrow<T>(p1 - p0) * S.lvT[k];
     const T sc = (T)S.sigc[k], omc = (T)1 - sc;
-    const T DelxSc = omc * (T)S.cf_hx[q] - sc * (T)S.cf_ex[q];
-    const T DelySc = omc * (T)S.cf_hy[q] - sc * (T)S.cf_ey[q];
-    const T g = (T)S.sc->dt_rho, f = (T)S.D[q] * g;
+    const T DelxSc = omc * chx - sc * cex;
+    const T DelySc = omc * chy - sc * cey;
     S.DU[o] = S.DU[o] - f * (DelxP + DelzP * DelxSc);
     S.DV[o] = S.DV[o] - f * (DelyP + DelzP * DelySc);
     S.DW[o] = S.DW[o] - g * DelzP;
+    p0 = p1;
+    dx0 = dx1;
+    dy0 = dy1;
   }
-};
+}
 
-// SSP-RK combination, mask and Froude cap (src/nhwave.F:1227-1261)
 struct OpSSP {
   static constexpr const char* kName = "ssp_combine";
   int istep;
@@ -3344,16 +3398,31 @@ struct OpOmegaScan {
     const double rdx = 2.0 * S.i2dx, rdy = 2.0 * S.i2dy;   // 1/dx, 1/dy
     double om = 0.0;
     S.Omega[i3(S, i, j, S.KB)] = (T)0;
-    for (int k = S.KB + 1; k <= S.KE + 1; ++k) {
-      const long long o = i3(S, i, j, k - 1);
-      const double dEx = (double)S.Ex[o + 1] - (double)S.Ex[o];
-      const double dEy = (double)S.Ey[o + S.sy] - (double)S.Ey[o];
-      double v;
-      if constexpr (sizeof(T) == 4) v = om - S.dsig[k - 1] * (r1 + dEx * rdx + dEy * rdy);   // FP32 form: products
-      else v = om - S.dsig[k - 1] * (r1 + dEx / S.dx + dEy / S.dy);
-      if (!wet) v = 0.0;
-      S.Omega[i3(S, i, j, k)] = (T)v;
-      om = (double)(T)v;
+    const long long o0 = i3(S, i, j, S.KB);
+    // four levels' loads before the first of their stores, which would hold
+    // them back
+    for (int m = 0; m < S.K; m += 4) {
+      T xe[4], xw[4], yn[4], ys[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const long long o = o0 + S.sz * min(m + t, S.K - 1);
+        xe[t] = S.Ex[o + 1]; xw[t] = S.Ex[o];
+        yn[t] = S.Ey[o + S.sy]; ys[t] = S.Ey[o];
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        if (m + t >= S.K) break;
+        const double dEx = widen(xe[t]) - widen(xw[t]);
+        const double dEy = widen(yn[t]) - widen(ys[t]);
+        const double ds = S.dsig[S.KB + m + t];
+        double v;
+        if constexpr (sizeof(T) == 4) v = om - ds * (r1 + dEx * rdx + dEy * rdy);   // FP32 form: products
+        else v = om - ds * (r1 + dEx / S.dx + dEy / S.dy);
+        if (!wet) v = 0.0;
+        const T w = narrow<T>(v);
+        S.Omega[o0 + S.sz * (m + t + 1)] = w;
+        om = widen(w);
+      }
     }
   }
 };

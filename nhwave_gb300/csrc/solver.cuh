@@ -1130,7 +1130,6 @@ class Solver final : public SolverBase {
       mg_forked = true;
     }
     incols(OpLineFactor{});
-    cells(OpXFromP{});
   }
   // P from the solution, ghosts mirrored (src/pressure.F:185-239)
   void poisson_finish() {
@@ -1485,7 +1484,12 @@ class Solver final : public SolverBase {
   void stage_post(int s) {
     if (S.non_hydro) {
       poisson_finish();
-      if (kFP32) cells(OpProjection32{});
+      if (kFP32) {
+        const long long cols = (long long)S.M * S.N;
+        const int chunks = (int)std::min<long long>(S.K, std::max<long long>(1, 152LL * 1024 / cols));
+        const int kc = (S.K + chunks - 1) / chunks;
+        L("projection", [&] { k_projection32<T><<<cdiv(cols * cdiv(S.K, kc), 128), 128, 0, st>>>(S, kc); });
+      }
       else cells(OpProjection{});
     }
     cells(OpSSP{s});
