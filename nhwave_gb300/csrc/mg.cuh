@@ -9,8 +9,8 @@
 //     level -- the sigma-layer coupling is usually the strong one;
 //   * coarse operators: Galerkin products P^T A P with piecewise-constant P,
 //     which keep the 15-point pattern, hence the compact form of krylov.cuh
-//     plus explicit in-level couplings (uneven last aggregates make those
-//     non-uniform);
+//     with in-level couplings of their own (two constants a direction: the
+//     last aggregate may be uneven);
 //   * smoother: red-black ("zebra") vertical-line Gauss-Seidel -- each colour
 //     solves the tridiagonal (C13, C1, C6) system of its columns with the
 //     neighbouring columns (the other colour) fixed; one sweep before and one
@@ -25,31 +25,49 @@ template <class T>
 struct MGL {
   int M, N, K, n;
   const T* coef;        // [7][n] compact operator of this level
-  const T* cxr;         // [n] coupling to i+1 (nullptr: the constant cxx)
-  const T* cyr;         // [n] coupling to j+1 (nullptr: the constant cyy)
-  T cxx, cyy;
+  // In-level couplings.  Those of level 0 are constant; an aggregate's is the
+  // sum over its face's fine cells, rescaled (k_mg_galerkin), so it depends
+  // only on how many rows (columns) the aggregate has and the last row's
+  // (column's) alone may differ.
+  T cxx, cyy;           // to i-1 and i+1; to j-1 and j+1
+  T cxl, cyl;           // cxx in the last row, cyy in the last column
   const T* lcp;         // line factors of (C13, C1, C6)
   const T* linv;
   T* x;
   T* b;
   int rx, ry;           // aggregation to the next coarser level
   int Mc, Nc;
-  // Level 0 only (else nullptr): C13, 1/den, c/den, C4, C5, C7, C8 of the
-  // half-sweeps again, split by colour.  Slot s of colour c starts at
+  // Level 0, and coarse levels too large for the tiles of mg_tile.cuh (else
+  // nullptr): C13, 1/den, c/den, C4, C5, C7, C8 of the half-sweeps again,
+  // split by colour.  Slot s of colour c starts at
   // sp + (2 s + c) * K * N * Mh, Mh = (M + 1) / 2, and holds level k, row jj,
   // column ii of that colour at k * N * Mh + jj * Mh + ii / 2.
   const T* sp;
   T* xp;                // colour 0 of x between the two halves of a V-cycle (mg_tile.cuh)
 };
 
+// in-level couplings along i in row jj, along j in column ii
 template <class T>
-__device__ __forceinline__ T cx_p(const MGL<T>& L, int ic) { return L.cxr ? L.cxr[ic] : L.cxx; }
+__device__ __forceinline__ T cx_of(const MGL<T>& L, int jj) { return jj == L.N - 1 ? L.cxl : L.cxx; }
 template <class T>
-__device__ __forceinline__ T cx_m(const MGL<T>& L, int ic) { return L.cxr ? L.cxr[ic - 1] : L.cxx; }
+__device__ __forceinline__ T cy_of(const MGL<T>& L, int ii) { return ii == L.M - 1 ? L.cyl : L.cyy; }
+
+// the couplings of level c, whose aggregates are rx x ry cells of level f: the
+// sums and the scale that k_mg_galerkin takes, in its order
 template <class T>
-__device__ __forceinline__ T cy_p(const MGL<T>& L, int ic) { return L.cyr ? L.cyr[ic] : L.cyy; }
-template <class T>
-__device__ __forceinline__ T cy_m(const MGL<T>& L, int ic) { return L.cyr ? L.cyr[ic - L.M] : L.cyy; }
+inline void coarse_couplings(const MGL<T>& f, MGL<T>& c) {
+  auto face = [](int r, int nf, T inner, T last, T& ci, T& cl) {
+    const int nl = nf - ((nf + r - 1) / r - 1) * r;   // fine rows of the last aggregate
+    ci = cl = (T)0;
+    for (int t = 0; t < r; ++t) ci += inner;
+    for (int t = 0; t < nl; ++t) cl += t == nl - 1 ? last : inner;
+  };
+  face(f.ry, f.N, f.cxx, f.cxl, c.cxx, c.cxl);
+  face(f.rx, f.M, f.cyy, f.cyl, c.cyy, c.cyl);
+  const T sx = (T)1 / (T)f.rx, sy = (T)1 / (T)f.ry;
+  c.cxx *= sx; c.cxl *= sx;
+  c.cyy *= sy; c.cyl *= sy;
+}
 
 // off-column part of (A x) at cell (ii, jj, kk): everything but C1, C6, C13;
 // c4, c5, c7, c8 are the cell's cross terms
@@ -59,10 +77,11 @@ __device__ __forceinline__ T off_column_c(const MGL<T>& L, const T* __restrict__
   const int M = L.M, MN = L.M * L.N;
   const bool im = ii > 0, ip = ii < L.M - 1, jm = jj > 0, jp = jj < L.N - 1, km = kk > 0, kp = kk < L.K - 1;
   T s = (T)0;
-  if (ip) s += cx_p(L, ic) * x[ic + 1];
-  if (im) s += cx_m(L, ic) * x[ic - 1];
-  if (jp) s += cy_p(L, ic) * x[ic + M];
-  if (jm) s += cy_m(L, ic) * x[ic - M];
+  const T cx = cx_of(L, jj), cy = cy_of(L, ii);
+  if (ip) s += cx * x[ic + 1];
+  if (im) s += cx * x[ic - 1];
+  if (jp) s += cy * x[ic + M];
+  if (jm) s += cy * x[ic - M];
   if (kp) {
     const int u = ic + MN;
     if (ip) s += c7 * x[u + 1];
@@ -173,10 +192,11 @@ __device__ __forceinline__ T off_column_pc(const MGL<T>& L, const T* __restrict_
     if (kp) s += cross * P.at(x, ic + off + MN, st, kk + 1);
     if (km) s -= cross * P.at(x, ic + off - MN, st, kk - 1);
   };
-  if (ip) column(1, cx_p(L, ic), c7, ii + 1, jj);
-  if (im) column(-1, cx_m(L, ic), c5, ii - 1, jj);
-  if (jp) column(M, cy_p(L, ic), c8, ii, jj + 1);
-  if (jm) column(-M, cy_m(L, ic), c4, ii, jj - 1);
+  const T cx = cx_of(L, jj), cy = cy_of(L, ii);
+  if (ip) column(1, cx, c7, ii + 1, jj);
+  if (im) column(-1, cx, c5, ii - 1, jj);
+  if (jp) column(M, cy, c8, ii, jj + 1);
+  if (jm) column(-M, cy, c4, ii, jj - 1);
   return s;
 }
 template <class T>
@@ -322,7 +342,7 @@ __global__ void __launch_bounds__(1024) k_mg_smooth_blk(MGL<T> L, const DevScal*
   }
 }
 
-// Level-0 half-sweep on the colour-split operator (MGL::sp).  A block holds
+// Half-sweep on the colour-split operator (MGL::sp).  A block holds
 // 32 consecutive columns of the colour in that layout, so its loads of C13,
 // the line factors and the cross terms are contiguous; in the natural layout
 // every other column of a row belongs to the other colour and half of each
@@ -365,9 +385,7 @@ k_mg_smooth_split(MGL<T> L, const DevScal* sc, int color, int zero_x, Prolong<T>
   const T* sp = L.sp + (size_t)color * cs + q;
   const bool im = ii > 0, ip = ii < M - 1, jm = jj > 0, jp = jj < L.N - 1;
   const T* __restrict__ x = L.x;
-  // level 0 couples the columns in a level by the constants cxx, cyy (cxr,
-  // cyr are null there; only coarse levels carry per-cell couplings)
-  const T cxx = L.cxx, cyy = L.cyy;
+  const T cxx = cx_of(L, jj), cyy = cy_of(L, ii);
   typename Prolong<T>::Stencil sxp{}, sxm{}, syp{}, sym{};
   if (kProlong && valid && !zero_x) {
     if (ip) sxp = P.stencil(ii + 1, jj);
@@ -709,7 +727,7 @@ __global__ void __launch_bounds__(256) k_mg_restrict_c0(MGL<T> F, MGL<T> C, cons
 
 // Galerkin coarse operator P^T A P (piecewise-constant P), compact form + couplings
 template <class T>
-__global__ void __launch_bounds__(256) k_mg_galerkin(MGL<T> F, T* ccoef, T* ccxr, T* ccyr, int Mc, int Nc) {
+__global__ void __launch_bounds__(256) k_mg_galerkin(MGL<T> F, T* ccoef, T* csp, int Mc, int Nc) {
   const int nc = Mc * Nc * F.K;
   const int ic = blockIdx.x * blockDim.x + threadIdx.x;
   if (ic >= nc) return;
@@ -731,10 +749,11 @@ __global__ void __launch_bounds__(256) k_mg_galerkin(MGL<T> F, T* ccoef, T* ccxr
       if (k > 0) dn += F.coef[2 * n + f];
       const T c4 = F.coef[3 * n + f], c5 = F.coef[4 * n + f], c7 = F.coef[5 * n + f], c8 = F.coef[6 * n + f];
       // in-level neighbours
-      if (i + 1 < F.M) { const T c = cx_p(F, f); if ((i + 1) / F.rx == I) d += c; else xp += c; }
-      if (i - 1 >= 0) { const T c = cx_m(F, f); if ((i - 1) / F.rx == I) d += c; else xm += c; }
-      if (j + 1 < F.N) { const T c = cy_p(F, f); if ((j + 1) / F.ry == J) d += c; else yp += c; }
-      if (j - 1 >= 0) { const T c = cy_m(F, f); if ((j - 1) / F.ry == J) d += c; else ym += c; }
+      const T cx = cx_of(F, j), cy = cy_of(F, i);
+      if (i + 1 < F.M) { const T c = cx; if ((i + 1) / F.rx == I) d += c; else xp += c; }
+      if (i - 1 >= 0) { const T c = cx; if ((i - 1) / F.rx == I) d += c; else xm += c; }
+      if (j + 1 < F.N) { const T c = cy; if ((j + 1) / F.ry == J) d += c; else yp += c; }
+      if (j - 1 >= 0) { const T c = cy; if ((j - 1) / F.ry == J) d += c; else ym += c; }
       // cross terms k+1 (+c) and k-1 (-c)
       if (k < K - 1) {
         if (i + 1 < F.M) { if ((i + 1) / F.rx == I) up += c7; else x7u += c7; }
@@ -759,26 +778,33 @@ __global__ void __launch_bounds__(256) k_mg_galerkin(MGL<T> F, T* ccoef, T* ccxr
   // correction of horizontally smooth errors on every level, which a uniform
   // correction weight cannot undo without over-correcting the vertical.  So
   // the in-level couplings are scaled by 1/rx and 1/ry, and the removed part
-  // goes to the diagonal: the row sums stay those of the product.
+  // goes to the diagonal: the row sums stay those of the product.  The couplings
+  // themselves are constants (coarse_couplings).
   const T sx = (T)1 / (T)F.rx, sy = (T)1 / (T)F.ry;
   d += ((T)1 - sx) * (xp + xm) + ((T)1 - sy) * (yp + ym);
-  xp *= sx;
-  yp *= sy;
   const bool top = (k == K - 1);
   ccoef[ic] = d;
   ccoef[nc + ic] = up;
   ccoef[2 * nc + ic] = dn;
-  ccoef[3 * nc + ic] = top ? -y4d : y4u;
-  ccoef[4 * nc + ic] = top ? -x5d : x5u;
-  ccoef[5 * nc + ic] = top ? -x7d : x7u;
-  ccoef[6 * nc + ic] = top ? -y8d : y8u;
-  ccxr[ic] = xp;
-  ccyr[ic] = yp;
+  const T c4 = top ? -y4d : y4u, c5 = top ? -x5d : x5u, c7 = top ? -x7d : x7u, c8 = top ? -y8d : y8u;
+  ccoef[3 * nc + ic] = c4;
+  ccoef[4 * nc + ic] = c5;
+  ccoef[5 * nc + ic] = c7;
+  ccoef[6 * nc + ic] = c8;
+  if (csp) {   // colour-split copy (MGL::sp)
+    const int Mh = (Mc + 1) >> 1;
+    const size_t nmh = (size_t)Mh * Nc, cs = nmh * K;
+    T* e = csp + (size_t)((I + J) & 1) * cs + nmh * k + (size_t)Mh * J + (I >> 1);
+    e[6 * cs] = c4;
+    e[8 * cs] = c5;
+    e[10 * cs] = c7;
+    e[12 * cs] = c8;
+  }
 }
 
 // line factors of one level (C13, C1, C6), one column per thread
 template <class T>
-__global__ void __launch_bounds__(256) k_mg_factor(MGL<T> L, T* lcp, T* linv) {
+__global__ void __launch_bounds__(256) k_mg_factor(MGL<T> L, T* lcp, T* linv, T* sp) {
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= L.M * L.N) return;
   const int MN = L.M * L.N, n = L.n;
@@ -792,6 +818,14 @@ __global__ void __launch_bounds__(256) k_mg_factor(MGL<T> L, T* lcp, T* linv) {
     cpm = c * inv;
     lcp[ic] = cpm;
     linv[ic] = inv;
+    if (sp) {   // colour-split copy (MGL::sp)
+      const int jj = col / L.M, ii = col - jj * L.M, Mh = (L.M + 1) >> 1;
+      const size_t nmh = (size_t)Mh * L.N, cs = nmh * L.K;
+      T* e = sp + (size_t)((ii + jj) & 1) * cs + nmh * k + (size_t)Mh * jj + (ii >> 1);
+      e[0] = a;
+      e[2 * cs] = inv;
+      e[4 * cs] = cpm;
+    }
   }
 }
 

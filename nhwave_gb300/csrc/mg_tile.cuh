@@ -96,16 +96,14 @@ __device__ __forceinline__ void line_solve_smem(T* __restrict__ x, const T* __re
 }
 
 // The operator of one level at a column of colour c: line factors, cross
-// terms and in-level couplings.  Level 0 (kFine) reads the colour-split copy
-// and constant in-level couplings, coarse levels the natural layout.
+// terms and in-level couplings.  Level 0 (kFine) reads the colour-split copy,
+// coarse levels the natural layout.
 template <class T, bool kFine>
 struct TileOp {
   const T *a_, *inv_, *cp_, *x_;   // C13, 1/den, c/den, first cross term at level 0
-  const T *cx_, *cy_;
   T cxx, cyy;
-  int sk, M;
+  int sk;
   size_t ss;                       // stride of a cross term
-  bool im, jm;
   __device__ __forceinline__ TileOp(const MGL<T>& L, int color, int ii, int jj) {
     if (kFine) {
       const int Mh = (L.M + 1) >> 1, nmh = Mh * L.N;
@@ -113,17 +111,15 @@ struct TileOp {
       a_ = L.sp + (size_t)color * cs + (Mh * jj + (ii >> 1));
       ss = 2 * cs;
       inv_ = a_ + ss; cp_ = inv_ + ss; x_ = cp_ + ss;
-      cxx = L.cxx; cyy = L.cyy;
       sk = nmh;
     } else {
       const int c = ii + L.M * jj;
       ss = (size_t)L.n;
       a_ = L.coef + 2 * ss + c; x_ = a_ + ss;
       inv_ = L.linv + c; cp_ = L.lcp + c;
-      cx_ = L.cxr + c; cy_ = L.cyr + c;
-      im = ii > 0; jm = jj > 0;
-      sk = L.M * L.N; M = L.M;
+      sk = L.M * L.N;
     }
+    cxx = cx_of(L, jj); cyy = cy_of(L, ii);
   }
   __device__ __forceinline__ T inv(int k) const { return inv_[sk * k]; }
   __device__ __forceinline__ T cp(int k) const { return cp_[sk * k]; }
@@ -133,16 +129,8 @@ struct TileOp {
   __device__ __forceinline__ void couplings(int k, T (&g)[8]) const {
     const T* f = x_ + sk * k;
     g[7] = f[0]; g[5] = f[ss]; g[4] = f[2 * ss]; g[6] = f[3 * ss];
-    if (kFine) {
-      g[0] = g[1] = cxx;
-      g[2] = g[3] = cyy;
-    } else {
-      const T *cx = cx_ + sk * k, *cy = cy_ + sk * k;
-      g[0] = cx[0];
-      g[1] = im ? cx[-1] : (T)0;
-      g[2] = cy[0];
-      g[3] = jm ? cy[-M] : (T)0;
-    }
+    g[0] = g[1] = cxx;
+    g[2] = g[3] = cyy;
   }
 };
 // Off-column part of A x at a slot from the couplings g and the other
@@ -502,10 +490,11 @@ struct CycleLevel {
           a[c][t] = k[t] > 0 ? cf[2 * n0] : (T)0;
           v[c][t] = L.linv[ic];
           p[c][t] = L.lcp[ic];
-          if (ip) { g[c][t][0] = cx_p(L, ic); g[c][t][4] = cf[5 * n0]; }
-          if (im) { g[c][t][1] = cx_m(L, ic); g[c][t][5] = cf[4 * n0]; }
-          if (jp) { g[c][t][2] = cy_p(L, ic); g[c][t][6] = cf[6 * n0]; }
-          if (jm) { g[c][t][3] = cy_m(L, ic); g[c][t][7] = cf[3 * n0]; }
+          const T cx = cx_of(L, jj[t]), cy = cy_of(L, ii[c][t]);
+          if (ip) { g[c][t][0] = cx; g[c][t][4] = cf[5 * n0]; }
+          if (im) { g[c][t][1] = cx; g[c][t][5] = cf[4 * n0]; }
+          if (jp) { g[c][t][2] = cy; g[c][t][6] = cf[6 * n0]; }
+          if (jm) { g[c][t][3] = cy; g[c][t][7] = cf[3 * n0]; }
         }
       }
     }

@@ -132,10 +132,11 @@ __device__ __forceinline__ T ps_off_column(const MGL<T>& L, const T* x, const Pr
   const int M = L.M, MN = L.M * L.N, n = L.n;
   const bool im = ii > 0, ip = ii < L.M - 1, jm = jj > 0, jp = jj < L.N - 1, km = kk > 0, kp = kk < L.K - 1;
   T s = (T)0;
-  if (ip) s += cx_p(L, ic) * ps_xval(x, P, ic + 1);
-  if (im) s += cx_m(L, ic) * ps_xval(x, P, ic - 1);
-  if (jp) s += cy_p(L, ic) * ps_xval(x, P, ic + M);
-  if (jm) s += cy_m(L, ic) * ps_xval(x, P, ic - M);
+  const T cx = cx_of(L, jj), cy = cy_of(L, ii);
+  if (ip) s += cx * ps_xval(x, P, ic + 1);
+  if (im) s += cx * ps_xval(x, P, ic - 1);
+  if (jp) s += cy * ps_xval(x, P, ic + M);
+  if (jm) s += cy * ps_xval(x, P, ic - M);
   const T c4 = L.coef[3 * n + ic], c5 = L.coef[4 * n + ic], c7 = L.coef[5 * n + ic], c8 = L.coef[6 * n + ic];
   if (kp) {
     const int u = ic + MN;

@@ -423,8 +423,9 @@ class Solver final : public SolverBase {
     for (size_t l = 1; l < mg.size(); ++l) {
       const size_t nl = (size_t)mg[l].n;
       add((T**)&mg[l].coef, sizeof(T) * NCOMPACT * nl);
-      add((T**)&mg[l].cxr, sizeof(T) * nl);
-      add((T**)&mg[l].cyr, sizeof(T) * nl);
+      // levels above the tiles' size take the half-sweeps of level 0
+      if (!tiled(mg[l]) && (long long)mg[l].M * mg[l].N > cta_columns)
+        add((T**)&mg[l].sp, sizeof(T) * 7 * 2 * (size_t)K * mg[l].N * ((mg[l].M + 1) / 2));
       add((T**)&mg[l].lcp, sizeof(T) * nl);
       add((T**)&mg[l].linv, sizeof(T) * nl);
       add(&mg[l].x, sizeof(T) * nl);
@@ -485,9 +486,10 @@ class Solver final : public SolverBase {
     // everything a step carries to the next lies in front of the Poisson scratch
     state_bytes = (size_t)((char*)(S.P + n3) - arena);
     if (!kFP32) S.coefT = (T*)S.coef64;
-    mg[0].coef = S.coefT; mg[0].cxr = nullptr; mg[0].cyr = nullptr;
+    mg[0].coef = S.coefT;
     mg[0].lcp = S.lcp; mg[0].linv = S.linv; mg[0].sp = S.sp0;
-    for (auto& L : mg) { L.cxx = (T)S.cxx; L.cyy = (T)S.cyy; }
+    mg[0].cxx = mg[0].cxl = (T)S.cxx; mg[0].cyy = mg[0].cyl = (T)S.cyy;
+    for (size_t l = 1; l < mg.size(); ++l) coarse_couplings(mg[l - 1], mg[l]);
     {
       const int shm = (int)(sizeof(T) * 4 * 32 * 64);
       NHW_CU(cudaFuncSetAttribute(k_mg_smooth_blk<T, true, MgB<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
@@ -1121,9 +1123,11 @@ class Solver final : public SolverBase {
         MGL<T>& c = mg[l];
         const int bg = block_of(c.n), bf = block_of((long long)c.M * c.N);
         L("mg_galerkin", [&] {
-          k_mg_galerkin<T><<<cdiv(c.n, bg), bg, 0, st>>>(f, (T*)c.coef, (T*)c.cxr, (T*)c.cyr, c.M, c.N);
+          k_mg_galerkin<T><<<cdiv(c.n, bg), bg, 0, st>>>(f, (T*)c.coef, (T*)c.sp, c.M, c.N);
         });
-        L("mg_factor", [&] { k_mg_factor<T><<<cdiv((long long)c.M * c.N, bf), bf, 0, st>>>(c, (T*)c.lcp, (T*)c.linv); });
+        L("mg_factor", [&] {
+          k_mg_factor<T><<<cdiv((long long)c.M * c.N, bf), bf, 0, st>>>(c, (T*)c.lcp, (T*)c.linv, (T*)c.sp);
+        });
       }
       cudaEventRecord(ev_join, st);
       st = main_st;
@@ -1300,7 +1304,7 @@ class Solver final : public SolverBase {
     const int by = std::min(Lv.K, 32);
     const size_t shm = sizeof(T) * 4 * 32 * Lv.K;
     L(names[level < 7 ? level : 7], [&] {
-      if (Lv.sp) {   // level 0: colour-split operator
+      if (Lv.sp) {   // colour-split operator
         const long long nq = (long long)((Lv.M + 1) / 2) * Lv.N;
         if constexpr (kFP32) {
           // one thread per column and chunk of kSplitLevels levels: short

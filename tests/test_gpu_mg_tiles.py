@@ -59,3 +59,16 @@ def test_tiled_levels_step_like_the_oracle(shape, precision, oracle_mod, gpu_lib
     p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
     po, _, _ = _case(*shape, 0, 1e-13)
     _against_oracle(p, po, depth, eta, oracle_mod)
+
+
+# second levels above the tiles' size, which take the colour-split half-sweeps: odd sides, a last aggregate of one row
+# or column, a height that is no multiple of the four levels a thread has, and one above 8192 columns
+SPLIT = [(133, 130, 5), (259, 129, 1), (131, 127, 9)]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", SPLIT, ids=lambda s: "x".join(map(str, s)))
+def test_split_coarse_levels_step_like_the_oracle(shape, precision, oracle_mod, gpu_lib):
+    p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
+    po, _, _ = _case(*shape, 0, 1e-13)
+    _against_oracle(p, po, depth, eta, oracle_mod)
