@@ -188,8 +188,9 @@ __device__ __forceinline__ void finish_reduce_of(const Dev<T>& S, double* part, 
   __threadfence();
   double acc[NV];
   for (int q = 0; q < NV; ++q) acc[q] = 0.0;
+#pragma unroll 4
   for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    for (int q = 0; q < NV; ++q) acc[q] += ((volatile double*)part)[(size_t)b * stride + q];
+    for (int q = 0; q < NV; ++q) acc[q] += __ldcg(part + (size_t)b * stride + q);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   for (int q = 0; q < NV; ++q)
     for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
@@ -247,7 +248,7 @@ struct FinRes {
       sc->conv = 0;
       sc->solves = sc->solves + 1;
     }
-    sc->bnorm = sqrt(a[1]);
+    if (kFirst) sc->bnorm = sqrt(a[1]);
     const double rel = sc->bnorm > 0.0 ? sqrt(a[0]) / sc->bnorm : 0.0;
     sc->relres64 = rel;
     int go = 0, st = 0;
@@ -290,10 +291,12 @@ struct FinInit {
 };
 template <class T>
 struct FinV {
+  double rho;   // read when the kernel starts, so that its end does not wait for it
+  __device__ explicit FinV(const DevScal* sc) : rho(sc->rho) {}
   __device__ void operator()(const Dev<T>& S2, double* a) const {
     DevScal* sc = S2.sc;
     if (a[0] == 0.0 || !(a[0] == a[0])) { sc->conv = 2; return; }
-    sc->alpha = sc->rho / a[0];
+    sc->alpha = rho / a[0];
   }
 };
 template <class T>
@@ -305,22 +308,25 @@ struct FinT {
 };
 template <class T>
 struct FinXr {
+  double tol_in, red, rho, alpha, omega;   // read when the kernel starts
+  int itmax_in, it, total_it, inner_total;
+  __device__ explicit FinXr(const DevScal* sc)
+      : tol_in(sc->tol_in), red(sc->red[0]), rho(sc->rho), alpha(sc->alpha), omega(sc->omega),
+        itmax_in(sc->itmax_in), it(sc->it + 1), total_it(sc->total_it + 1), inner_total(sc->inner_total + 1) {}
   __device__ void operator()(const Dev<T>& S2, double* a) const {
     DevScal* sc = S2.sc;
-    const double tol_in = sc->tol_in;
-    const int itmax_in = sc->itmax_in;
-    sc->it = sc->it + 1;
-    sc->total_it = sc->total_it + 1;
-    sc->inner_total = sc->inner_total + 1;
-    const double rel = sc->red[0] > 0.0 ? sqrt(a[1]) / sc->red[0] : 0.0;
+    sc->it = it;
+    sc->total_it = total_it;
+    sc->inner_total = inner_total;
+    const double rel = red > 0.0 ? sqrt(a[1]) / red : 0.0;
     sc->relres = rel;
     int conv = 0;
     if (!(rel == rel)) conv = 5;
     else if (rel <= tol_in) conv = 1;
-    else if (sc->it >= itmax_in) conv = 4;
-    else if (a[0] == 0.0 || sc->omega == 0.0) conv = 2;
+    else if (it >= itmax_in) conv = 4;
+    else if (a[0] == 0.0 || omega == 0.0) conv = 2;
     else {
-      sc->beta = (a[0] / sc->rho) * (sc->alpha / sc->omega);
+      sc->beta = (a[0] / rho) * (alpha / omega);
       sc->rho = a[0];
     }
     sc->conv = conv;
@@ -342,7 +348,8 @@ __global__ void __launch_bounds__(256) k_res64(Dev<T> S) {
   if (gated_off(S)) return;
   const int M = S.M, N = S.N, K = S.K;
   const size_t n = (size_t)S.neq;
-  double v[2] = {0.0, 0.0};
+  constexpr int NV = kFirst ? 2 : 1;   // later sweeps know ||b||
+  double v[NV] = {};
 #pragma unroll
   for (int q = 0; q < kCPT; ++q) {
     const int ic = (blockIdx.x * kCPT + q) * blockDim.x + threadIdx.x;
@@ -352,14 +359,14 @@ __global__ void __launch_bounds__(256) k_res64(Dev<T> S) {
       const double b = S.rhs64[ic];
       const double r = b - spmv_c<double, double>(S.coef64, S.xsol64, n, ic, ii, jj, kk, M, N, K, S.cxx, S.cyy);
       S.res64[ic] = r;
-      S.kr0[ic] = (T)r;
+      S.kr0[ic] = narrow<T>(r);
       v[0] += r * r;
-      v[1] += b * b;
+      if (kFirst) v[NV - 1] += b * b;
     }
   }
-  double out[2];
-  block_sum_t<2, double>(v, out);
-  finish_reduce<2>(S, out, FinRes<T, kFirst>{});
+  double out[NV];
+  block_sum_t<NV, double>(v, out);
+  finish_reduce<NV>(S, out, FinRes<T, kFirst>{});
 }
 
 // start of an inner solve from c = 0: r = r0 = rT, p = v = 0, rho = (r, r)
@@ -476,6 +483,7 @@ __global__ void __launch_bounds__(128) k_bicg_s(Dev<T> S) {
 template <class T>
 __global__ void __launch_bounds__(256) k_bicg_v(Dev<T> S) {
   if (S.sc->conv) return;
+  const FinV<T> fin(S.sc);
   using A = typename Acc<T>::type;
   A v[1] = {(A)0};
   const T* __restrict__ ph = S.kph;
@@ -504,7 +512,7 @@ __global__ void __launch_bounds__(256) k_bicg_v(Dev<T> S) {
   }
   double out[1];
   block_sum_t<1, A>(v, out);
-  finish_reduce<1>(S, out, FinV<T>{});
+  finish_reduce<1>(S, out, fin);
 }
 
 // t = A sh; omega = (t, s) / (t, t)
@@ -554,7 +562,8 @@ __global__ void __launch_bounds__(256) k_bicg_xr(Dev<T> S) {
     return;
   }
   using A = typename Acc<T>::type;
-  const T alpha = (T)S.sc->alpha, omega = (T)S.sc->omega;
+  const FinXr<T> fin(S.sc);
+  const T alpha = (T)fin.alpha, omega = (T)fin.omega;
   A v[2] = {(A)0, (A)0};
   T* __restrict__ x = S.kx;
   T* __restrict__ rr = S.kr;
@@ -577,7 +586,7 @@ __global__ void __launch_bounds__(256) k_bicg_xr(Dev<T> S) {
   }
   double out[2];
   block_sum_t<2, A>(v, out);
-  finish_reduce<2>(S, out, FinXr<T>{});
+  finish_reduce<2>(S, out, fin);
 }
 
 // x64 += c
@@ -621,7 +630,7 @@ __device__ __forceinline__ void sliced_reduce(const Dev<T>& S, int blk, int nblk
 template <class T, bool kFirst>
 __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_res64_sl(Dev<T> S) {
   if (gated_off(S)) return;
-  __shared__ double sr[256], sb[256];
+  __shared__ double sr[256], sb[kFirst ? 256 : 1];
   auto cl = cooperative_groups::this_cluster();
   const int blk = blockIdx.x / kSlices, q0 = (int)cl.block_rank(), tid = threadIdx.x;
   const int base = blk * kCPT * 256 + tid, ic = base + q0 * 256;
@@ -632,15 +641,19 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_res64_s
     const double r = b - spmv_c<double, double>(S.coef64, S.xsol64, (size_t)S.neq, ic, ii, jj, kk, S.M, S.N, S.K,
                                                 S.cxx, S.cyy);
     S.res64[ic] = r;
-    S.kr0[ic] = (T)r;
+    S.kr0[ic] = narrow<T>(r);
     sr[tid] = r;
-    sb[tid] = b;
+    if (kFirst) sb[tid] = b;
   }
-  sliced_reduce<2, double>(S, blk, gridDim.x / kSlices, kCPT, [&](int q, double (&v)[2]) {
+  constexpr int NV = kFirst ? 2 : 1;   // later sweeps know ||b||
+  sliced_reduce<NV, double>(S, blk, gridDim.x / kSlices, kCPT, [&](int q, double (&v)[NV]) {
     if (base + q * 256 < S.neq) {
-      const double r = cl.map_shared_rank(sr, q)[tid], b = cl.map_shared_rank(sb, q)[tid];
+      const double r = cl.map_shared_rank(sr, q)[tid];
       v[0] += r * r;
-      v[1] += b * b;
+      if (kFirst) {
+        const double b = cl.map_shared_rank(sb, q)[tid];
+        v[NV - 1] += b * b;
+      }
     }
   }, FinRes<T, kFirst>{});
 }
@@ -708,9 +721,10 @@ __device__ __forceinline__ void sliced_matvec(const Dev<T>& S, const T* __restri
 template <class T>
 __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_v_sl(Dev<T> S) {
   if (S.sc->conv) return;
+  const FinV<T> fin(S.sc);
   using A = typename Acc<T>::type;
   const T* __restrict__ r0 = S.kr0;
-  sliced_matvec<1>(S, S.kph, S.kv, [&](int ic, T y, A (&v)[1]) { v[0] += (A)r0[ic] * (A)y; }, FinV<T>{});
+  sliced_matvec<1>(S, S.kph, S.kv, [&](int ic, T y, A (&v)[1]) { v[0] += (A)r0[ic] * (A)y; }, fin);
 }
 template <class T>
 __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_t_sl(Dev<T> S) {
@@ -733,7 +747,8 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_xr
   auto cl = cooperative_groups::this_cluster();
   const int blk = blockIdx.x / kSlices, tid = threadIdx.x;
   const int base = blk * kCPT * 256 + tid, ic = base + (int)cl.block_rank() * 256;
-  const T alpha = (T)S.sc->alpha, omega = (T)S.sc->omega;
+  const FinXr<T> fin(S.sc);
+  const T alpha = (T)fin.alpha, omega = (T)fin.omega;
   if (ic < S.neq) {
     S.kx[ic] = S.kx[ic] + alpha * S.kph[ic] + omega * S.ksh[ic];
     const T r = S.ks[ic] - omega * S.kt[ic];
@@ -748,7 +763,7 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_xr
       v[0] += (A)r0[base + q * 256] * (A)r;
       v[1] += (A)r * (A)r;
     }
-  }, FinXr<T>{});
+  }, fin);
 }
 
 // ------------------------------------------------------------------ GMRES
