@@ -1076,7 +1076,8 @@ __global__ void __launch_bounds__(128) k_flux_z_walk(Dev<T> S, int kc) {
   }
 }
 
-// Faces across x (y) of the FP64 form.  A block has 256 cells of a row (16 rows
+// Faces across x (y) of the FP64 form, and across y on large grids of the
+// FP32+IR form.  A block has 256 cells of a row (16 rows
 // of 32 cells) and walks kc levels: each cell forms its difference quotients
 // once, takes the lower neighbour's from shared memory for its limited slopes,
 // and hands its upper face's left states to the next cell.  Face by face the
@@ -1103,7 +1104,7 @@ k_faces(Dev<T> S, int kc, int ntile, int nrow) {
   const bool cell = c <= last && (kX || x <= S.IE), face = cell && pos >= 2;
   const int i = kX ? c : x, j = kX ? x : c;
   const long long step = kX ? 1 : S.sy, o0 = i3(S, i, j, 0);
-  const R h = kX ? S.dxT : S.dyT, hd = kX ? S.hdxT : S.hdyT;
+  const R h = kX ? S.dxT : S.dyT, ih = kX ? S.idxT : S.idyT, hd = kX ? S.hdxT : S.hdyT;
   const bool wet = cell && S.Mask[i2(S, i, j)] != 0;
   Face F;
   if (face) F.load(S, i, j, k0 == S.KB);
@@ -1114,7 +1115,7 @@ k_faces(Dev<T> S, int kc, int ntile, int nrow) {
       for (int m = 0; m < NF; ++m) {
         const T* A = Face::field(S, m) + o0 + S.sz * k;
         a[m] = A[0];
-        q[m] = (A[step] - a[m]) / h;
+        q[m] = sizeof(R) == 4 ? (A[step] - a[m]) * ih : (A[step] - a[m]) / h;
         sq[m][me] = q[m];
       }
     }
@@ -1125,9 +1126,14 @@ k_faces(Dev<T> S, int kc, int ntile, int nrow) {
         const R t2 = sq[m][before];
         R s = (R)0;
         if (wet && !((fabs(q[m]) + fabs(t2)) < (R)kSmall)) s = limiter(q[m], t2);
-        s = hd * s;
-        sl[m][me] = a[m] + s;
-        a[m] = a[m] - s;
+        if constexpr (sizeof(R) == 4) {
+          sl[m][me] = fmaf(hd, s, a[m]);
+          a[m] = fmaf(-hd, s, a[m]);
+        } else {
+          s = hd * s;
+          sl[m][me] = a[m] + s;
+          a[m] = a[m] - s;
+        }
       }
     }
     __syncthreads();

@@ -1046,8 +1046,14 @@ class Solver final : public SolverBase {
   // The FP64 form's face kernels share quotients and slopes between faces in
   // blocks; below about 2^16 cells the FP64 pipes are not full and a face a
   // thread has the shorter chain (256 x 8 x 10, all five: 156 against 169 us).
-  // FP32+IR multiplies by reciprocals and keeps a face a thread.
-  bool face_blocks() const { return !kFP32 && S.neq >= 65536; }
+  // FP32+IR, which multiplies by reciprocals, keeps a face a thread across x
+  // (1024 x 64 x 20: flux_x 49.5 us against 61.2, 768 x 768 x 20: 467 against
+  // 509); across y, where a face a thread reads each row four times, blocks
+  // pay from about 2^20 cells (flux_y + omega_y 515 x 30 x 15: 28.7 against
+  // 33.3 us in blocks, 1024 x 64 x 20: 86.0 against 76.5, 768 x 768 x 20: 758
+  // against 545).
+  bool face_blocks_x() const { return !kFP32 && S.neq >= 65536; }
+  bool face_blocks_y() const { return S.neq >= (kFP32 ? 1 << 20 : 65536); }
   // as few chunks of levels as leave about 8 blocks an SM
   template <class Face>
   void faces() {
@@ -1070,15 +1076,16 @@ class Solver final : public SolverBase {
   int fluxes() override {
     allcols(OpSlopeEta{});
     if (S.fxT) box(OpFacePrep{0}, S.M + 1, S.N + 1, 1, S.IB, S.JB, 0);
-    if (!face_blocks()) {
+    if constexpr (kFP32) {
       box(OpFluxX{}, S.M + 1, S.N, S.K, S.IB, S.JB, S.KB);
-      box(OpFluxY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
-      box(OpFluxZ{}, S.M, S.N, S.K + 1, S.IB, S.JB, S.KB);
-    } else if constexpr (!kFP32) {
-      faces<FluxXFace<T>>();
-      faces<FluxYFace<T>>();
-      flux_z_walk();
+    } else {
+      if (face_blocks_x()) faces<FluxXFace<T>>();
+      else box(OpFluxX{}, S.M + 1, S.N, S.K, S.IB, S.JB, S.KB);
     }
+    if (face_blocks_y()) faces<FluxYFace<T>>();
+    else box(OpFluxY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
+    if (kFP32 || !face_blocks_x()) box(OpFluxZ{}, S.M, S.N, S.K + 1, S.IB, S.JB, S.KB);
+    else if constexpr (!kFP32) flux_z_walk();
     if (S.keDxW) cells(OpKeSlopes{0});   // delxyzFun's DelxW / DelyW, read by the 3-D k-epsilon
     return check();
   }
@@ -1499,13 +1506,14 @@ class Solver final : public SolverBase {
     cells(OpSSP{s});
     get_uvw();
     if (S.fxT) box(OpFacePrep{1}, S.M + 1, S.N + 1, 1, S.IB, S.JB, 0);
-    if (!face_blocks()) {
+    if constexpr (kFP32) {
       box(OpOmegaX{}, S.M + 1, S.N, S.K, S.IB, S.JB, S.KB);
-      box(OpOmegaY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
-    } else if constexpr (!kFP32) {
-      faces<OmegaXFace<T>>();
-      faces<OmegaYFace<T>>();
+    } else {
+      if (face_blocks_x()) faces<OmegaXFace<T>>();
+      else box(OpOmegaX{}, S.M + 1, S.N, S.K, S.IB, S.JB, S.KB);
     }
+    if (face_blocks_y()) faces<OmegaYFace<T>>();
+    else box(OpOmegaY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
     incols(OpOmegaScan{});
     if (S.keDxU) cells(OpKeSlopes{1});   // get_Omega's DelxU .. DelyV, before sponge_damping
   }

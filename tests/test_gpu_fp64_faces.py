@@ -49,3 +49,45 @@ def test_faces_bit_exact(grid, hllc, oracle_mod, gpu_lib):
             a, b = g.get(f)[sl(f)], o.get(f)[sl(f)]
             assert np.array_equal(a, b), f"{n} stage {s}: max |d| {np.abs(a - b).max():.3e}"
     g.close()
+
+
+# FP32+IR, which takes the blocks across y from 2^20 cells on: 14 faces a block and a remainder, columns that are no
+# multiple of 32, levels that do not divide into the chunks.  A flux is some twenty roundings of 2^-24 of terms no larger
+# than the field's largest, limited slopes included (1.2e-6); Omega's face values are two limited slopes.
+FP32_GRIDS = [(1090, 55, 18), (33, 2000, 16)]
+
+
+@pytest.mark.parametrize("hllc", [0, 1])
+@pytest.mark.parametrize("grid", FP32_GRIDS, ids=lambda g: "x".join(map(str, g)))
+def test_fp32_y_faces(grid, hllc, oracle_mod, gpu_lib):
+    from nhwave_gb300 import default_params, fields as F, lib
+    M, N, K = grid
+    assert M * N * K >= 1 << 20
+    x, y = np.arange(M)[None, :], np.arange(N)[:, None]
+    depth = 1.5 + 0.3 * np.sin(0.03 * x) * np.cos(0.05 * y)
+    eta = 0.1 * np.sin(0.13 * x + 0.21 * y)
+    uvw = (0.2 * np.random.default_rng(4).standard_normal((3, K, N, M))).astype(np.float32).astype(np.float64)
+    hs = []
+    for prec, make in ((1, lib.Scenario), (0, oracle_mod.Oracle)):
+        p = default_params(Mglob=M, Nglob=N, Kglob=K, dx=0.7, dy=0.9, dt_ini=0.01, non_hydro=0, hllc=hllc)
+        p.precision = prec
+        hs.append(make(p, depth.ravel(), eta.ravel(), uvw.ravel()))
+    g, o = hs
+    sl = o.shape.interior
+    for h in hs:
+        assert h.estimate_dt() == 0
+        h.update_mask()
+        h.update_vars()
+        h.source_terms()
+        h.fluxes()
+    for n in ("EY", "FY", "GY", "HY"):
+        f = getattr(F, n)
+        a, b = g.get(f)[sl(f)], o.get(f)[sl(f)]
+        assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max(), n
+    for h in hs:
+        h.eval_duvw(1)
+    for n in ("OMEGA", "ETAYL", "ETAYR", "V"):
+        f = getattr(F, n)
+        a, b = g.get(f)[sl(f)], o.get(f)[sl(f)]
+        assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max(), n
+    g.close()
