@@ -1831,59 +1831,71 @@ struct OpKeTop {
 // HLPA face value (src/nhwave.F:7809-7847): the upstream value Fw and, where
 // the profile is monotone (|Fp - 2 Fw + Fww| < |Fp - Fww|), its correction,
 // whose division the other (finite) faces skip
+// The magnitudes are compared as bit patterns, whose order is theirs: a
+// comparison in FP64 takes as long as any FP64 operation.
 __device__ __forceinline__ double ke_hlpa_side(double Fww, double Fw, double Fp) {
   const double d = Fp - Fww, c = fabs(Fp - 2.0 * Fw + Fww);
-  if (fabs(d) <= (double)1.e-16f || (c >= fabs(d) && c <= 1.0e300)) return Fw;
-  const double a = c < fabs(d) ? 1.0 : 0.0;
+  const long long db = __double_as_longlong(fabs(d)), cb = __double_as_longlong(c);
+  if (db <= __double_as_longlong((double)1.e-16f) || (cb >= db && cb <= __double_as_longlong(1.0e300))) return Fw;
+  const double a = cb < db && db <= 0x7ff0000000000000ll ? 1.0 : 0.0;   // 0 where one is not a number
   return Fw + a * (Fp - Fw) * (Fw - Fww) / d;
 }
-__device__ __forceinline__ double ke_hlpa(double Uw, double Fww, double Fw, double Fp, double Fe) {
-  if (Uw >= 0.0) return ke_hlpa_side(Fww, Fw, Fp);
-  if (Uw < 0.0) return ke_hlpa_side(Fe, Fp, Fw);
+template <class V>
+__device__ __forceinline__ double ke_hlpa(V Uw, double Fww, double Fw, double Fp, double Fe) {
+  if (Uw >= (V)0) return ke_hlpa_side(Fww, Fw, Fp);
+  if (Uw < (V)0) return ke_hlpa_side(Fe, Fp, Fw);
   return 0.0;
 }
 
-// adv_scalar_hlpa with flux_scalar_bc (src/nhwave.F:7604-7806, 7850-7986) at
-// one interior cell: minus the divergence of the HLPA fluxes of Phi by Ex,
-// Ey and Omega (the boundary scalar of a BC_X0 = 3 side is zero; faces of
-// dry cells carry none) plus the horizontal diffusion with Cmu + CmuHt /
-// SchtH; zero in a dry cell
+// HLPA fluxes of flux_scalar_bc (src/nhwave.F:7850-7986) through the lower
+// faces f of a cell in x, y and sigma, by Ex, Ey and Omega: the boundary
+// scalar of a BC_X0 = 3 side is zero, faces of dry cells carry none
 template <class T>
-__device__ double ke_r5(const Dev<T>& S, int i, int j, int k, const T* Phi, double SchtH) {
+__device__ __forceinline__ double ke_flux_x(const Dev<T>& S, int f, int j, int k, const T* Phi) {
+  if ((f <= S.IE && S.Mask[i2(S, f, j)] == 0) || (f - 1 >= S.IB && S.Mask[i2(S, f - 1, j)] == 0)) return 0.0;
+  if (f == S.IE + 1) return 0.0;
+  const long long o = i3(S, f, j, k);
+  const T uT = S.Ex[o];
+  const double u = widen(uT);
+  if (f == S.IB) {
+    if (S.bc_x0 == 1 || S.bc_x0 == 2 || S.bc_x0 == 5) return 0.0;
+    if (S.bc_x0 == 3) return u * 0.0;
+  }
+  return u * ke_hlpa(uT, widen(Phi[o - 2]), widen(Phi[o - 1]), widen(Phi[o]), widen(Phi[o + 1]));
+}
+template <class T>
+__device__ __forceinline__ double ke_flux_y(const Dev<T>& S, int i, int f, int k, const T* Phi) {
+  if ((f <= S.JE && S.Mask[i2(S, i, f)] == 0) || (f - 1 >= S.JB && S.Mask[i2(S, i, f - 1)] == 0)) return 0.0;
+  if (f == S.JB && (S.bc_y0 == 1 || S.bc_y0 == 2 || S.bc_y0 == 5)) return 0.0;
+  if (f == S.JE + 1 && (S.bc_yn == 1 || S.bc_yn == 2 || S.bc_yn == 5)) return 0.0;
+  const long long o = i3(S, i, f, k);
+  const long long y = S.sy;
+  const T vT = S.Ey[o];
+  return widen(vT) * ke_hlpa(vT, widen(Phi[o - 2 * y]), widen(Phi[o - y]), widen(Phi[o]), widen(Phi[o + y]));
+}
+template <class T>
+__device__ __forceinline__ double ke_flux_z(const Dev<T>& S, int i, int j, int f, const T* Phi) {
+  if (f == S.KB || f == S.KE + 1) return 0.0;
+  const long long o = i3(S, i, j, f);
+  const long long z = S.sz;
+  const T wT = S.Omega[o];
+  return widen(wT) * ke_hlpa(wT, widen(Phi[o - 2 * z]), widen(Phi[o - z]), widen(Phi[o]), widen(Phi[o + z]));
+}
+
+// adv_scalar_hlpa (src/nhwave.F:7604-7806) at one interior cell from the
+// fluxes through its x and sigma faces: minus the divergence of the fluxes of
+// Phi plus the horizontal diffusion with Cmu + CmuHt / SchtH; zero in a dry
+// cell
+template <class T>
+__device__ double ke_r5(const Dev<T>& S, int i, int j, int k, const T* Phi, Quot<T> Sc, double fx0, double fx1,
+                        double fz0, double fz1) {
   if (S.Mask[i2(S, i, j)] == 0) return 0.0;
-  auto scx = [&](int f) -> double {
-    if ((f <= S.IE && S.Mask[i2(S, f, j)] == 0) || (f - 1 >= S.IB && S.Mask[i2(S, f - 1, j)] == 0)) return 0.0;
-    if (f == S.IE + 1) return 0.0;
-    const long long o = i3(S, f, j, k);
-    const double u = (double)S.Ex[o];
-    if (f == S.IB) {
-      if (S.bc_x0 == 1 || S.bc_x0 == 2 || S.bc_x0 == 5) return 0.0;
-      if (S.bc_x0 == 3) return u * 0.0;
-    }
-    return u * ke_hlpa(u, (double)Phi[o - 2], (double)Phi[o - 1], (double)Phi[o], (double)Phi[o + 1]);
-  };
-  auto scy = [&](int f) -> double {
-    if ((f <= S.JE && S.Mask[i2(S, i, f)] == 0) || (f - 1 >= S.JB && S.Mask[i2(S, i, f - 1)] == 0)) return 0.0;
-    if (f == S.JB && (S.bc_y0 == 1 || S.bc_y0 == 2 || S.bc_y0 == 5)) return 0.0;
-    if (f == S.JE + 1 && (S.bc_yn == 1 || S.bc_yn == 2 || S.bc_yn == 5)) return 0.0;
-    const long long o = i3(S, i, f, k);
-    const long long y = S.sy;
-    const double v = (double)S.Ey[o];
-    return v * ke_hlpa(v, (double)Phi[o - 2 * y], (double)Phi[o - y], (double)Phi[o], (double)Phi[o + y]);
-  };
-  auto scz = [&](int f) -> double {
-    if (f == S.KB || f == S.KE + 1) return 0.0;
-    const long long o = i3(S, i, j, f);
-    const long long z = S.sz;
-    const double w = (double)S.Omega[o];
-    return w * ke_hlpa(w, (double)Phi[o - 2 * z], (double)Phi[o - z], (double)Phi[o], (double)Phi[o + z]);
-  };
   const double cmu = S.v_cmu;
-  const Quot<T> Sc = over<T>(SchtH), dx2 = over<T>(S.dx * S.dx), dy2 = over<T>(S.dy * S.dy);
+  const Quot<T> dx2{S.dx * S.dx, -S.cxx}, dy2{S.dy * S.dy, -S.cyy};   // cxx = -1 / dx^2
   auto nu = [&](double ha, double hb) { return 0.5 * (cmu + cmu) + 0.5 * (ha + hb) / Sc; };
-  auto H = [&](int ii, int jj) { return (double)S.CmuHt[i3(S, ii, jj, k)]; };
+  auto H = [&](int ii, int jj) { return widen(S.CmuHt[i3(S, ii, jj, k)]); };
   auto Dq = [&](int ii, int jj) { return S.D[i2(S, ii, jj)]; };
-  auto Ph = [&](int ii, int jj) { return (double)Phi[i3(S, ii, jj, k)]; };
+  auto Ph = [&](int ii, int jj) { return widen(Phi[i3(S, ii, jj, k)]); };
   const double Sdx = 0.5 *
                      (nu(H(i + 1, j), H(i, j)) * (Dq(i + 1, j) + Dq(i, j)) * (Ph(i + 1, j) - Ph(i, j)) -
                       nu(H(i, j), H(i - 1, j)) * (Dq(i, j) + Dq(i - 1, j)) * (Ph(i, j) - Ph(i - 1, j))) /
@@ -1893,16 +1905,18 @@ __device__ double ke_r5(const Dev<T>& S, int i, int j, int k, const T* Phi, doub
                       nu(H(i, j), H(i, j - 1)) * (Dq(i, j) + Dq(i, j - 1)) * (Ph(i, j) - Ph(i, j - 1))) /
                      dy2;
   // 2 i2dx = 1/dx and lv_ds = 1/dsig, rounded alike
-  return -(2.0 * S.i2dx * (scx(i + 1) - scx(i))) - 2.0 * S.i2dy * (scy(j + 1) - scy(j)) -
-         S.lv_ds[k] * (scz(k + 1) - scz(k)) + Sdx + Sdy;
+  return -(2.0 * S.i2dx * (fx1 - fx0)) -
+         2.0 * S.i2dy * (ke_flux_y(S, i, j + 1, k, Phi) - ke_flux_y(S, i, j, k, Phi)) - S.lv_ds[k] * (fz1 - fz0) + Sdx +
+         Sdy;
 }
 
 // shear production of the nonlinear model (ke_model = 2, src/nhwave.F:
 // 10139-10274): Reynolds stresses from the velocity gradient G, contracted
 // with G per PRODTYPE (1 vertical shear of U, V; 2 vertical shear; else 3-D).
 // kOrdered: the reference's order of sums, term by term (FP64 form); else the
-// same sums, in FP64 too, with the traces formed once and the stresses that
-// the contraction does not read left out (a seventh of the operations).
+// same sums, in FP64 too, with the traces formed once, the symmetric stresses
+// once for both gradients and those that the contraction does not read left
+// out (a tenth of the operations).
 template <bool kOrdered>
 __device__ inline double ke_production(const double (&G)[3][3], double tk, double ep, int prod_type) {
   const double c23 = (double)(2.0f / 3.0f), c13 = (double)(1.0f / 3.0f);
@@ -1911,15 +1925,26 @@ __device__ inline double ke_production(const double (&G)[3][3], double tk, doubl
   for (int n = 0; n < 3; ++n)
     if (fabs(G[n][n]) > smax) smax = fabs(G[n][n]);
   smax = kOrdered ? smax * tk / ep : smax * tke;
-  const double c_d = c23 * (1.0 / ((double)7.4f + 2.0 * smax));
+  double c_d = 0.0, c_1 = 0.0, c_2 = 0.0, c_3 = 0.0;
+  if (kOrdered) c_d = c23 * (1.0 / ((double)7.4f + 2.0 * smax));
   double dmx = 0.0;
   for (int n = 0; n < 3; ++n)
     for (int m = 0; m < 3; ++m)
       if (fabs(G[n][m]) > dmx) dmx = fabs(G[n][m]);
   dmx = kOrdered ? dmx * tk / ep : dmx * tke;
-  const double c_1 = 1.0 / ((double)185.2f + 3.0 * (dmx * dmx));
-  const double c_2 = -(1.0 / (58.5 + 2.0 * (dmx * dmx)));
-  const double c_3 = 1.0 / ((double)370.4f + 3.0 * (dmx * dmx));
+  if (kOrdered) {
+    c_1 = 1.0 / ((double)185.2f + 3.0 * (dmx * dmx));
+    c_2 = -(1.0 / (58.5 + 2.0 * (dmx * dmx)));
+    c_3 = 1.0 / ((double)370.4f + 3.0 * (dmx * dmx));
+  } else {   // two denominators a division
+    const double d2 = dmx * dmx, ad = (double)7.4f + 2.0 * smax, a1 = (double)185.2f + 3.0 * d2, a2 = 58.5 + 2.0 * d2,
+                 a3 = (double)370.4f + 3.0 * d2;
+    const double p = 1.0 / (a1 * a3), q = 1.0 / (ad * a2);
+    c_1 = a3 * p;
+    c_3 = a1 * p;
+    c_d = c23 * (a2 * q);
+    c_2 = -(ad * q);
+  }
   const int n1 = prod_type == 1 ? 2 : 3, m0 = (prod_type == 1 || prod_type == 2) ? 2 : 0;
   double P = 0.0;
   if constexpr (!kOrdered) {
@@ -1931,16 +1956,21 @@ __device__ inline double ke_production(const double (&G)[3][3], double tk, doubl
         gt += G[l][g] * G[l][g];
       }
     const double iso = -c23 * tk - c23 * k1 * gg - c13 * (k2 + k3) * gt;
+    // the stresses are symmetric: n <= m, contracted with both gradients
+    const bool all = n1 == 3 && m0 == 0;
+#pragma unroll
     for (int n = 0; n < 3; ++n)
-      for (int m = 0; m < 3; ++m) {
-        if (!(n < n1 && m >= m0)) continue;
+#pragma unroll
+      for (int m = n; m < 3; ++m) {
+        if (!all && !(n < n1 && m >= m0)) continue;
         double s1 = 0.0, s2 = 0.0, s3 = 0.0;
         for (int l = 0; l < 3; ++l) {
           s1 += G[n][l] * G[l][m] + G[m][l] * G[l][n];
           s2 += G[n][l] * G[m][l];
           s3 += G[l][n] * G[l][m];
         }
-        P += (kd * (G[n][m] + G[m][n]) + k1 * s1 + k2 * s2 + k3 * s3 + (n == m ? iso : 0.0)) * G[n][m];
+        const double g = n != m && all ? G[n][m] + G[m][n] : G[n][m];
+        P += (kd * (G[n][m] + G[m][n]) + k1 * s1 + k2 * s2 + k3 * s3 + (n == m ? iso : 0.0)) * g;
       }
     return P;
   }
@@ -1975,26 +2005,30 @@ __device__ inline double ke_production(const double (&G)[3][3], double tk, doubl
 // DelySl; neighbours are read only through Tke, Eps, CmuHt, D, U, V, W, Ex,
 // Ey, Omega, Mask and the surface values, which no thread writes here.
 //
-// A block has 32 columns and up to 16 threads a column: every cell's
-// production and coefficients are formed side by side, and one warp solves the
-// 32 tridiagonal systems in shared memory.  (One thread a column leaves a
-// 515 x 30 grid with 15,450 threads, each with 15 levels of some 2,000 FP64
-// operations in a row: 2967 us a stage in FP32+IR, now 632 us.)  Bound by the
-// FP64 pipe, most of it divisions; the FP32+IR form shares its reciprocals
-// (Quot) and production sums.
-constexpr int kKeThreadsY = 16;
-inline size_t ke_smem(int K) { return sizeof(double) * (size_t)(5 * 32 * K); }
+// A block has 32, 16 or 8 columns and 256 threads: every cell's production and
+// coefficients are formed side by side, and one warp solves the tridiagonal
+// systems in shared memory.  (One thread a column leaves a 515 x 30 grid with
+// 15,450 threads, each with 15 levels of some 2,000 FP64 operations in a row:
+// 2967 us a stage in FP32+IR.)  Bound by the FP64 pipe, most of it divisions;
+// the FP32+IR form shares its reciprocals (Quot; those of the levels come
+// from a table) and production sums, widens on the integer pipes and
+// compares bit patterns; the advective fluxes are formed once a face in x and
+// sigma (32 columns a block: 636 -> 444 us; blocks of 480 threads, one an
+// SM, took four waves for what three blocks an SM do in two).
+constexpr int kKeThreads = 256;
+inline size_t ke_smem(int cb, int K) { return sizeof(double) * ((size_t)7 * cb * K + K); }
 template <class T>
-__global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int istep) {
+__global__ void __launch_bounds__(kKeThreads, 3) k_ke_column(Dev<T> S, int istep) {
   if (gated_off(S)) return;
   extern __shared__ double ke_sh[];
-  const int K = S.K, KB = S.KB, KE = S.KE;
-  double *prod = ke_sh, *A = prod + 32 * K, *B = A + 32 * K, *C = B + 32 * K, *X = C + 32 * K;
+  const int K = S.K, KB = S.KB, KE = S.KE, cb = blockDim.x;
+  double *prod = ke_sh, *A = prod + cb * K, *B = A + cb * K, *C = B + cb * K, *X = C + cb * K;
+  double *FX = X + cb * K, *FZ = FX + cb * K, *FE = FZ + cb * K;   // fluxes of the lower faces; of the last column's east face
   const double* sigc = S.sigc;
   const double* sig = S.sig;
   const double* dsig = S.dsig;
   const int tx = threadIdx.x, ty = threadIdx.y, by = blockDim.y;
-  const int t = blockIdx.x * 32 + tx;
+  const int t = blockIdx.x * cb + tx;
   const bool valid = t < S.M * S.N;
   const int i = S.IB + (valid ? t % S.M : 0), j = S.JB + (valid ? t / S.M : 0);
   const long long q = i2(S, i, j);
@@ -2005,16 +2039,34 @@ __global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int is
   const double c1e = rng ? (double)1.42f : (double)1.44f;
   const double c3e = 0.0, Prod_b = 0.0;
   const double cmiu = rng ? (double)0.085f : (double)0.09f;
-  const double Sche = rng ? (double)0.72f : (double)1.3f, Schk = rng ? (double)0.72f : 1.0;
   const bool set = S.sc->sig_set != 0;
-  const Quot<T> scD = over<T>(S.scD[q]), Dq = over<T>(Dc), D2 = over<T>(Dc * Dc);
-  const double shx = S.scHx[q], sex = S.scEx[q], shy = S.scHy[q], sey = S.scEy[q];
-  auto Scx = [&](int kk) { return set ? (1.0 - sigc[kk]) / scD * shx - sigc[kk] / scD * sex : 0.0; };
-  auto Scy = [&](int kk) { return set ? (1.0 - sigc[kk]) / scD * shy - sigc[kk] / scD * sey : 0.0; };
-  auto Slx = [&](int kk) { return set ? (1.0 - sig[kk]) / scD * shx - sig[kk] / scD * sex : 0.0; };
-  auto Sly = [&](int kk) { return set ? (1.0 - sig[kk]) / scD * shy - sig[kk] / scD * sey : 0.0; };
-  auto at = [&](const T* a, int kk) -> double { return (double)a[i3(S, i, j, kk)]; };
-  auto dsq = [&](int kk) { return over<T>(sigc[kk + 1] - sigc[kk - 1]); };
+  // FP32+IR: the column's reciprocals formed by one thread each
+  Quot<T> scD{S.scD[q], 0.0}, Dq{Dc, 0.0}, D2{Dc * Dc, 0.0};
+  double shx = S.scHx[q], sex = S.scEx[q], shy = S.scHy[q], sey = S.scEy[q];
+  if constexpr (sizeof(T) == 4) {
+    for (int m = ty; m < 3; m += by) prod[m * cb + tx] = 1.0 / (m == 0 ? scD.b : m == 1 ? Dq.b : D2.b);
+    __syncthreads();
+    scD.r = prod[tx]; Dq.r = prod[cb + tx]; D2.r = prod[2 * cb + tx];
+    shx *= scD.r; sex *= scD.r; shy *= scD.r; sey *= scD.r;
+    __syncthreads();
+  }
+  // slopes of sigma at a level of sig or sigc (src/nhwave.F:6505-6541)
+  auto slope = [&](double sg, double h, double e) {
+    if (!set) return 0.0;
+    if constexpr (sizeof(T) == 4) return (1.0 - sg) * h - sg * e;   // h and e over D already
+    else return (1.0 - sg) / scD * h - sg / scD * e;
+  };
+  auto Scx = [&](int kk) { return slope(sigc[kk], shx, sex); };
+  auto Scy = [&](int kk) { return slope(sigc[kk], shy, sey); };
+  auto Slx = [&](int kk) { return slope(sig[kk], shx, sex); };
+  auto Sly = [&](int kk) { return slope(sig[kk], shy, sey); };
+  auto at = [&](const T* a, int kk) -> double { return widen(a[i3(S, i, j, kk)]); };
+  auto dsq = [&](int kk) { return Quot<T>{sigc[kk + 1] - sigc[kk - 1], S.lvv[kLvR2 * S.Kloc + kk]}; };
+  // the viscosity Cmu + CmuR at a face, from both sides' weights
+  auto face = [&](double l1, double l2, double a, double b, Quot<T> Sc) {
+    if constexpr (sizeof(T) == 4) return (l1 * cmu + l2 * cmu) + (l1 * a + l2 * b) / Sc;   // CmuR = 0
+    else return (l1 * cmu + l2 * cmu) + (l1 * cmuR + l2 * cmuR) + (l1 * a + l2 * b) / Sc;
+  };
   auto lv = [&](int n, int kk) { return S.lvv[n * S.Kloc + kk]; };
   const double dxh = S.DelxH[q], dyh = S.DelyH[q], dxe = S.DelxEta[q], dye = S.DelyEta[q];
   const bool wet = Dc >= Dmin && mk == 1;
@@ -2042,16 +2094,30 @@ __global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int is
         P = ke_production<sizeof(T) == 8>(G, at(S.Tke, k), at(S.Eps, k), S.ke_prod);
         if (k == KE && P < 0.0) P = 0.0;
       }
-      prod[m * 32 + tx] = P;
+      prod[m * cb + tx] = P;
     }
   // one equation: eq = 2 epsilon, 1 tke
   for (int eq = 2; eq >= 1; --eq) {
     const T* Old = eq == 2 ? S.Eps : S.Tke;
     T* Dv = eq == 2 ? S.DEps : S.DTke;
     const double zL = eq == 2 ? S.keTopE[q] : S.keTopK[q];
-    const double SchV = eq == 2 ? Sche : Schk;
-    const Quot<T> Sch = over<T>(SchV);
+    const Quot<T> Sch = eq == 2 ? (rng ? Quot<T>{(double)0.72f, 1.0 / (double)0.72f} : Quot<T>{(double)1.3f, 1.0 / (double)1.3f})
+                                : (rng ? Quot<T>{(double)0.72f, 1.0 / (double)0.72f} : Quot<T>{1.0, 1.0});
     const double DxD = (dxh + dxe) / Dq, DyD = (dyh + dye) / Dq;
+    // the fluxes through the cells' lower faces, once a face: a column's east
+    // face is the next column's west face, the last one's are one more warp's
+    if (valid)
+      for (int m = ty; m < K; m += by) {
+        FX[m * cb + tx] = ke_flux_x(S, i, j, KB + m, Old);
+        FZ[m * cb + tx] = ke_flux_z(S, i, j, KB + m, Old);
+      }
+    {
+      const int tl = min((int)blockIdx.x * cb + cb, S.M * S.N) - 1;
+      for (int m = by * cb - 1 - (tx + cb * ty); m < K; m += by * cb)   // from the last warp on
+        FE[m] = ke_flux_x(S, S.IB + tl % S.M + 1, S.JB + tl / S.M, KB + m, Old);
+    }
+    __syncthreads();
+    const bool last = tx == cb - 1 || t == S.M * S.N - 1;
     if (solve)
       for (int m = ty; m < K; m += by) {
         const int k = KB + m;
@@ -2062,19 +2128,14 @@ __global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int is
         const Quot<T> dsk{dsig[k], S.lv_ds[k]};
         const double vt0 = at(S.CmuVt, k), vtu = at(S.CmuVt, k + 1), vtd = at(S.CmuVt, k - 1);
         const double ht0 = at(S.CmuHt, k), htu = at(S.CmuHt, k + 1), htd = at(S.CmuHt, k - 1);
-        const double nuV_top = (L1top * cmu + L2top * cmu) + (L1top * cmuR + L2top * cmuR) +
-                               (L1top * vt0 + L2top * vtu) / Sch;
-        const double nuH_top = (L1top * cmu + L2top * cmu) + (L1top * cmuR + L2top * cmuR) +
-                               (L1top * ht0 + L2top * htu) / Sch;
-        const double nuV_bot = (L1bot * cmu + L2bot * cmu) + (L1bot * cmuR + L2bot * cmuR) +
-                               (L1bot * vtd + L2bot * vt0) / Sch;
-        const double nuH_bot = (L1bot * cmu + L2bot * cmu) + (L1bot * cmuR + L2bot * cmuR) +
-                               (L1bot * htd + L2bot * ht0) / Sch;
+        const double nuV_top = face(L1top, L2top, vt0, vtu, Sch), nuH_top = face(L1top, L2top, ht0, htu, Sch);
+        const double nuV_bot = face(L1bot, L2bot, vtd, vt0, Sch), nuH_bot = face(L1bot, L2bot, htd, ht0, Sch);
         const double tk = at(S.Tke, k), ep = at(S.Eps, k);
         const Quot<T> tkq = over<T>(eq == 2 ? tk : 1.0);
-        double r = ke_r5(S, i, j, k, Old, SchV);
-        if (eq == 2) r = r + c1e * Dc * (prod[m * 32 + tx] + c3e * Prod_b) * ep / tkq;
-        else r = r + Dc * (prod[m * 32 + tx] + Prod_b) - at(S.DEps, k);
+        const double east = i == S.IE ? 0.0 : last ? FE[m] : FX[m * cb + tx + 1];   // none through the east side
+        double r = ke_r5(S, i, j, k, Old, Sch, FX[m * cb + tx], east, FZ[m * cb + tx], m + 1 < K ? FZ[(m + 1) * cb + tx] : 0.0);
+        if (eq == 2) r = r + c1e * Dc * (prod[m * cb + tx] + c3e * Prod_b) * ep / tkq;
+        else r = r + Dc * (prod[m * cb + tx] + Prod_b) - at(S.DEps, k);
         const double slx1 = Slx(k + 1), sly1 = Sly(k + 1), slx0 = Slx(k), sly0 = Sly(k);
         if (k == KB) {
           r = r - (-(nuH_bot * (dxh * DxD + dyh * DyD) * at(Old, k))) / dsk +
@@ -2096,13 +2157,13 @@ __global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int is
         } else if (k == KE) a = -dt * (3.0 / 2.0 * bot(sxd, syd) / (dsigck1 * (dsigck1 + dsig[k] / 2.0)));
         else {
           const double tp = top(sxd, syd), bt = bot(sxd, syd);
-          a = -dt * ((tp - bt) * alpha_c / dsk + (tp + bt) / (dsigck1 * (dsigck1 + dsigck)));
+          a = -dt * ((tp - bt) * alpha_c / dsk + (tp + bt) / Quot<T>{dsigck1 * (dsigck1 + dsigck), lv(kLvRa, k)});
         }
         if (k == KB) c = -dt * (3.0 / 2.0 * top(sxu, syu) / (dsigck * (dsigck + dsig[k] / 2.0)));
         else if (k == KE) {
         } else {
           const double tp = top(sxu, syu), bt = bot(sxu, syu);
-          c = -dt * ((tp - bt) * gamma_c / dsk + (tp + bt) / (dsigck * (dsigck1 + dsigck)));
+          c = -dt * ((tp - bt) * gamma_c / dsk + (tp + bt) / Quot<T>{dsigck * (dsigck1 + dsigck), lv(kLvRc, k)});
         }
         double b0 = 1.0;
         if (eq == 2) {
@@ -2132,10 +2193,10 @@ __global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int is
         else if (k == KE) b = b0 - dt * (-(3.0 / 2.0 - dsigck1 / dsk) * bot(sx0, sy0) / (dsig[k] / 2.0 * dsigck1));
         else {
           const double tp = top(sx0, sy0), bt = bot(sx0, sy0);
-          b = b0 - dt * ((tp - bt) * beta_c / dsk - (tp + bt) / (dsigck * dsigck1));
+          b = b0 - dt * ((tp - bt) * beta_c / dsk - (tp + bt) / Quot<T>{dsigck * dsigck1, lv(kLvRb, k)});
         }
-        A[m * 32 + tx] = a; B[m * 32 + tx] = b; C[m * 32 + tx] = c;
-        X[m * 32 + tx] = at(Dv, k) + dt * r;
+        A[m * cb + tx] = a; B[m * cb + tx] = b; C[m * cb + tx] = c;
+        X[m * cb + tx] = at(Dv, k) + dt * r;
       }
     __syncthreads();
     // trig (src/nhwave.F:13182-13224): elimination in place, then back
@@ -2144,16 +2205,16 @@ __global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int is
       Quot<T> pb = over<T>(B[tx]);
       if constexpr (sizeof(T) == 4) B[tx] = pb.r;
       for (int m = 1; m < K; ++m) {
-        const int w = m * 32 + tx;
+        const int w = m * cb + tx;
         const double coeff = A[w] / pb;
-        pb = over<T>(B[w] - coeff * C[w - 32]);
+        pb = over<T>(B[w] - coeff * C[w - cb]);
         B[w] = sizeof(T) == 4 ? pb.r : pb.b;
-        X[w] = X[w] - coeff * X[w - 32];
+        X[w] = X[w] - coeff * X[w - cb];
       }
-      double x = X[(K - 1) * 32 + tx] / pb;
-      X[(K - 1) * 32 + tx] = x;
+      double x = X[(K - 1) * cb + tx] / pb;
+      X[(K - 1) * cb + tx] = x;
       for (int m = K - 2; m >= 0; --m) {
-        const int w = m * 32 + tx;
+        const int w = m * cb + tx;
         const double e = X[w] - C[w] * x;
         x = sizeof(T) == 4 ? e * B[w] : e / B[w];
         X[w] = x;
@@ -2168,7 +2229,7 @@ __global__ void __launch_bounds__(32 * kKeThreadsY) k_ke_column(Dev<T> S, int is
       for (int m = ty; m < K; m += by) {
         const long long o = i3(S, i, j, KB + m);
         T x = Dv[o];
-        if (solve) x = (T)X[m * 32 + tx];
+        if (solve) x = (T)X[m * cb + tx];
         if (wet) {
           const double v = al * (double)Dv0[o] + be * (double)x;
           x = (T)dmax_(v, Dc * vmin);
@@ -2479,7 +2540,8 @@ struct OpKe2Column {
       const double SchtH = rng ? (double)0.72f : (eq == 2 ? (double)1.3f : 1.0);
       for (int k = KB; k <= KE; ++k) {
         const int m = k - KB;
-        double r = ke_r5(S, i, j, k, Old, SchtH);
+        double r = ke_r5(S, i, j, k, Old, over<T>(SchtH), ke_flux_x(S, i, j, k, Old), ke_flux_x(S, i + 1, j, k, Old),
+                         ke_flux_z(S, i, j, k, Old), ke_flux_z(S, i, j, k + 1, Old));
         if (eq == 2) r = r + c1e * Dc * (prod[m] + c3e * Prod_b) * at(S.Eps, k) / at(S.Tke, k);
         else r = r + Dc * (prod[m] + Prod_b) - at(S.DEps, k);
         A[m] = k == KB ? 0.0
@@ -2809,7 +2871,7 @@ struct OpLdVisc {
 // A block has 32 columns: all its threads form the coefficients, which DU, DV
 // and DW share, in shared memory, and one warp each then solves DU, DV and DW.
 // Bound by the chain of FP64 divisions of the elimination (515 x 30 x 15
-// FP32+IR, against one thread a column for all three: 415 -> 68 us).
+// FP32+IR, against one thread a column for all three: 415 -> 55 us).
 constexpr int kVvThreadsY = 8;
 inline size_t vv_smem(int K) { return sizeof(double) * (size_t)(8 * 32 * K); }
 template <class T>
@@ -2826,7 +2888,7 @@ __global__ void __launch_bounds__(32 * kVvThreadsY) k_vert_visc(Dev<T> S) {
   const bool wet = in && S.Mask[c] != 0;
   const double dt = S.sc->dt, Dc = S.D[c];
   // CmuVt of level k and the face viscosity between levels k1 and k2
-  auto vt = [&](int k) { return (double)S.CmuVt[i3(S, i, j, k)]; };
+  auto vt = [&](int k) { return widen(S.CmuVt[i3(S, i, j, k)]); };
   const Quot<T> sch = over<T>(S.v_schmidt);
   auto nuz = [&](int k1, int k2) { return 0.5 * (S.v_cmu + S.v_cmu) + 0.5 * (vt(k1) + vt(k2)) / sch; };
   const double* dsg = S.dsig;
@@ -2834,8 +2896,10 @@ __global__ void __launch_bounds__(32 * kVvThreadsY) k_vert_visc(Dev<T> S) {
   if (wet)
     for (int m = ty; m < K; m += by) {
       const int k = KB + m;
-      As[m * 32 + tx] = k == KB ? 0.0 : dtD2 * nuz(k - 1, k) / (0.5 * dsg[k] * (dsg[k] + dsg[k - 1]));
-      Cs[m * 32 + tx] = k == KE ? 0.0 : dtD2 * nuz(k, k + 1) / (0.5 * dsg[k] * (dsg[k] + dsg[k + 1]));
+      const Quot<T> qa{0.5 * dsg[k] * (dsg[k] + dsg[k - 1]), S.lvv[kLvRd * S.Kloc + k]},
+          qc{0.5 * dsg[k] * (dsg[k] + dsg[k + 1]), S.lvv[kLvRu * S.Kloc + k]};
+      As[m * 32 + tx] = k == KB ? 0.0 : dtD2 * nuz(k - 1, k) / qa;
+      Cs[m * 32 + tx] = k == KE ? 0.0 : dtD2 * nuz(k, k + 1) / qc;
       const long long e = o + S.sz * m;
       rs[m * 32 + tx] = (double)S.DU[e];
       rs[nk + m * 32 + tx] = (double)S.DV[e];

@@ -527,7 +527,7 @@ class Solver final : public SolverBase {
       NHW_CU(cudaFuncSetAttribute(k_mg_cycle<T, 1>, at, (int)cycle_smem<T>(KMAX)));
       NHW_CU(cudaFuncSetAttribute(k_mg_cycle<T, 2>, at, (int)cycle_smem<T>(KMAX)));
     }
-    NHW_CU(cudaFuncSetAttribute(k_ke_column<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ke_smem(KMAX)));
+    NHW_CU(cudaFuncSetAttribute(k_ke_column<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ke_smem(32, KMAX)));
     NHW_CU(cudaFuncSetAttribute(k_vert_visc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vv_smem(KMAX)));
     NHW_CU(cudaFuncSetAttribute(k_mg_cta_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(sizeof(T) * 4 * 32 * 64)));
@@ -873,7 +873,10 @@ class Solver final : public SolverBase {
         const double d0 = h.dsig[k], du = h.dsig[k + 1], dd = h.dsig[k - 1];
         const double ck = (d0 + du) / 2.0, ck1 = (dd + d0) / 2.0;
         const double v[kLvN] = {du / (d0 + du), d0 / (d0 + du), d0 / (d0 + dd), dd / (d0 + dd), ck, ck1,
-                                -ck / (ck + ck1) / ck1, (ck - ck1) / (ck * ck1), ck1 / (ck + ck1) / ck};
+                                -ck / (ck + ck1) / ck1, (ck - ck1) / (ck * ck1), ck1 / (ck + ck1) / ck,
+                                1.0 / (ck1 * (ck1 + ck)), 1.0 / (ck * (ck1 + ck)), 1.0 / (ck * ck1),
+                                1.0 / (h.sigc[k + 1] - h.sigc[k - 1]), 1.0 / (0.5 * d0 * (d0 + dd)),
+                                1.0 / (0.5 * d0 * (d0 + du))};
         for (int n = 0; n < kLvN; ++n) lv[n * (size_t)S.Kloc + k] = v[n];
       }
       if (S.lvv)
@@ -1543,7 +1546,14 @@ class Solver final : public SolverBase {
     if (S.ivturb == 10) {
       allcols(OpKeTop{});
       L("kepsilon_column", [&] {
-        k_ke_column<T><<<cdiv((long long)S.M * S.N, 32), dim3(32, std::min(S.K, kKeThreadsY)), ke_smem(S.K), st>>>(S, s);
+        // blocks of 32 columns, of 16 or 8 while those are fewer than two an
+        // SM (FP32+IR, 32 / 16 / 8 columns: 96 x 6 x 20 210 / 151 / 99 us,
+        // 200 x 12 x 10 140 / 91 / 90, 515 x 30 x 15 480 / 493 / 518)
+        const long long cols = (long long)S.M * S.N;
+        int cb = 32;
+        while (cb > 8 && cols < 152LL * 2 * cb) cb /= 2;
+        const int by = std::min(S.K, kKeThreads / cb);
+        k_ke_column<T><<<cdiv((long long)S.M * S.N, cb), dim3(cb, by), ke_smem(cb, S.K), st>>>(S, s);
       });
       box(OpKeSidesX{}, S.N * S.Kloc, 1, 1, 0, 0, 0);
       box(OpKeSidesY{}, S.Mloc * S.Kloc, 1, 1, 0, 0, 0);

@@ -160,7 +160,9 @@ struct Dev {
   // viscous flow only: constants of a sigma level k in the vertical operators,
   // [kLvN][Kloc]: dsig_k+1 / (dsig_k + dsig_k+1), dsig_k / (..), dsig_k /
   // (dsig_k + dsig_k-1), dsig_k-1 / (..), the cell spacings above and below,
-  // and the three-point weights at k-1, k, k+1
+  // and the three-point weights at k-1, k, k+1; then the reciprocals of those
+  // weights' divisors, ck1 (ck + ck1), ck (ck + ck1), ck ck1, of the two cells'
+  // distance sigc_k+1 - sigc_k-1, and of dsig_k (dsig_k + dsig_k-+1) / 2
   const double* lvv;
   double *Hfx, *Hfy, *Hfx0, *Hfy0, *DelxH, *DelyH, *DeltH, *DeltHo, *Delt2H;
   double *DelxEta, *DelyEta, *SourceX, *SourceY, *SourceC, *Sponge, *R1, *Wsx, *Wsy;
@@ -224,7 +226,7 @@ struct Dev {
   DevScal* sc;
 };
 
-enum { kLvL1t, kLvL2t, kLvL1b, kLvL2b, kLvCk, kLvCk1, kLvAc, kLvBc, kLvGc, kLvN };
+enum { kLvL1t, kLvL2t, kLvL1b, kLvL2b, kLvCk, kLvCk1, kLvAc, kLvBc, kLvGc, kLvRa, kLvRc, kLvRb, kLvR2, kLvRd, kLvRu, kLvN };
 
 // -------------------------------------------------------------- indexing
 template <class T>

@@ -65,3 +65,10 @@ def test_viscous_columns(grid, closure, oracle_mod, gpu_lib):
         assert rel_l2(f.get(fid), a) < 2e-5, f"FP32+IR {n} rel {rel_l2(f.get(fid), a):.3e}"
     for h in (g, f):
         h.close()
+
+
+# enough columns for blocks of 16 and of 32, the last of them partly filled, rows ending inside blocks
+@pytest.mark.parametrize("closure", [KE, RNG], ids=["ke", "ke_rng"])
+@pytest.mark.parametrize("grid", [(162, 31, 3), (331, 30, 9)], ids=lambda g: "x".join(map(str, g)))
+def test_viscous_columns_wider_blocks(grid, closure, oracle_mod, gpu_lib):
+    test_viscous_columns(grid, closure, oracle_mod, gpu_lib)
