@@ -766,6 +766,134 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_xr
   }, fin);
 }
 
+// ----------------------------------------------- and on grids of a few waves
+// A few blocks an SM leave some SMs a block more than others: 640 blocks
+// (1024 x 64 x 20) are five on a third of the SMs and four on the rest, and
+// the FP64 pipes of the latter wait.  Here a pair of blocks does one block's
+// work, half of every thread's cells each; the first hands its running sums
+// to the second, so vectors and sums are the same bit for bit.  Taken between
+// kSlicedBlocks and kPairedBlocks blocks; from there on the difference is
+// small (GB300, 1024 x 64 x 20 FP64: res64 120 -> 105 us, bicg_v 49.3 -> 45.6,
+// bicg_t 53.1 -> 49.5; 263 x 187 x 9 56 -> 43.5, 25.1 -> 21.7, 26.8 -> 23.0;
+// FP32+IR res64 70.7 -> 66.2; 512 x 512 x 10, 1280 blocks: none).  bicg_xr,
+// bound by memory, gains up to 2 kSlicedBlocks blocks (515 x 50 x 15 FP32+IR
+// 13.6 -> 12.1 us, 1024 x 64 x 20 16.7 -> 17.5).
+constexpr int kPairedBlocks = 152 * 7;
+template <int NV, class A, class V, class T, class Cell, class Sum, class Fin>
+__device__ __forceinline__ void paired_cells(const Dev<T>& S, Cell cell, Sum sum, Fin fin) {
+  constexpr int Q = kCPT / 2;
+  __shared__ A sv[NV][256];
+  auto cl = cooperative_groups::this_cluster();
+  const int tid = threadIdx.x, rank = (int)cl.block_rank(), blk = blockIdx.x / 2;
+  const int base = (blk * kCPT + rank * Q) * 256 + tid;
+  V val[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (base + q * 256 < S.neq) val[q] = cell(base + q * 256);
+  A v[NV];
+  for (int n = 0; n < NV; ++n) v[n] = (A)0;
+  if (rank == 0) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (base + q * 256 < S.neq) sum(val[q], v);
+    for (int n = 0; n < NV; ++n) sv[n][tid] = v[n];
+  }
+  cl.sync();
+  if (rank == 1)
+    for (int n = 0; n < NV; ++n) v[n] = cl.map_shared_rank(&sv[n][0], 0)[tid];
+  cl.sync();   // the first block stays until its sums have been read
+  if (rank == 0) return;
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (base + q * 256 < S.neq) sum(val[q], v);
+  double out[NV];
+  block_sum_t<NV, A>(v, out);
+  finish_reduce_of<NV>(S, S.partials, 8, blk, gridDim.x / 2, out, fin);
+}
+template <class A>
+struct Two {
+  A a, b;
+};
+
+template <class T, bool kFirst>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) k_res64_pr(Dev<T> S) {
+  if (gated_off(S)) return;
+  constexpr int NV = kFirst ? 2 : 1;   // later sweeps know ||b||
+  paired_cells<NV, double, Two<double>>(S, [&](int ic) {
+    int ii, jj, kk;
+    decode(ic, S.M, S.N, ii, jj, kk);
+    const double b = S.rhs64[ic];
+    const double r = b - spmv_c<double, double>(S.coef64, S.xsol64, (size_t)S.neq, ic, ii, jj, kk, S.M, S.N, S.K,
+                                                S.cxx, S.cyy);
+    S.res64[ic] = r;
+    S.kr0[ic] = narrow<T>(r);
+    return Two<double>{r, b};
+  }, [&](const Two<double>& q, double (&v)[NV]) {
+    v[0] += q.a * q.a;
+    if (kFirst) v[NV - 1] += q.b * q.b;
+  }, FinRes<T, kFirst>{});
+}
+// FP64 form (the FP32+IR form's matvecs walk columns)
+template <class T>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) k_bicg_v_pr(Dev<T> S) {
+  if (S.sc->conv) return;
+  const FinV<T> fin(S.sc);
+  using A = typename Acc<T>::type;
+  const T* __restrict__ ph = S.kph;
+  const T* __restrict__ r0 = S.kr0;
+  paired_cells<1, A, Two<A>>(S, [&](int ic) {
+    int ii, jj, kk;
+    decode(ic, S.M, S.N, ii, jj, kk);
+    const T y = spmv_c<T, T>(S.coefT, ph, (size_t)S.neq, ic, ii, jj, kk, S.M, S.N, S.K, (T)S.cxx, (T)S.cyy);
+    S.kv[ic] = y;
+    return Two<A>{(A)r0[ic], (A)y};
+  }, [&](const Two<A>& q, A (&v)[1]) { v[0] += q.a * q.b; }, fin);
+}
+template <class T>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) k_bicg_t_pr(Dev<T> S) {
+  if (S.sc->conv) return;
+  using A = typename Acc<T>::type;
+  const T* __restrict__ sh = S.ksh;
+  const T* __restrict__ ss = S.ks;
+  paired_cells<2, A, Two<A>>(S, [&](int ic) {
+    int ii, jj, kk;
+    decode(ic, S.M, S.N, ii, jj, kk);
+    const T y = spmv_c<T, T>(S.coefT, sh, (size_t)S.neq, ic, ii, jj, kk, S.M, S.N, S.K, (T)S.cxx, (T)S.cyy);
+    S.kt[ic] = y;
+    return Two<A>{(A)ss[ic], (A)y};
+  }, [&](const Two<A>& q, A (&v)[2]) {
+    v[0] += q.b * q.a;
+    v[1] += q.b * q.b;
+  }, FinT<T>{});
+}
+template <class T>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) k_bicg_xr_pr(Dev<T> S) {
+  if (S.sc->conv) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) set_cond(S, S.h_inner, false);
+    return;
+  }
+  const FinXr<T> fin(S.sc);
+  const T alpha = (T)fin.alpha, omega = (T)fin.omega;
+  using A = typename Acc<T>::type;
+  T* __restrict__ x = S.kx;
+  T* __restrict__ rr = S.kr;
+  const T* __restrict__ ph = S.kph;
+  const T* __restrict__ sh = S.ksh;
+  const T* __restrict__ ss = S.ks;
+  const T* __restrict__ tt = S.kt;
+  const T* __restrict__ r0 = S.kr0;
+  paired_cells<2, A, Two<A>>(S, [&](int t) {
+    x[t] = x[t] + alpha * ph[t] + omega * sh[t];
+    const T r = ss[t] - omega * tt[t];
+    rr[t] = r;
+    if (S.kq) S.kq[t] = S.kp[t] - omega * S.kv[t];
+    return Two<A>{(A)r0[t], (A)r};
+  }, [&](const Two<A>& q, A (&v)[2]) {
+    v[0] += q.a * q.b;
+    v[1] += q.b * q.b;
+  }, fin);
+}
+
 // ------------------------------------------------------------------ GMRES
 // Right-preconditioned GMRES: one cycle of at most kGmMax iterations per
 // refinement sweep, so the sweeps of k_res64 are its restarts.  It is the

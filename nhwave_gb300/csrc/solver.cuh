@@ -1223,10 +1223,12 @@ class Solver final : public SolverBase {
   // the reducing Krylov kernels in slices (krylov.cuh) while their blocks are
   // fewer than the SMs
   bool sliced() const { return red_blocks() <= (unsigned)kSlicedBlocks; }
+  bool paired() const { return red_blocks() <= (unsigned)kPairedBlocks; }
   template <bool kFirst>
   void residual() {
     L("res64", [&] {
       if (sliced()) k_res64_sl<T, kFirst><<<red_blocks() * kSlices, 256, 0, st>>>(S);
+      else if (paired()) k_res64_pr<T, kFirst><<<red_blocks() * 2, 256, 0, st>>>(S);
       else k_res64<T, kFirst><<<red_blocks(), 256, 0, st>>>(S);
     });
   }
@@ -1286,8 +1288,16 @@ class Solver final : public SolverBase {
       L("bicg_p", [&] { k_bicg_p<T><<<cb, 128, 0, st>>>(S); });
     }
     L("bicg_v", [&] {
-      if (sliced()) k_bicg_v_sl<T><<<matvec_blocks() * kSlices, 256, 0, st>>>(S);
-      else k_bicg_v<T><<<matvec_blocks(), 256, 0, st>>>(S);
+      if (sliced()) {
+        k_bicg_v_sl<T><<<matvec_blocks() * kSlices, 256, 0, st>>>(S);
+        return;
+      }
+      if constexpr (!kColumnWalk<T>)
+        if (paired()) {
+          k_bicg_v_pr<T><<<red_blocks() * 2, 256, 0, st>>>(S);
+          return;
+        }
+      k_bicg_v<T><<<matvec_blocks(), 256, 0, st>>>(S);
     });
     if (use_mg) {
       vcycle(S.ks, S.ksh, 2);   // s likewise
@@ -1295,11 +1305,20 @@ class Solver final : public SolverBase {
       L("bicg_s", [&] { k_bicg_s<T><<<cb, 128, 0, st>>>(S); });
     }
     L("bicg_t", [&] {
-      if (sliced()) k_bicg_t_sl<T><<<matvec_blocks() * kSlices, 256, 0, st>>>(S);
-      else k_bicg_t<T><<<matvec_blocks(), 256, 0, st>>>(S);
+      if (sliced()) {
+        k_bicg_t_sl<T><<<matvec_blocks() * kSlices, 256, 0, st>>>(S);
+        return;
+      }
+      if constexpr (!kColumnWalk<T>)
+        if (paired()) {
+          k_bicg_t_pr<T><<<red_blocks() * 2, 256, 0, st>>>(S);
+          return;
+        }
+      k_bicg_t<T><<<matvec_blocks(), 256, 0, st>>>(S);
     });
     L("bicg_xr", [&] {
       if (sliced()) k_bicg_xr_sl<T><<<red_blocks() * kSlices, 256, 0, st>>>(S);
+      else if (red_blocks() <= 2u * kSlicedBlocks) k_bicg_xr_pr<T><<<red_blocks() * 2, 256, 0, st>>>(S);
       else k_bicg_xr<T><<<red_blocks(), 256, 0, st>>>(S);
     });
   }
