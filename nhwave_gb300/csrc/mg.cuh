@@ -282,6 +282,90 @@ struct MgInV {
   }
 };
 
+// Line solve of one column whose right-hand sides and factors are in shared
+// memory, NS elements from level to level, by a warp on its own: the forward
+// sweep y_k = (rhs_k - a_k y_{k-1}) / den_k, then the back substitution, whose
+// values go to put(k, x_k).  Up to KM levels, written out, the loads of CH
+// levels issued ahead of the chain; the forward values stay in registers
+// (FP32) or go through rhs (FP64, whose registers are short and whose
+// operations take some 80 cycles each in a chain).  As loops over shared
+// memory the same solve waits for its loads level by level (GB300, one warp:
+// FP32 10 levels 1580 -> 440 cycles, 20 levels 1690 -> 800; FP64 10 levels
+// 5050 -> 4290).
+template <int NS, int KM, int CH, class T, class Put>
+__device__ __forceinline__ void line_solve_regs(T* __restrict__ rhs, const T* __restrict__ a,
+                                                const T* __restrict__ inv, const T* __restrict__ c, int K, Put put) {
+  constexpr int NC = KM / CH;
+  constexpr bool kKeep = sizeof(T) == 4;
+  static_assert(KM % CH == 0, "whole chunks");
+  T y[kKeep ? KM : 1], r[2][CH], f[2][CH], d[2][CH];
+  auto fetch = [&](int ch) {
+#pragma unroll
+    for (int t = 0; t < CH; ++t) {
+      const int k = ch * CH + t;
+      if (k < K) { r[ch & 1][t] = rhs[k * NS]; f[ch & 1][t] = a[k * NS]; d[ch & 1][t] = inv[k * NS]; }
+    }
+  };
+  fetch(0);
+  T z = (T)0;
+#pragma unroll
+  for (int ch = 0; ch < NC; ++ch) {
+    if (ch + 1 < NC) fetch(ch + 1);
+#pragma unroll
+    for (int t = 0; t < CH; ++t) {
+      const int k = ch * CH + t;
+      if (k < K) {
+        z = (r[ch & 1][t] - f[ch & 1][t] * z) * d[ch & 1][t];
+        if (!kKeep) rhs[k * NS] = z;
+      }
+      if (kKeep) y[kKeep ? k : 0] = z;
+    }
+  }
+  auto fetch_back = [&](int ch) {
+#pragma unroll
+    for (int t = 0; t < CH; ++t) {
+      const int k = ch * CH + t;
+      if (k < K - 1) {
+        f[ch & 1][t] = c[k * NS];
+        r[ch & 1][t] = kKeep ? y[kKeep ? k : 0] : rhs[k * NS];
+      }
+    }
+  };
+  fetch_back(NC - 1);
+#pragma unroll
+  for (int ch = NC - 1; ch >= 0; --ch) {
+    if (ch > 0) fetch_back(ch - 1);
+#pragma unroll
+    for (int t = CH - 1; t >= 0; --t) {
+      const int k = ch * CH + t;
+      if (k < K - 1) z = r[ch & 1][t] - f[ch & 1][t] * z;
+      if (k < K) put(k, z);
+    }
+  }
+}
+// The same by the number of levels, and in loops through rhs beyond 20 levels
+// and in the FP64 half-sweeps, whose 32 registers hold no more.
+template <int NS, class T, class Put>
+__device__ __forceinline__ void line_solve(T* __restrict__ rhs, const T* __restrict__ a, const T* __restrict__ inv,
+                                           const T* __restrict__ c, int K, Put put) {
+  if constexpr (sizeof(T) == 4) {
+    if (K <= 10) return line_solve_regs<NS, 10, 5>(rhs, a, inv, c, K, put);
+    if (K <= 20) return line_solve_regs<NS, 20, 5>(rhs, a, inv, c, K, put);
+  }
+  T z = (T)0;
+#pragma unroll 4
+  for (int k = 0; k < K; ++k) {
+    z = (rhs[k * NS] - a[k * NS] * z) * inv[k * NS];
+    rhs[k * NS] = z;
+  }
+  put(K - 1, z);
+#pragma unroll 4
+  for (int k = K - 2; k >= 0; --k) {
+    z = rhs[k * NS] - c[k * NS] * z;
+    put(k, z);
+  }
+}
+
 // Same half-sweep, block-parallel: a block holds 32 columns of the colour and
 // up to 32 levels (blockDim = 32 x min(K,32)); every thread forms the line
 // right-hand sides of its (column, level) cells -- loads coalesced along the
@@ -325,21 +409,7 @@ __global__ void __launch_bounds__(1024) k_mg_smooth_blk(MGL<T> L, const DevScal*
   }
   __syncthreads();
   if (ty != 0 || !valid) return;
-  // the Thomas sweeps, unrolled so that the shared-memory loads of several
-  // levels issue ahead of the dependent chain
-  T prev = (T)0;
-#pragma unroll 4
-  for (int k = 0; k < K; ++k) {
-    prev = (s_rhs[k * 32 + tx] - s_a[k * 32 + tx] * prev) * s_inv[k * 32 + tx];
-    s_rhs[k * 32 + tx] = prev;
-  }
-  T z = prev;
-  L.x[col + MN * (K - 1)] = z;
-#pragma unroll 4
-  for (int k = K - 2; k >= 0; --k) {
-    z = s_rhs[k * 32 + tx] - s_cp[k * 32 + tx] * z;
-    L.x[col + MN * k] = z;
-  }
+  line_solve<32>(s_rhs + tx, s_a + tx, s_inv + tx, s_cp + tx, K, [&](int k, T z) { L.x[col + MN * k] = z; });
 }
 
 // Half-sweep on the colour-split operator (MGL::sp).  A block holds
@@ -459,21 +529,7 @@ k_mg_smooth_split(MGL<T> L, const DevScal* sc, int color, int zero_x, Prolong<T>
   }
   __syncthreads();
   if (ty != 0 || !valid) return;
-  // the Thomas sweeps, unrolled so that the shared-memory loads of several
-  // levels issue ahead of the dependent chain
-  T prev = (T)0;
-#pragma unroll 4
-  for (int k = 0; k < K; ++k) {
-    prev = (s_rhs[k * 32 + tx] - s_a[k * 32 + tx] * prev) * s_inv[k * 32 + tx];
-    s_rhs[k * 32 + tx] = prev;
-  }
-  T z = prev;
-  L.x[col + MN * (K - 1)] = z;
-#pragma unroll 4
-  for (int k = K - 2; k >= 0; --k) {
-    z = s_rhs[k * 32 + tx] - s_cp[k * 32 + tx] * z;
-    L.x[col + MN * k] = z;
-  }
+  line_solve<32>(s_rhs + tx, s_a + tx, s_inv + tx, s_cp + tx, K, [&](int k, T z) { L.x[col + MN * k] = z; });
 }
 
 // The same half-sweep for the FP64 form: each thread of a column forms the
@@ -525,21 +581,7 @@ __global__ void __launch_bounds__(1024, 2) k_mg_smooth_split_strided(MGL<T> L, c
   }
   __syncthreads();
   if (ty != 0 || !valid) return;
-  // the Thomas sweeps, unrolled so that the shared-memory loads of several
-  // levels issue ahead of the dependent chain
-  T prev = (T)0;
-#pragma unroll 4
-  for (int k = 0; k < K; ++k) {
-    prev = (s_rhs[k * 32 + tx] - s_a[k * 32 + tx] * prev) * s_inv[k * 32 + tx];
-    s_rhs[k * 32 + tx] = prev;
-  }
-  T z = prev;
-  L.x[col + MN * (K - 1)] = z;
-#pragma unroll 4
-  for (int k = K - 2; k >= 0; --k) {
-    z = s_rhs[k * 32 + tx] - s_cp[k * 32 + tx] * z;
-    L.x[col + MN * k] = z;
-  }
+  line_solve<32>(s_rhs + tx, s_a + tx, s_inv + tx, s_cp + tx, K, [&](int k, T z) { L.x[col + MN * k] = z; });
 }
 
 // Coarse-grid correction of the colour-0 cells of a level, in place:

@@ -33,11 +33,13 @@ struct TileS {
   static_assert(NS == 32, "a level's slots fill one warp");
 };
 
-// Line solve of one column, in place, as the half-sweeps of mg.cuh do it:
-// y_k = (rhs_k - a_k y_{k-1}) / den_k up the column, then the back substitution.
-// Levels go through registers four at a time, the next four's shared loads
-// issued before the current ones' stores (a store to x holds back every later
-// load of it).  x, a, inv, c point at level 0; NS elements to the next.
+// Line solve of one column, in place, of more than 20 levels and in the block
+// cycle below, where line_solve_regs' code and registers cost more than its
+// loads save (256 x 8 x 10 FP32+IR: 11.6 against 12.4 to 24 us a cycle, as a
+// call, in one loop or written out).  Levels go through registers four at a
+// time, the next four's shared loads issued before the current ones' stores (a
+// store to x holds back every later load of it).  x, a, inv, c point at level
+// 0; NS elements to the next.
 template <int NS, class T>
 __device__ __forceinline__ void line_solve_smem(T* __restrict__ x, const T* __restrict__ a, const T* __restrict__ inv,
                                                 const T* __restrict__ c, int K) {
@@ -93,6 +95,18 @@ __device__ __forceinline__ void line_solve_smem(T* __restrict__ x, const T* __re
     k -= 4;
   }
   for (; k >= 0; --k, x -= NS, c -= NS) { y = *x - *c * y; *x = y; }
+}
+
+// CH: levels fetched ahead (line_solve_regs); as many as the registers hold
+template <class T>
+constexpr int kAhead = sizeof(T) == 4 ? 5 : 2;
+template <int NS, int CH, class T>
+__device__ __forceinline__ void line_solve_tile(T* __restrict__ x, const T* __restrict__ a, const T* __restrict__ inv,
+                                                const T* __restrict__ c, int K) {
+  auto put = [&](int k, T z) { x[k * NS] = z; };
+  if (K <= 10) line_solve_regs<NS, 10, CH>(x, a, inv, c, K, put);
+  else if (K <= 20) line_solve_regs<NS, 20, CH>(x, a, inv, c, K, put);
+  else line_solve_smem<NS>(x, a, inv, c, K);
 }
 
 // The operator of one level at a column of colour c: line factors, cross
@@ -289,7 +303,7 @@ __global__ void __launch_bounds__(1024) k_mg_down(MGL<T> L, MGL<T> C, int ntile_
     x1[q] = (T)0; x1[(K + 1) * NS + q] = (T)0;
   }
   __syncthreads();
-  if (ty == 0 && u0) line_solve_smem<NS>(x0 + NS + q, l0 + q, l0 + K * NS + q, l0 + 2 * K * NS + q, K);
+  if (ty == 0 && u0) line_solve_tile<NS, kAhead<T>>(x0 + NS + q, l0 + q, l0 + K * NS + q, l0 + 2 * K * NS + q, K);
   __syncthreads();
 #pragma unroll
   for (int t = 0; t < LPT; ++t) {
@@ -307,7 +321,7 @@ __global__ void __launch_bounds__(1024) k_mg_down(MGL<T> L, MGL<T> C, int ntile_
     if (own0 && k < K) L.xp[col0 + MN * k] = x0[(k + 1) * NS + q];
   }
   __syncthreads();
-  if (ty == 0 && u1) line_solve_smem<NS>(x1 + NS + q, l1 + q, l1 + K * NS + q, l1 + 2 * K * NS + q, K);
+  if (ty == 0 && u1) line_solve_tile<NS, kAhead<T>>(x1 + NS + q, l1 + q, l1 + K * NS + q, l1 + 2 * K * NS + q, K);
   __syncthreads();
   // the off-column part at the tile's colour-0 cells, in place of x0, then its
   // sums over the aggregates
@@ -410,7 +424,7 @@ __global__ void __launch_bounds__(1024) k_mg_up(MGL<T> L, Prolong<T> P, int ntil
     if (k < K) x1[(k + 1) * NS + q] = b1[t];
   }
   __syncthreads();
-  if (ty == 0 && u1) line_solve_smem<NS>(x1 + NS + q, l1 + q, l1 + K * NS + q, l1 + 2 * K * NS + q, K);
+  if (ty == 0 && u1) line_solve_tile<NS, kAhead<T>>(x1 + NS + q, l1 + q, l1 + K * NS + q, l1 + 2 * K * NS + q, K);
   __syncthreads();
 #pragma unroll
   for (int t = 0; t < LPT; ++t) {
@@ -422,7 +436,7 @@ __global__ void __launch_bounds__(1024) k_mg_up(MGL<T> L, Prolong<T> P, int ntil
     if (own1 && k < K) L.x[col1 + MN * k] = x1[(k + 1) * NS + q];
   }
   __syncthreads();
-  if (ty == 0 && own0) line_solve_smem<NS>(x0 + NS + q, l0 + q, l0 + K * NS + q, l0 + 2 * K * NS + q, K);
+  if (ty == 0 && own0) line_solve_tile<NS, kAhead<T>>(x0 + NS + q, l0 + q, l0 + K * NS + q, l0 + 2 * K * NS + q, K);
   __syncthreads();
 #pragma unroll
   for (int t = 0; t < LPT; ++t) {
