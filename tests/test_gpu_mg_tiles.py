@@ -72,3 +72,17 @@ def test_split_coarse_levels_step_like_the_oracle(shape, precision, oracle_mod, 
     p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
     po, _, _ = _case(*shape, 0, 1e-13)
     _against_oracle(p, po, depth, eta, oracle_mod)
+
+
+# levels at the edges of the written-out line solves (10 and 20, chunks of 5 and 2), on tiles and on half-sweeps
+HEIGHTS = [(24, 12, 5), (24, 12, 6), (24, 12, 10), (24, 12, 11), (24, 12, 19), (70, 61, 10), (70, 61, 11), (70, 61, 21)]
+# 153 blocks of 2048 cells, the last of 977: the sums in pairs of blocks
+PAIRED = [(157, 153, 13)]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", HEIGHTS + PAIRED, ids=lambda s: "x".join(map(str, s)))
+def test_line_solves_and_paired_sums_step_like_the_oracle(shape, precision, oracle_mod, gpu_lib):
+    p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
+    po, _, _ = _case(*shape, 0, 1e-13)
+    _against_oracle(p, po, depth, eta, oracle_mod)
