@@ -344,7 +344,7 @@ __device__ __forceinline__ void line_solve_regs(T* __restrict__ rhs, const T* __
   }
 }
 // The same by the number of levels, and in loops through rhs beyond 20 levels
-// and in the FP64 half-sweeps, whose 32 registers hold no more.
+// and in FP64 (k_mg_smooth_blk's blocks of 1024 threads leave it no registers).
 template <int NS, class T, class Put>
 __device__ __forceinline__ void line_solve(T* __restrict__ rhs, const T* __restrict__ a, const T* __restrict__ inv,
                                            const T* __restrict__ c, int K, Put put) {
@@ -536,10 +536,13 @@ k_mg_smooth_split(MGL<T> L, const DevScal* sc, int color, int zero_x, Prolong<T>
 // right-hand sides of the levels ty, ty + blockDim.y, ... (no register
 // window: its doubles would take twice the registers, and with them fewer
 // blocks fit an SM; C2 level 0, graph of 400 half-sweeps: 25.1 us per launch
-// against 27.7-33.8 us for windows of 2-7 levels).  Otherwise as
-// k_mg_smooth_blk.
+// against 27.7-33.8 us for windows of 2-7 levels).  Blocks are at most 8 rows
+// of threads; five of them an SM, 48 registers, are the fastest with the
+// written-out line solve (1024 x 64 x 20, levels 0 to 2, a launch: 23.6 us with
+// loops at 32 registers, 22.6 / 21.8 / 23.0 us with 64 / 48 / 40).  Otherwise
+// as k_mg_smooth_blk.
 template <class T, bool kProlong, class In>
-__global__ void __launch_bounds__(1024, 2) k_mg_smooth_split_strided(MGL<T> L, const DevScal* sc, int color, int zero_x,
+__global__ void __launch_bounds__(256, 5) k_mg_smooth_split_strided(MGL<T> L, const DevScal* sc, int color, int zero_x,
                                                           Prolong<T> P, In in) {
   if (sc->conv) return;
   const In inb = in.bind(sc);
@@ -581,7 +584,10 @@ __global__ void __launch_bounds__(1024, 2) k_mg_smooth_split_strided(MGL<T> L, c
   }
   __syncthreads();
   if (ty != 0 || !valid) return;
-  line_solve<32>(s_rhs + tx, s_a + tx, s_inv + tx, s_cp + tx, K, [&](int k, T z) { L.x[col + MN * k] = z; });
+  auto put = [&](int k, T z) { L.x[col + MN * k] = z; };
+  if (K <= 10) line_solve_regs<32, 10, 2>(s_rhs + tx, s_a + tx, s_inv + tx, s_cp + tx, K, put);
+  else if (K <= 20) line_solve_regs<32, 20, 2>(s_rhs + tx, s_a + tx, s_inv + tx, s_cp + tx, K, put);
+  else line_solve<32>(s_rhs + tx, s_a + tx, s_inv + tx, s_cp + tx, K, put);
 }
 
 // Coarse-grid correction of the colour-0 cells of a level, in place:
