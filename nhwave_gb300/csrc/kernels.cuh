@@ -1779,7 +1779,9 @@ constexpr double kTkeMin = (double)1.e-9f, kEpsMin = (double)1.e-9f;
 
 // limited horizontal slopes (delxFun_3D / delyFun_3D) of U and V as
 // get_Omega leaves them (uv = 1, before sponge_damping), or of W as fluxes
-// leaves them (uv = 0), at the interior cells the production reads
+// leaves them (uv = 0), at the interior cells the production reads.  In FP64
+// in both forms; FP32+IR multiplies by the spacings' reciprocals and widens on
+// the integer pipes (515 x 30 x 15: 58 -> 43 us).
 struct OpKeSlopes {
   static constexpr const char* kName = "ke_slopes";
   int uv;
@@ -1787,12 +1789,14 @@ struct OpKeSlopes {
   __device__ void operator()(const Dev<T>& S, int i, int j, int k) const {
     const long long q = i2(S, i, j), o = i3(S, i, j, k);
     const bool dry = S.Mask[q] == 0;
-    auto sx = [&](const T* a) -> T {
-      return dry ? (T)0 : (T)lim_slope<double>((double)a[o - 1], (double)a[o], (double)a[o + 1], S.dx, S.dx);
+    auto slope = [&](const T* a, long long st, double h, double i2h) -> T {
+      if (dry) return (T)0;
+      const double am = widen(a[o - st]), a0 = widen(a[o]), ap = widen(a[o + st]);
+      if constexpr (sizeof(T) == 4) return narrow<T>(lim_slope_r<double>(am, a0, ap, 2.0 * i2h, 2.0 * i2h));
+      else return lim_slope<double>(am, a0, ap, h, h);
     };
-    auto sy = [&](const T* a) -> T {
-      return dry ? (T)0 : (T)lim_slope<double>((double)a[o - S.sy], (double)a[o], (double)a[o + S.sy], S.dy, S.dy);
-    };
+    auto sx = [&](const T* a) { return slope(a, 1, S.dx, S.i2dx); };
+    auto sy = [&](const T* a) { return slope(a, S.sy, S.dy, S.i2dy); };
     if (uv) {
       S.keDxU[o] = sx(S.U); S.keDyU[o] = sy(S.U);
       S.keDxV[o] = sx(S.V); S.keDyV[o] = sy(S.V);
