@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(1024) k_mg_smooth_blk(MGL<T> L, const DevScal*
 // The right-hand sides are summed in the order of off_column_c /
 // off_column_pc, so the result is the strided kernel's, bit for bit.
 constexpr int kSplitLevels = 4;      // levels per thread (a chunk)
-constexpr int kSplitRegs = 56;       // no spills; 7 blocks of 32 x 5 threads fit an SM
+constexpr int kSplitRegs = 56;       // 7 blocks of 32 x 5 threads fit an SM
 constexpr int kSplitMaxThreads = 1024;   // 56 registers x 1024 threads fit the 64K register file
 template <class T, bool kProlong, class In>
 __global__ void __maxnreg__(kSplitRegs)
