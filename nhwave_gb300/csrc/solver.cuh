@@ -424,7 +424,7 @@ class Solver final : public SolverBase {
       const size_t nl = (size_t)mg[l].n;
       add((T**)&mg[l].coef, sizeof(T) * NCOMPACT * nl);
       // levels above the tiles' size take the half-sweeps of level 0
-      if (!tiled(mg[l]) && (long long)mg[l].M * mg[l].N > cta_columns)
+      if (!tiled(mg[l]) && (int)l < first_block_level() && (long long)mg[l].M * mg[l].N > cta_columns)
         add((T**)&mg[l].sp, sizeof(T) * 7 * 2 * (size_t)K * mg[l].N * ((mg[l].M + 1) / 2));
       add((T**)&mg[l].lcp, sizeof(T) * nl);
       add((T**)&mg[l].linv, sizeof(T) * nl);
@@ -721,12 +721,8 @@ class Solver final : public SolverBase {
     g.S = S;
     g.S.graph_mode = 0;
     const int nl = (int)mg.size();
-    int lc = 0;
-    while (lc < nl && (long long)mg[lc].M * mg[lc].N > cta_columns) ++lc;
-    if (nl - lc > kCtaLevels) lc = nl - kCtaLevels;
-    if (lc >= nl) lc = nl - 1;   // the first block always solves at least the coarsest level
     for (int l = 0; l < nl; ++l) g.L[l] = mg[l];
-    g.nl = lc;
+    g.nl = first_block_level();   // the first block always solves at least the coarsest level
     g.ntot = nl;
     g.w = mg_w;
     g.coarse_sweeps = coarse_sweeps;
@@ -1324,6 +1320,15 @@ class Solver final : public SolverBase {
   }
   // multigrid V-cycle: x ~= A^-1 b on level 0
   int cta_columns = 64;    // levels up to this many columns run in one block (mg_cta_columns)
+  // the first level of the block cycle: at most its kCtaLevels last levels, and
+  // always the coarsest, which has no level below it to restrict to, even where
+  // it has more than cta_columns columns
+  int first_block_level() const {
+    const int nl = (int)mg.size();
+    int lc = 0;
+    while (lc < nl && (long long)mg[lc].M * mg[lc].N > cta_columns) ++lc;
+    return std::min(std::max(lc, nl - kCtaLevels), nl - 1);
+  }
   template <class In>
   void smooth(const MGL<T>& Lv, int color, int zero_x, int level, const Prolong<T>& P, In in) {
     static const char* names[] = {"mg_smooth_l0", "mg_smooth_l1", "mg_smooth_l2", "mg_smooth_l3",
@@ -1418,11 +1423,7 @@ class Solver final : public SolverBase {
   void vcycle(T* b, T* x, int fine_in) {
     mg[0].b = b;
     mg[0].x = x;
-    const int nl = (int)mg.size();
-    // first level handled by the single-block cycle
-    int lc = 0;
-    while (lc < nl && (long long)mg[lc].M * mg[lc].N > cta_columns) ++lc;
-    if (nl - lc > kCtaLevels) lc = nl - kCtaLevels;
+    const int nl = (int)mg.size(), lc = first_block_level();
     const Prolong<T> none{nullptr, (T)0, 1, 1, 1, 1, 1, 1};
     if (lc == 0 && fine_in != 0) {   // the whole hierarchy in one block: form b first
       if (fine_in == 1) L("bicg_p", [&] { k_bicg_p_cell<T><<<cdiv(S.neq, 256), 256, 0, st>>>(S); });
@@ -1448,7 +1449,7 @@ class Solver final : public SolverBase {
       MGL<T> f = mg[l], c = mg[l + 1];
       L(rnames[l < 7 ? l : 7], [&] { k_mg_restrict_c0<T><<<cdiv(c.n, 256), 256, 0, st>>>(f, c, S.sc); });
     }
-    if (lc < nl) {
+    {
       MGSet<T> set{};
       int slots = 0;
       for (int l = lc; l < nl; ++l) {

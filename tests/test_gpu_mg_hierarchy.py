@@ -1,0 +1,24 @@
+"""GPU: where the multigrid cycle hands over to its single block.
+
+The block takes the last levels, always the coarsest among them, whatever
+mg_cta_columns says: below the coarsest level's 8 to 32 columns every level but
+it must run outside the block, and the pressure must be solved as the oracle
+does (the bounds that every FP64 and FP32+IR grid is held to).
+"""
+import pytest
+
+from test_gpu_mg_tiles import _against_oracle
+from test_gpu_shapes import _case
+
+pytestmark = pytest.mark.gpu
+
+
+# a hierarchy of three levels, of one, and with a level above the tiles' size
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("columns", [1, 8, 31])
+@pytest.mark.parametrize("shape", [(24, 12, 6), (8, 4, 5), (90, 61, 4)], ids=lambda s: "x".join(map(str, s)))
+def test_block_takes_the_coarsest_level(shape, columns, precision, oracle_mod, gpu_lib):
+    p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
+    po, _, _ = _case(*shape, 0, 1e-13)
+    p.mg_cta_columns = columns
+    _against_oracle(p, po, depth, eta, oracle_mod)
