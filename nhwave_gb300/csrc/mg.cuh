@@ -892,5 +892,12 @@ __global__ void __launch_bounds__(256) k_bicg_s_cell(Dev<T> S) {
   if (t >= S.neq) return;
   S.ks[t] = S.kr[t] - (T)S.sc->alpha * S.kv[t];
 }
+// GMRES' basis vector (MgInV)
+template <class T>
+__global__ void __launch_bounds__(256) k_gm_v_cell(Dev<T> S, MgInV<T> in) {
+  if (S.sc->conv) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < S.neq) in(S.sc, t, 0, 0, 0);
+}
 
 }  // namespace nhw

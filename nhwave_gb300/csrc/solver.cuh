@@ -1272,14 +1272,14 @@ class Solver final : public SolverBase {
   }
   void one_iteration() {
     if (use_gmres) {   // z_j = M^-1 v_j (v_j formed by the first sweeps), then Arnoldi
-      vcycle(S.kp, S.kph, 3);
+      vcycle(S.kp, S.kph, kFineV);
       L("gm_arnoldi", [&] { k_gm_arnoldi<T><<<red_blocks(), 256, 0, st>>>(S); });
       L("gm_orth", [&] { k_gm_orth<T><<<red_blocks(), 256, 0, st>>>(S); });
       return;
     }
     const unsigned cb = cdiv((long long)S.M * S.N, 128);
     if (use_mg) {
-      vcycle(S.kp, S.kph, 1);   // p is formed by the fine level's first sweeps
+      vcycle(S.kp, S.kph, kFineP);   // p is formed by the fine level's first sweeps
     } else {
       L("bicg_p", [&] { k_bicg_p<T><<<cb, 128, 0, st>>>(S); });
     }
@@ -1296,7 +1296,7 @@ class Solver final : public SolverBase {
       k_bicg_v<T><<<matvec_blocks(), 256, 0, st>>>(S);
     });
     if (use_mg) {
-      vcycle(S.ks, S.ksh, 2);   // s likewise
+      vcycle(S.ks, S.ksh, kFineS);   // s likewise
     } else {
       L("bicg_s", [&] { k_bicg_s<T><<<cb, 128, 0, st>>>(S); });
     }
@@ -1419,32 +1419,36 @@ class Solver final : public SolverBase {
                                                                                            mg_coarse_sweeps);
     });
   }
-  // fine_in: 0 b as given; 1 b = p formed on the fly; 2 b = s formed on the fly
-  void vcycle(T* b, T* x, int fine_in) {
+  // b is formed on the fly by level 0's first passes: BiCGSTAB's p or s, or
+  // GMRES' basis vector
+  enum FineIn { kFineP, kFineS, kFineV };
+  void vcycle(T* b, T* x, FineIn fine_in) {
     mg[0].b = b;
     mg[0].x = x;
     const int nl = (int)mg.size(), lc = first_block_level();
     const Prolong<T> none{nullptr, (T)0, 1, 1, 1, 1, 1, 1};
-    if (lc == 0 && fine_in != 0) {   // the whole hierarchy in one block: form b first
-      if (fine_in == 1) L("bicg_p", [&] { k_bicg_p_cell<T><<<cdiv(S.neq, 256), 256, 0, st>>>(S); });
-      else L("bicg_s", [&] { k_bicg_s_cell<T><<<cdiv(S.neq, 256), 256, 0, st>>>(S); });
+    auto in_v = [&] { return MgInV<T>{S.kt, S.kp, S.gmV, S.gmT + kGmTInv, (size_t)S.neq}; };
+    if (lc == 0) {   // the whole hierarchy in one block: form b first
+      const unsigned nb = cdiv(S.neq, 256);
+      if (fine_in == kFineP) L("bicg_p", [&] { k_bicg_p_cell<T><<<nb, 256, 0, st>>>(S); });
+      else if (fine_in == kFineS) L("bicg_s", [&] { k_bicg_s_cell<T><<<nb, 256, 0, st>>>(S); });
+      else L("gm_v", [&] { k_gm_v_cell<T><<<nb, 256, 0, st>>>(S, in_v()); });
     }
     static const char* rnames[] = {"mg_restrict_l0", "mg_restrict_l1", "mg_restrict_l2", "mg_restrict_l3",
                                    "mg_restrict_l4", "mg_restrict_l5", "mg_restrict_l6", "mg_restrict_l7+"};
     for (int l = 0; l < lc; ++l) {
-      if (tiled(mg[l]) && (l > 0 || fine_in != 3)) {   // GMRES forms its basis vector in the separate passes
+      if (tiled(mg[l]) && (l > 0 || fine_in != kFineV)) {   // GMRES forms its basis vector in the separate passes
         if (l > 0) down<false>(l, TileB<T>{mg[l].b});
-        else if (fine_in == 1) down<true>(0, TileInP<T>{S.kp, S.kr, S.kq});
+        else if (fine_in == kFineP) down<true>(0, TileInP<T>{S.kp, S.kr, S.kq});
         else down<true>(0, TileInS<T>{S.ks, S.kr, S.kv});
         continue;
       }
       for (int color = 0; color < 2; ++color) {
         const int zx = color == 0 ? 1 : 0;
-        if (l == 0 && fine_in == 1) smooth(mg[0], color, zx, 0, none, MgInP<T>{S.kp, S.kr, S.kq});
-        else if (l == 0 && fine_in == 2) smooth(mg[0], color, zx, 0, none, MgInS<T>{S.ks, S.kr, S.kv});
-        else if (l == 0 && fine_in == 3)
-          smooth(mg[0], color, zx, 0, none, MgInV<T>{S.kt, S.kp, S.gmV, S.gmT + kGmTInv, (size_t)S.neq});
-        else smooth(mg[l], color, zx, l, none, MgB<T>{mg[l].b});
+        if (l > 0) smooth(mg[l], color, zx, l, none, MgB<T>{mg[l].b});
+        else if (fine_in == kFineP) smooth(mg[0], color, zx, 0, none, MgInP<T>{S.kp, S.kr, S.kq});
+        else if (fine_in == kFineS) smooth(mg[0], color, zx, 0, none, MgInS<T>{S.ks, S.kr, S.kv});
+        else smooth(mg[0], color, zx, 0, none, in_v());
       }
       MGL<T> f = mg[l], c = mg[l + 1];
       L(rnames[l < 7 ? l : 7], [&] { k_mg_restrict_c0<T><<<cdiv(c.n, 256), 256, 0, st>>>(f, c, S.sc); });
@@ -1475,7 +1479,7 @@ class Solver final : public SolverBase {
       const MGL<T>& f = mg[l];
       const MGL<T>& c = mg[l + 1];
       const Prolong<T> pr = prolong_from(f, c, mg_w);
-      if (tiled(f) && (l > 0 || fine_in != 3)) {
+      if (tiled(f) && (l > 0 || fine_in != kFineV)) {
         if (l > 0) up<false>(l, pr);
         else up<true>(0, pr);
         continue;

@@ -1,6 +1,7 @@
 """GPU: where the multigrid cycle hands over to its single block.
 
-The block takes the last levels, always the coarsest among them, whatever
+GMRES forms its basis vector in level 0's first passes, and on its own where
+the block has level 0 too.  The block takes the last levels, always the coarsest among them, whatever
 mg_cta_columns says: below the coarsest level's 8 to 32 columns every level but
 it must run outside the block, and the pressure must be solved as the oracle
 does (the bounds that every FP64 and FP32+IR grid is held to).
@@ -21,4 +22,15 @@ def test_block_takes_the_coarsest_level(shape, columns, precision, oracle_mod, g
     p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
     po, _, _ = _case(*shape, 0, 1e-13)
     p.mg_cta_columns = columns
+    _against_oracle(p, po, depth, eta, oracle_mod)
+
+
+# levels of 64 columns and fewer are the block's from level 0 on; the others have a level above it
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", [(8, 8, 5), (16, 4, 3), (5, 4, 9), (60, 1, 4), (13, 5, 4), (8, 9, 21)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_gmres_on_small_grids(shape, precision, oracle_mod, gpu_lib):
+    p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
+    po, _, _ = _case(*shape, 0, 1e-13)
+    p.krylov_kernel = 2
     _against_oracle(p, po, depth, eta, oracle_mod)
