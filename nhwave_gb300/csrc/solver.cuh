@@ -398,7 +398,13 @@ class Solver final : public SolverBase {
         // 4.3, 6.70 -> 3.48.  Drawn at 1.5 because the further level costs
         // as much as it saves there (dy/dx = 1.37: 4.75 -> 5.53 ms/step
         // with it; 1.5: 7.96 -> 7.72).
-        if (!fixed && semi < 6) {
+        // A row of cells has no weak coupling, but pairs save a long one
+        // iterations too (1000 x 1: 8.2 -> 7.2).  From 64 cells on they would
+        // make a coarsest level of up to 32, which the block's sweeps solve
+        // poorly (60 x 1 x 8, dy/dx = 2: 18.6 iterations, 7.2 ms/step FP64; in
+        // fours 9.6 and 4.4; 100 x 1, dy/dx = 4: 10.3 -> 7.2).
+        const bool last_of_row = (f.M == 1 || f.N == 1) && f.M * f.N <= 64;
+        if (!fixed && semi < 6 && !last_of_row) {
           if (rx > 1 && ratio >= 1.5) {
             rx = 2; ry = 1; ratio *= 0.5; ++semi;
           } else if (ry > 1 && ratio * 1.5 <= 1.0) {

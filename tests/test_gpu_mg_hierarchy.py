@@ -34,3 +34,26 @@ def test_gmres_on_small_grids(shape, precision, oracle_mod, gpu_lib):
     po, _, _ = _case(*shape, 0, 1e-13)
     p.krylov_kernel = 2
     _against_oracle(p, po, depth, eta, oracle_mod)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [34, 60, 100, 301])
+@pytest.mark.parametrize("along_y", [False, True], ids=["x", "y"])
+def test_rows_do_not_depend_on_the_spacing_across(n, along_y, precision, gpu_lib):
+    """A row of cells has no coupling across it, so a wider cell must cost its
+    solves no more than a few iterations (a fifth, and two for the rounding)."""
+    from nhwave_gb300 import lib
+    its = []
+    for ratio in (1.0, 4.0):
+        p, depth, eta = _case(*((1, n) if along_y else (n, 1)), 6, precision, 1e-11 if precision == 0 else 1e-8)
+        if along_y:
+            p.dx = ratio * p.dy
+        else:
+            p.dy = ratio * p.dx
+        p.dt_max = p.dt_ini
+        g = lib.Scenario(p, depth, eta)
+        g.run(4)
+        s = g.scalars()
+        its.append(s.total_krylov_iters / s.poisson_solves)
+        g.close()
+    assert its[1] <= 1.2 * its[0] + 2.0, its
