@@ -1377,11 +1377,20 @@ class Solver final : public SolverBase {
   // (GB300, one level of 20 sigma levels, down / up in us): FP32 64 x 8
   // 9.3 / 8.3 -> 5.1 / 4.8, 128 x 32 10.5 / 8.8 -> 7.1 / 7.3, but 256 x 32
   // 10.3 / 8.8 -> 12.4 / 13.2; FP64 64 x 8 15.6 / 34 -> 12.6 / 15.0, 128 x 32
-  // 16.3 / 34 -> 19.6 / 24.3.  Aggregates must fill whole tiles.
+  // 16.3 / 34 -> 19.6 / 24.3.  Narrow levels leave most of a tile's rows
+  // empty, so the tiles are limited too: to those of 4096 columns and a
+  // quarter more in FP64, and to twice as many in FP32, whose idle lanes cost
+  // less (ms/step without tiles / with up to 256 / 512 / 1024 of them, 20
+  // sigma levels: FP64 4096 x 1 17.3 / 17.8 / 22.3 / 28.5, 2048 x 1 14.4 / 14.9
+  // / 19.6, 819 x 5, 410 tiles, 31.9 / 24.6 / 25.7, 63 x 65, 272 tiles, 16.0 /
+  // 12.7 / 12.4; FP32 4096 x 1 5.2 / 4.5 / 4.6 / 4.9, 819 x 5 8.0 / 5.3 / 4.6).
+  // Aggregates must fill whole tiles.
+  static constexpr int kTiles = kFP32 ? 512 : 320;
   static bool tiled(const MGL<T>& Lv) {
     auto pow2 = [](int r) { return r == 1 || r == 2 || r == 4; };
-    return (long long)Lv.M * Lv.N <= 4096 && pow2(Lv.rx) && pow2(Lv.ry);
+    return (long long)Lv.M * Lv.N <= 4096 && tiles_of(Lv) <= kTiles && pow2(Lv.rx) && pow2(Lv.ry);
   }
+  static unsigned tiles_of(const MGL<T>& Lv) { return cdiv(Lv.M, TileS::TX) * cdiv(Lv.N, TileS::TY); }
   // Levels a thread: two where one each would not fit a block, or where the
   // blocks (2 threads a cell) are more than the 152 SMs hold at 64 registers
   // a thread (FP32 128 x 32 x 20: 9.5 / 9.1 -> 7.1 / 7.3 us; 64 x 64 x 10
@@ -1393,7 +1402,7 @@ class Solver final : public SolverBase {
                                   "mg_down_l4", "mg_down_l5", "mg_down_l6", "mg_down_l7+"};
     const MGL<T> f = mg[l], c = mg[l + 1];
     const int nx = (int)cdiv(f.M, TileS::TX);
-    const unsigned nb = (unsigned)nx * cdiv(f.N, TileS::TY);
+    const unsigned nb = tiles_of(f);
     L(names[l < 7 ? l : 7], [&] {
       if (tile_lpt(f) == 1)
         k_mg_down<T, kFine, TileS, 1, In><<<nb, dim3(32, f.K), tile_smem<TileS, T>(f.K), st>>>(f, c, nx, S.sc, in);
@@ -1408,7 +1417,7 @@ class Solver final : public SolverBase {
                                   "mg_up_l4", "mg_up_l5", "mg_up_l6", "mg_up_l7+"};
     const MGL<T> f = mg[l];
     const int nx = (int)cdiv(f.M, TileS::TX);
-    const unsigned nb = (unsigned)nx * cdiv(f.N, TileS::TY);
+    const unsigned nb = tiles_of(f);
     L(names[l < 7 ? l : 7], [&] {
       if (tile_lpt(f) == 1)
         k_mg_up<T, kFine, TileS, 1><<<nb, dim3(32, f.K), tile_smem<TileS, T>(f.K), st>>>(f, pr, nx, S.sc);

@@ -57,3 +57,13 @@ def test_rows_do_not_depend_on_the_spacing_across(n, along_y, precision, gpu_lib
         its.append(s.total_krylov_iters / s.poisson_solves)
         g.close()
     assert its[1] <= 1.2 * its[0] + 2.0, its
+
+
+# narrow levels at the limits of the tiles: 320 (FP64) and 512 (FP32) of them, one more, and a row of 4096 columns
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", [(1280, 3, 2), (1281, 3, 2), (2, 2048, 2), (2049, 1, 3), (4096, 1, 2)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_narrow_levels_step_like_the_oracle(shape, precision, oracle_mod, gpu_lib):
+    p, depth, eta = _case(*shape, precision, 1e-13 if precision == 0 else 1e-10)
+    po, _, _ = _case(*shape, 0, 1e-13)
+    _against_oracle(p, po, depth, eta, oracle_mod)
