@@ -1057,8 +1057,20 @@ class Solver final : public SolverBase {
   // pay from about 2^20 cells (flux_y + omega_y 515 x 30 x 15: 28.7 against
   // 33.3 us in blocks, 1024 x 64 x 20: 86.0 against 76.5, 768 x 768 x 20: 758
   // against 545).
-  bool face_blocks_x() const { return !kFP32 && S.neq >= 65536; }
-  bool face_blocks_y() const { return S.neq >= (kFP32 ? 1 << 20 : 65536); }
+  // Narrow grids leave most of a block without faces (flux + omega in us, a
+  // face a thread against blocks; FP64, 82,000 cells: x, M = 12 235 against 501,
+  // 24 235 / 265, 33 235 / 236, 36 234 / 221, 48 230 / 177; y, M = 16 188 / 207, 20 192 / 146,
+  // 36 186 / 200, 40 186 / 179, N = 1 366 / 373, 2 290 / 267; FP32+IR across y,
+  // 1,060,000 cells, by the share of threads with a face: 0.6 77 / 91, 0.75 76 /
+  // 79, 0.93 78 / 74).
+  bool face_blocks_x() const { return !kFP32 && S.neq >= 65536 && S.M >= 33; }
+  bool face_blocks_y() const {
+    constexpr int rows = kFaceYy - 2;   // of faces
+    const double lanes = (double)S.M / ((double)kFaceYx * cdiv(S.M, kFaceYx));
+    if (!kFP32) return S.neq >= 65536 && S.N >= 2 && lanes >= 0.6;
+    return S.neq >= 1 << 20 && lanes * (S.N + 1) / ((double)rows * cdiv(S.N + 1, rows)) >= 0.8;
+  }
+  bool flux_z_walks() const { return !kFP32 && S.neq >= 65536; }
   // as few chunks of levels as leave about 8 blocks an SM
   template <class Face>
   void faces() {
@@ -1089,7 +1101,7 @@ class Solver final : public SolverBase {
     }
     if (face_blocks_y()) faces<FluxYFace<T>>();
     else box(OpFluxY{}, S.M, S.N + 1, S.K, S.IB, S.JB, S.KB);
-    if (kFP32 || !face_blocks_x()) box(OpFluxZ{}, S.M, S.N, S.K + 1, S.IB, S.JB, S.KB);
+    if (!flux_z_walks()) box(OpFluxZ{}, S.M, S.N, S.K + 1, S.IB, S.JB, S.KB);
     else if constexpr (!kFP32) flux_z_walk();
     if (S.keDxW) cells(OpKeSlopes{0});   // delxyzFun's DelxW / DelyW, read by the 3-D k-epsilon
     return check();
