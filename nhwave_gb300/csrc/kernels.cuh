@@ -3030,34 +3030,35 @@ struct OpColFactors {
   }
 };
 
-// The Poisson operator and right-hand side.  A block has 30 x 8 columns with a
-// ring of halo threads and walks kc levels up: DelxS / DelyS and the
+// The Poisson operator and right-hand side.  A block has (PX - 2) x (PY - 2)
+// columns with a ring of halo threads and walks kc levels up: DelxS / DelyS and the
 // velocities at the level's faces, which up to five cells read, are formed
 // once a cell and passed through shared memory (the halo columns form only
 // theirs), and a level's velocities are converted once.  Bound by the FP64
 // pipe: a cell at a time it takes about 80 FP64 operations a cell, so about 45
 // (GB300 FP32+IR, 1024 x 64 x 20: 215 -> 179 us; 768 x 768 x 20: 1860 -> 1420
-// us, coefT included, whose copy of its own was 200).
-constexpr int kPcX = 32, kPcY = 10;
+// us, coefT included, whose copy of its own was 200).  30 x 8 columns, and 8 x
+// 30, 2 x 78 or 78 x 2 on narrow grids (poisson_blocks), where the same values
+// are formed by fewer threads.
 // a b + c as the two forms are built: fused in FP32+IR, rounded twice in FP64
 template <class T>
 __device__ __forceinline__ double mad_as(double a, double b, double c) {
   if constexpr (sizeof(T) == 4) return fma(a, b, c);
   else return a * b + c;
 }
-template <class T>
-__global__ void __launch_bounds__(kPcX * kPcY) k_poisson_coef(Dev<T> S, int kc, int ntile_x, int ntile_y) {
+template <class T, int PX, int PY>
+__global__ void __launch_bounds__(PX * PY) k_poisson_coef(Dev<T> S, int kc, int ntile_x, int ntile_y) {
   if (gated_off(S)) return;
-  __shared__ double sh[2][4][kPcY][kPcX];   // [level parity]: DelxS, DelyS, U and V at the level's face
+  __shared__ double sh[2][4][PY][PX];   // [level parity]: DelxS, DelyS, U and V at the level's face
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int b = blockIdx.x, tile = b % ntile_x, r = b / ntile_x, trow = r % ntile_y, ch = r / ntile_y;
-  const int i = S.IB + tile * (kPcX - 2) + tx - 1, j = S.JB + trow * (kPcY - 2) + ty - 1;
+  const int i = S.IB + tile * (PX - 2) + tx - 1, j = S.JB + trow * (PY - 2) + ty - 1;
   const int k0 = S.KB + ch * kc, k1 = min(S.KE, k0 + kc - 1);
   const bool inx = i >= S.IB && i <= S.IE, iny = j >= S.JB && j <= S.JE, in = inx && iny;
-  const bool own = in && tx > 0 && tx < kPcX - 1 && ty > 0 && ty < kPcY - 1;
+  const bool own = in && tx > 0 && tx < PX - 1 && ty > 0 && ty < PY - 1;
   // which of a column's values its neighbours or itself read
-  const bool needx = iny && i >= S.IB - 1 && i <= S.IE + 1 && ty > 0 && ty < kPcY - 1;
-  const bool needy = inx && j >= S.JB - 1 && j <= S.JE + 1 && tx > 0 && tx < kPcX - 1;
+  const bool needx = iny && i >= S.IB - 1 && i <= S.IE + 1 && ty > 0 && ty < PY - 1;
+  const bool needy = inx && j >= S.JB - 1 && j <= S.JE + 1 && tx > 0 && tx < PX - 1;
   const long long sy = S.sy, sz = S.sz;
   const long long q = (needx || needy) ? i2(S, i, j) : 0, o2 = q;
   double hx = 0.0, ex = 0.0, hy = 0.0, ey = 0.0;   // zero outside (src/pressure.F:494-505)
@@ -3074,7 +3075,7 @@ __global__ void __launch_bounds__(kPcX * kPcY) k_poisson_coef(Dev<T> S, int kc, 
     if (own) wd = widen(S.W[o]);
   }
   for (int k = k0; k <= k1; ++k) {
-    double(*s)[kPcY][kPcX] = sh[k & 1];
+    double(*s)[PY][PX] = sh[k & 1];
     const long long o = o2 + sz * k;
     const double sgk = S.sig[k], omk = 1. - sgk;
     // Uf/Vf: linear interpolation to sig(k) (src/nhwave.F:1346-1355)

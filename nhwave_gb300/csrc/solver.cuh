@@ -1128,15 +1128,35 @@ class Solver final : public SolverBase {
     cudaStreamWaitEvent(st, ev_join, 0);
     mg_forked = false;
   }
+  // as few chunks of levels as leave about 8 blocks an SM
+  template <int PX, int PY>
+  void poisson_coef() {
+    const int nx = (int)cdiv(S.M, PX - 2), ny = (int)cdiv(S.N, PY - 2);
+    const int chunks = (int)std::min<long long>(S.K, std::max<long long>(1, 152LL * 8 / ((long long)nx * ny)));
+    const int kc = (S.K + chunks - 1) / chunks;
+    const unsigned nb = (unsigned)nx * ny * cdiv(S.K, kc);
+    L("poisson_coef", [&] { k_poisson_coef<T, PX, PY><<<nb, dim3(PX, PY), 0, st>>>(S, kc, nx, ny); });
+  }
+  // The block shape with the fewest threads for the grid's columns, and 30 x 8
+  // columns, whose rows are the longest reads, unless another saves a quarter of
+  // them; below 2048 columns, where the launch's latency decides, a third (us,
+  // 30 x 8 against the shape taken, 20 levels: 1 x 4100 402 / 55, 4 x 1025 107 /
+  // 33, 16 x 256 35 / 27, 40 x 1500 307 / 223, 4100 x 1 60 / 33; FP32+IR 32 x 1875
+  // 395 / 223; 10 levels: 12 x 125 18.4 / 14.3, but 16 x 93 12.3 / 14.3 in 8 x 30)
+  void poisson_blocks() {
+    auto threads = [&](int px, int py) { return (long long)px * py * cdiv(S.M, px - 2) * cdiv(S.N, py - 2); };
+    const double most = (long long)S.M * S.N < 2048 ? 0.65 : 0.75;
+    const long long n = (long long)(threads(32, 10) * most), ny = threads(10, 32), nyy = threads(4, 80),
+                    nxx = threads(80, 4);
+    const long long best = std::min({n, ny, nyy, nxx});
+    if (best == n) poisson_coef<32, 10>();
+    else if (best == ny) poisson_coef<10, 32>();
+    else if (best == nyy) poisson_coef<4, 80>();
+    else poisson_coef<80, 4>();
+  }
   void poisson_setup() {
     incols(OpColFactors{});
-    {
-      const int nx = (int)cdiv(S.M, kPcX - 2), ny = (int)cdiv(S.N, kPcY - 2);
-      const int chunks = (int)std::min<long long>(S.K, std::max<long long>(1, 152LL * 8 / ((long long)nx * ny)));
-      const int kc = (S.K + chunks - 1) / chunks;
-      const unsigned nb = (unsigned)nx * ny * cdiv(S.K, kc);
-      L("poisson_coef", [&] { k_poisson_coef<T><<<nb, dim3(kPcX, kPcY), 0, st>>>(S, kc, nx, ny); });
-    }
+    poisson_blocks();
     if (use_mg && mg.size() > 1) {
       cudaEventRecord(ev_fork, st);
       cudaStreamWaitEvent(mg_st, ev_fork, 0);
