@@ -2,6 +2,7 @@
 // device arena, the reference's subroutine sequence as kernel launches, the
 // Poisson solve with FP64 iterative refinement, and field transfer.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -679,30 +680,49 @@ class Solver final : public SolverBase {
     *eb = d.kind == 2 ? 4 : 8;
     return NHW_OK;
   }
-  // the device address of `bytes` of page-locked host memory, nullptr for
-  // other memory
-  static void* mapped(void* host, size_t bytes) {
-    cudaPointerAttributes a{}, e{};
-    char* h = static_cast<char*>(host);
-    if (cudaPointerGetAttributes(&a, h) != cudaSuccess || cudaPointerGetAttributes(&e, h + bytes - 1) != cudaSuccess) {
-      cudaGetLastError();
+  // The device address of `bytes` of page-locked host memory that a kernel can
+  // store `elem`-byte values to, nullptr for any other: the address must be a
+  // multiple of elem (a copy takes any, a store does not), all of the bytes must
+  // lie in one allocation or registration (between two there may be a gap), and
+  // the device must be allowed to write them.
+  static void* mapped(void* host, size_t bytes, size_t elem) {
+    static const auto get = [] {
+      void* f = nullptr;
+      cudaDriverEntryPointQueryResult r;
+      if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+          r != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        f = nullptr;
+      }
+      return reinterpret_cast<decltype(&cuPointerGetAttributes)>(f);
+    }();
+    if (!get) return nullptr;
+    CUmemorytype type = (CUmemorytype)0;   // stays so for pageable memory
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    unsigned managed = 0;
+    unsigned long long access = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                  CU_POINTER_ATTRIBUTE_IS_MANAGED,       CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void* out[] = {&type, &dev, &start, &size, &managed, &access};
+    if (get(6, what, out, (CUdeviceptr)host) != CUDA_SUCCESS) return nullptr;
+    if (type != CU_MEMORYTYPE_HOST || managed || !dev || dev % elem ||
+        access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE || dev < start || dev - start > size ||
+        size - (dev - start) < bytes)
       return nullptr;
-    }
-    if (a.type != cudaMemoryTypeHost || e.type != cudaMemoryTypeHost || !a.devicePointer || !e.devicePointer ||
-        (char*)e.devicePointer - (char*)a.devicePointer != (ptrdiff_t)(bytes - 1))
-      return nullptr;
-    return a.devicePointer;
+    return (void*)dev;
   }
   // Into page-locked memory the packing kernel writes directly, which spares
   // the staging pass and the copy's start (GB300, one field read with its
   // call: 0.6 MB 25 -> 21 us, 3 MB 37 -> 32 us, 13 MB 104 -> 87 us); other host
-  // memory goes through the staging buffer and the copy engine.
+  // memory (mapped) goes through the staging buffer and the copy engine.
   int get_field(int f, void* host) override {
     FieldDesc d = desc(f);
     if (!d.ptr || !host) return NHW_ERR_ARG;
     const long long n = (long long)d.nx * d.ny * d.nz;
-    const size_t bytes = (size_t)n * (d.kind == 2 ? 4 : 8);
-    void* direct = mapped(host, bytes);
+    const size_t elem = d.kind == 2 ? 4 : 8, bytes = (size_t)n * elem;
+    void* direct = mapped(host, bytes, elem);
     double* out = direct ? (double*)direct : d_stage;
     k_pack<T><<<cdiv(n, 256), 256, 0, st>>>(d.ptr, d.kind, out, (int*)out, d.nx, d.ny, d.nz, S.sy, S.sz);
     NHW_CU(cudaGetLastError());
