@@ -309,10 +309,11 @@ struct FinT {
 template <class T>
 struct FinXr {
   double tol_in, red, rho, alpha, omega;   // read when the kernel starts
-  int itmax_in, it, total_it, inner_total;
+  int itmax_in, it, inner_total;
+  int64_t total_it;
   __device__ explicit FinXr(const DevScal* sc)
       : tol_in(sc->tol_in), red(sc->red[0]), rho(sc->rho), alpha(sc->alpha), omega(sc->omega),
-        itmax_in(sc->itmax_in), it(sc->it + 1), total_it(sc->total_it + 1), inner_total(sc->inner_total + 1) {}
+        itmax_in(sc->itmax_in), it(sc->it + 1), inner_total(sc->inner_total + 1), total_it(sc->total_it + 1) {}
   __device__ void operator()(const Dev<T>& S2, double* a) const {
     DevScal* sc = S2.sc;
     sc->it = it;
