@@ -45,12 +45,8 @@ def test_rows_do_not_depend_on_the_spacing_across(n, along_y, precision, gpu_lib
     from nhwave_gb300 import lib
     its = []
     for ratio in (1.0, 4.0):
-        p, depth, eta = _case(*((1, n) if along_y else (n, 1)), 6, precision, 1e-11 if precision == 0 else 1e-8)
-        if along_y:
-            p.dx = ratio * p.dy
-        else:
-            p.dy = ratio * p.dx
-        p.dt_max = p.dt_ini
+        p, depth, eta = _case(*((1, n) if along_y else (n, 1)), 8, precision, 1e-11 if precision == 0 else 1e-8)
+        p.dx, p.dy = (0.1 * ratio, 0.1) if along_y else (0.1, 0.1 * ratio)
         g = lib.Scenario(p, depth, eta)
         g.run(4)
         s = g.scalars()
