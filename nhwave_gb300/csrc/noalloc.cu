@@ -63,6 +63,12 @@ __device__ __forceinline__ double from_key(long long k) {
   return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
 
+// a >= b where b is a normal number that no rounding to zero or infinity made
+__device__ __forceinline__ bool above(double a, double b) {
+  const unsigned long long lo = 0x0010000000000000ull, hi = 0x7ff0000000000000ull;   // bits of 2^-1022 and infinity
+  return a >= b && (unsigned long long)__double_as_longlong(b) - lo < hi - lo;
+}
+
 // the block's minimum of m and, with kAll, maxima of u and v, valid in thread 0
 template <bool kAll>
 __device__ __forceinline__ void block_reduce(long long& m, long long& u, long long& v) {
@@ -108,7 +114,7 @@ __device__ __forceinline__ void block_reduce(long long& m, long long& u, long lo
 // integers off the FP64 pipe (1.2 TFLOP/s on GB300).  The dsig D / |W| of the
 // levels are divided only where products, with a margin far above their
 // rounding, do not show the smallest of them to be above dx/(|U| + sqrt(g D))
-// or its y counterpart.  Read once, coalesced along i: bound by the launch on
+// or its y counterpart; products out of range and negative dsig show nothing.  Read once, coalesced along i: bound by the launch on
 // small grids and by HBM on large ones (GB300, a call in a graph with its
 // memset: 256 x 8 x 10 33.1 -> 10.4 us, 1024 x 64 x 20 129 -> 18.6 us,
 // 600 x 300 x 24 348 -> 30.9 us, whose bytes alone take 0.1, 5 and 15 us).
@@ -144,7 +150,7 @@ k_dt_min_noalloc(const double* __restrict__ U, const double* __restrict__ V, con
     bv = max_ll(bv, __double_as_longlong(tv));
     const double a = __longlong_as_double(sg) * Dq, wm = w < 0 ? kSmall : na_max(__longlong_as_double(w), kSmall);
     const double wf = wm * 1.0000001;
-    if (!(a * tu >= dx * wf || a * tv >= dy * wf))
+    if (sg < 0 || !(above(a * tu, dx * wf) || above(a * tv, dy * wf)))
       for (int k = k0; k < k1; ++k) m = na_min(m, dsig[NG + k] * Dq / na_max(fabs(W[c3 + lev * (k - k0)]), kSmall));
   }
   long long key = order_key(m);
