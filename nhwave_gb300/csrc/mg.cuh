@@ -291,10 +291,10 @@ struct MgInV {
 // operations take some 80 cycles each in a chain).  As loops over shared
 // memory the same solve waits for its loads level by level (GB300, one warp:
 // FP32 10 levels 1580 -> 440 cycles, 20 levels 1690 -> 800; FP64 10 levels
-// 5050 -> 4290).
+// 5050 -> 4290).  put may write rhs itself, so rhs is not __restrict__.
 template <int NS, int KM, int CH, class T, class Put>
-__device__ __forceinline__ void line_solve_regs(T* __restrict__ rhs, const T* __restrict__ a,
-                                                const T* __restrict__ inv, const T* __restrict__ c, int K, Put put) {
+__device__ __forceinline__ void line_solve_regs(T* rhs, const T* __restrict__ a, const T* __restrict__ inv,
+                                                const T* __restrict__ c, int K, Put put) {
   constexpr int NC = KM / CH;
   constexpr bool kKeep = sizeof(T) == 4;
   static_assert(KM % CH == 0, "whole chunks");
@@ -346,7 +346,7 @@ __device__ __forceinline__ void line_solve_regs(T* __restrict__ rhs, const T* __
 // The same by the number of levels, and in loops through rhs beyond 20 levels
 // and in FP64 (k_mg_smooth_blk's blocks of 1024 threads leave it no registers).
 template <int NS, class T, class Put>
-__device__ __forceinline__ void line_solve(T* __restrict__ rhs, const T* __restrict__ a, const T* __restrict__ inv,
+__device__ __forceinline__ void line_solve(T* rhs, const T* __restrict__ a, const T* __restrict__ inv,
                                            const T* __restrict__ c, int K, Put put) {
   if constexpr (sizeof(T) == 4) {
     if (K <= 10) return line_solve_regs<NS, 10, 5>(rhs, a, inv, c, K, put);

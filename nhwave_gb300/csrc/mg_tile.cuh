@@ -101,7 +101,7 @@ __device__ __forceinline__ void line_solve_smem(T* __restrict__ x, const T* __re
 template <class T>
 constexpr int kAhead = sizeof(T) == 4 ? 5 : 2;
 template <int NS, int CH, class T>
-__device__ __forceinline__ void line_solve_tile(T* __restrict__ x, const T* __restrict__ a, const T* __restrict__ inv,
+__device__ __forceinline__ void line_solve_tile(T* x, const T* __restrict__ a, const T* __restrict__ inv,
                                                 const T* __restrict__ c, int K) {
   auto put = [&](int k, T z) { x[k * NS] = z; };
   if (K <= 10) line_solve_regs<NS, 10, CH>(x, a, inv, c, K, put);
