@@ -133,22 +133,6 @@ __device__ __forceinline__ double operator/(double a, const Quot<T>& q) {
   else return a / q.b;
 }
 
-// the same for divisors in the working precision R of a cell kernel
-template <class R>
-struct QuotR {
-  R b, r;
-};
-template <class R>
-__device__ __forceinline__ QuotR<R> over_r(R b) {
-  if constexpr (sizeof(R) == 4) return QuotR<R>{b, (R)1 / b};
-  else return QuotR<R>{b, (R)0};
-}
-template <class R>
-__device__ __forceinline__ R operator/(R a, const QuotR<R>& q) {
-  if constexpr (sizeof(R) == 4) return a * q.r;
-  else return a / q.b;
-}
-
 __device__ __forceinline__ int mirror(int i, int b, int e) {
   return i < b ? 2 * b - 1 - i : (i > e ? 2 * e + 1 - i : i);
 }
@@ -1540,7 +1524,9 @@ struct OpVelBcB {
 // DelxSc / DelySc and DelxSl / DelySl of the last sigma_transform (zero
 // before the first one), which OpDiffusion reads: formed once a column and
 // level, since each of that stencil's 30 uses costs two FP64 divisions
-// (515 x 30 x 15 FP32+IR: 679 us with the slopes in place, now below 30).
+// (515 x 30 x 15 FP32+IR: diffusion 677 us with the slopes in place, 60 + 19 for
+// the slopes).  The other quotients are divisions in both forms: multiplied by
+// reciprocals in FP32, OpDiffusion would take 23 us but round twice.
 struct OpViscSlopes {
   static constexpr const char* kName = "visc_slopes";
   template <class T>
@@ -1576,9 +1562,8 @@ struct OpDiffusion {
     const T* DV = S.DV;
     const T* DW = S.DW;
     auto F = [&](const T* a, int ii, int jj, int kk) -> R { return a[i3(S, ii, jj, kk)]; };
-    const QuotR<R> dx = over_r<R>((R)S.dx), dy = over_r<R>((R)S.dy);
-    const R cmu = (R)S.v_cmu;
-    const QuotR<R> sch = over_r<R>((R)S.v_schmidt);
+    const R dx = (R)S.dx, dy = (R)S.dy;
+    const R cmu = (R)S.v_cmu, sch = (R)S.v_schmidt;
     // CmuHt of a cell; face viscosity between two cells; cell viscosity
     auto H = [&](int ii, int jj, int kk) -> R { return (R)S.CmuHt[i3(S, ii, jj, kk)]; };
     auto nuF = [&](R ha, R hb) -> R { return (R)0.5 * (cmu + cmu) + (R)0.5 * (ha + hb) / sch; };
@@ -1591,11 +1576,10 @@ struct OpDiffusion {
     auto lv = [&](int n) { return S.lvv[n * S.Kloc + k]; };
     const double L1top = lv(kLvL1t), L2top = lv(kLvL2t), L1bot = lv(kLvL1b), L2bot = lv(kLvL2b);
     const R rck = (R)lv(kLvCk), rck1 = (R)lv(kLvCk1);
-    const QuotR<R> qck = over_r<R>(rck), qck1 = over_r<R>(rck1), qcc = over_r<R>(rck + rck1);
     const R ac = (R)lv(kLvAc), bc = (R)lv(kLvBc), gc = (R)lv(kLvGc);
     const R nuH_top = ((R)L1top * cmu + (R)L2top * cmu) + ((R)L1top * h0 + (R)L2top * H(i, j, k + 1)) / sch;
     const R nuH_bot = ((R)L1bot * cmu + (R)L2bot * cmu) + ((R)L1bot * H(i, j, k - 1) + (R)L2bot * h0) / sch;
-    const QuotR<R> Dc = over_r<R>((R)S.D[c]), dsk = over_r<R>((R)S.dsig[k]);
+    const R Dc = (R)S.D[c], dsk = (R)S.dsig[k];
     auto s3 = [&](const T* a, bool y, int ii, int jj) -> R {   // a F(k-1) Sc(k-1) + b .. + c ..
       auto sc = [&](int kk) { return y ? Scy(ii, jj, kk) : Scx(ii, jj, kk); };
       return ac * F(a, ii, jj, k - 1) * sc(k - 1) + bc * F(a, ii, jj, k) * sc(k) + gc * F(a, ii, jj, k + 1) * sc(k + 1);
@@ -1615,9 +1599,9 @@ struct OpDiffusion {
       const T* sl = y ? S.vly : S.vlx;
       const R st = sl[o + S.sz], sb = sl[o];
       const R Pq = nuH_top * st - nuH_bot * sb, Sq = nuH_top * st + nuH_bot * sb;
-      cA = Pq * ac / dsk + Sq / qck1 / qcc;
-      cB = Pq * bc / dsk - Sq / qck1 / qck;
-      cC = Pq * gc / dsk + Sq / qck / qcc;
+      cA = Pq * ac / dsk + Sq / rck1 / (rck + rck1);
+      cB = Pq * bc / dsk - Sq / rck1 / rck;
+      cC = Pq * gc / dsk + Sq / rck / (rck + rck1);
     };
     R xA, xB, xC, yA, yB, yC;
     vco(false, xA, xB, xC);
