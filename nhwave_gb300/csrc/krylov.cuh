@@ -383,12 +383,8 @@ __global__ void __launch_bounds__(256) k_bicg_init(Dev<T> S) {
       const T r = S.kr0[t];
       S.kr[t] = r;
       S.kx[t] = (T)0;
-      if (S.kq) {
-        S.kq[t] = (T)0;
-      } else {
-        S.kp[t] = (T)0;
-        S.kv[t] = (T)0;
-      }
+      S.kp[t] = (T)0;
+      S.kv[t] = (T)0;
       v[0] += (A)r * (A)r;
     }
   }
@@ -580,7 +576,6 @@ __global__ void __launch_bounds__(256) k_bicg_xr(Dev<T> S) {
       x[t] = x[t] + alpha * ph[t] + omega * sh[t];
       const T r = ss[t] - omega * tt[t];
       rr[t] = r;
-      if (S.kq) S.kq[t] = S.kp[t] - omega * S.kv[t];   // for the next p, which the smoother forms
       v[0] += (A)r0[t] * (A)r;
       v[1] += (A)r * (A)r;
     }
@@ -605,7 +600,9 @@ __global__ void __launch_bounds__(256) k_xupd(Dev<T> S) {
 // cells, keeps the values that the sums need in shared memory, and the
 // cluster's first block adds them from there in the order of the kernel above,
 // so that vectors and sums are the same bit for bit.  Used up to kSlicedBlocks
-// blocks: beyond, the kernels above fill the SMs by themselves.
+// blocks: beyond, the kernels above fill the SMs by themselves.  The grids whose
+// level 0 takes the tiles of mg_tile.cuh, and with them kq, are among these: at
+// most 4096 columns of 64 levels are 128 blocks.
 constexpr int kSlices = kCPT;        // a portable cluster; kCPT cells a thread, one a slice
 constexpr int kSlicedBlocks = 152;
 constexpr int kSliceLevels = (64 + kSlices - 1) / kSlices;   // levels of a column chunk a slice (K <= 64)
@@ -754,7 +751,7 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(256) k_bicg_xr
     S.kx[ic] = S.kx[ic] + alpha * S.kph[ic] + omega * S.ksh[ic];
     const T r = S.ks[ic] - omega * S.kt[ic];
     S.kr[ic] = r;
-    if (S.kq) S.kq[ic] = S.kp[ic] - omega * S.kv[ic];
+    if (S.kq) S.kq[ic] = S.kp[ic] - omega * S.kv[ic];   // for the next p, which the tiles form
     sr[tid] = r;
   }
   const T* __restrict__ r0 = S.kr0;
@@ -887,7 +884,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) k_bicg_xr_pr(De
     x[t] = x[t] + alpha * ph[t] + omega * sh[t];
     const T r = ss[t] - omega * tt[t];
     rr[t] = r;
-    if (S.kq) S.kq[t] = S.kp[t] - omega * S.kv[t];
     return Two<A>{(A)r0[t], (A)r};
   }, [&](const Two<A>& q, A (&v)[2]) {
     v[0] += q.a * q.b;

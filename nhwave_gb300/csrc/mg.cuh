@@ -212,8 +212,8 @@ __device__ __forceinline__ T off_column_p(const MGL<T>& L, const T* __restrict__
 //
 // Right-hand sides of a half-sweep:
 //   MgB            b as stored;
-//   MgInP / MgInS  the BiCGSTAB vectors p = r + beta q (q = p - omega v, from
-//                  k_bicg_xr) and s = r - alpha v, formed on the fine level by the sweep that
+//   MgInP / MgInS  the BiCGSTAB vectors p = r + beta (p - omega v) and
+//                  s = r - alpha v, formed on the fine level by the sweep that
 //                  owns each column (colour 0 in the first half-sweep, colour 1
 //                  in the second) and stored -- no launch of their own.
 //
@@ -231,15 +231,16 @@ template <class T>
 struct MgInP {
   T* p;
   const T* r;
-  const T* q;
-  T beta = (T)0;   // set by bind
+  const T* v;
+  T beta = (T)0, omega = (T)0;   // set by bind
   __device__ __forceinline__ MgInP bind(const DevScal* sc) const {
     MgInP u = *this;
     u.beta = (T)sc->beta;
+    u.omega = (T)sc->omega;
     return u;
   }
   __device__ __forceinline__ T operator()(const DevScal*, int ic, int, int, int) const {
-    const T val = r[ic] + beta * q[ic];
+    const T val = r[ic] + beta * (p[ic] - omega * v[ic]);
     p[ic] = val;
     return val;
   }
@@ -877,13 +878,14 @@ __global__ void __launch_bounds__(256) k_mg_factor(MGL<T> L, T* lcp, T* linv, T*
   }
 }
 
-// p = r + beta q   /   s = r - alpha v   (cell kernels when MG preconditions)
+// p = r + beta (p - omega v)   /   s = r - alpha v   (cell kernels when MG preconditions)
 template <class T>
 __global__ void __launch_bounds__(256) k_bicg_p_cell(Dev<T> S) {
   if (S.sc->conv) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S.neq) return;
-  S.kp[t] = S.kr[t] + (T)S.sc->beta * S.kq[t];
+  const T beta = (T)S.sc->beta, omega = (T)S.sc->omega;
+  S.kp[t] = S.kr[t] + beta * (S.kp[t] - omega * S.kv[t]);
 }
 template <class T>
 __global__ void __launch_bounds__(256) k_bicg_s_cell(Dev<T> S) {

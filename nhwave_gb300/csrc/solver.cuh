@@ -365,6 +365,7 @@ class Solver final : public SolverBase {
     add(&S.partials, sizeof(double) * 8 * (cdiv((long long)neq, 256) + 8));
     // multigrid levels: horizontal 2x2 aggregation while a direction has >= 4 cells
     use_mg = p.precond == 0;
+    use_gmres = use_mg && p.krylov_kernel == 2;
     mg_w = (T)(p.mg_weight > 0.f ? p.mg_weight : 1.0f);
     if (p.mg_coarse_sweeps > 0) mg_coarse_sweeps = p.mg_coarse_sweeps;
     if (p.mg_cta_columns > 0) cta_columns = p.mg_cta_columns;
@@ -422,8 +423,10 @@ class Solver final : public SolverBase {
     std::vector<T**> mgptr;
     if (use_mg) {
       add(&S.sp0, sizeof(T) * 7 * 2 * (size_t)K * N * ((M + 1) / 2));
-      add(&S.kq, sizeof(T) * neq);
-      add(&mg[0].xp, sizeof(T) * neq);
+      if (tiles_at(0)) {
+        add(&S.kq, sizeof(T) * neq);
+        add(&mg[0].xp, sizeof(T) * neq);
+      }
     }
     if (kFP32 && !p.hllc)   // 2-D face states (scratch of one stage)
       for (T** ft : {&S.fxT, &S.fyT}) add(ft, sizeof(T) * 6 * n2);
@@ -436,13 +439,12 @@ class Solver final : public SolverBase {
       add((T**)&mg[l].lcp, sizeof(T) * nl);
       add((T**)&mg[l].linv, sizeof(T) * nl);
       add(&mg[l].x, sizeof(T) * nl);
-      add(&mg[l].xp, sizeof(T) * nl);
+      if (tiles_at((int)l)) add(&mg[l].xp, sizeof(T) * nl);
       add(&mg[l].b, sizeof(T) * nl);
     }
     // persistent solve: every block resident (cooperative launch), at most
     // one block per 2048 unknowns
     use_persistent = use_mg && p.krylov_kernel == 1 && (int)mg.size() <= kPsMaxLevels;
-    use_gmres = use_mg && p.krylov_kernel == 2;
     if (use_gmres) {
       add(&S.gmV, sizeof(T) * (kGmMax + 1) * (size_t)neq);
       add(&S.gmZ, sizeof(T) * kGmMax * (size_t)neq);
@@ -1442,6 +1444,9 @@ class Solver final : public SolverBase {
     auto pow2 = [](int r) { return r == 1 || r == 2 || r == 4; };
     return (long long)Lv.M * Lv.N <= 4096 && tiles_of(Lv) <= kTiles && pow2(Lv.rx) && pow2(Lv.ry);
   }
+  // whether level l's half of the V-cycle runs so: GMRES forms its basis vector
+  // in the separate passes of level 0
+  bool tiles_at(int l) const { return l < first_block_level() && tiled(mg[l]) && (l > 0 || !use_gmres); }
   static unsigned tiles_of(const MGL<T>& Lv) { return cdiv(Lv.M, TileS::TX) * cdiv(Lv.N, TileS::TY); }
   // Levels a thread: two where one each would not fit a block, or where the
   // blocks (2 threads a cell) are more than the 152 SMs hold at 64 registers
@@ -1504,7 +1509,7 @@ class Solver final : public SolverBase {
     static const char* rnames[] = {"mg_restrict_l0", "mg_restrict_l1", "mg_restrict_l2", "mg_restrict_l3",
                                    "mg_restrict_l4", "mg_restrict_l5", "mg_restrict_l6", "mg_restrict_l7+"};
     for (int l = 0; l < lc; ++l) {
-      if (tiled(mg[l]) && (l > 0 || fine_in != kFineV)) {   // GMRES forms its basis vector in the separate passes
+      if (tiles_at(l)) {
         if (l > 0) down<false>(l, TileB<T>{mg[l].b});
         else if (fine_in == kFineP) down<true>(0, TileInP<T>{S.kp, S.kr, S.kq});
         else down<true>(0, TileInS<T>{S.ks, S.kr, S.kv});
@@ -1513,7 +1518,7 @@ class Solver final : public SolverBase {
       for (int color = 0; color < 2; ++color) {
         const int zx = color == 0 ? 1 : 0;
         if (l > 0) smooth(mg[l], color, zx, l, none, MgB<T>{mg[l].b});
-        else if (fine_in == kFineP) smooth(mg[0], color, zx, 0, none, MgInP<T>{S.kp, S.kr, S.kq});
+        else if (fine_in == kFineP) smooth(mg[0], color, zx, 0, none, MgInP<T>{S.kp, S.kr, S.kv});
         else if (fine_in == kFineS) smooth(mg[0], color, zx, 0, none, MgInS<T>{S.ks, S.kr, S.kv});
         else smooth(mg[0], color, zx, 0, none, in_v());
       }
@@ -1546,7 +1551,7 @@ class Solver final : public SolverBase {
       const MGL<T>& f = mg[l];
       const MGL<T>& c = mg[l + 1];
       const Prolong<T> pr = prolong_from(f, c, mg_w);
-      if (tiled(f) && (l > 0 || fine_in != kFineV)) {
+      if (tiles_at(l)) {
         if (l > 0) up<false>(l, pr);
         else up<true>(0, pr);
         continue;

@@ -199,7 +199,7 @@ struct Dev {
   T *lcp, *linv;      // line preconditioner factors [neq]
   T* sp0;             // colour-split copy of the level-0 smoother's operator (MGL::sp), or nullptr
   T *kx, *kr, *kr0, *kp, *kph, *kv, *ks, *ksh, *kt;
-  T* kq;              // p - omega v of the last iteration (multigrid-preconditioned solve only, else nullptr)
+  T* kq;              // p - omega v of the last iteration (where tiles form p, mg_tile.cuh, else nullptr)
   // velocities of the last two steps, read by the Orlanski boundary
   // (BC_Xn = 6) only, else nullptr
   T *U0, *V0, *W0, *U00, *V00, *W00;
