@@ -164,7 +164,8 @@ typedef struct nhw_params {
                                               without it BiCGSTAB runs phase by phase */
   int32_t mg_coarse_sweeps;                /* red-black sweeps on the coarsest level (0: 2) */
   int32_t mg_cta_columns;                  /* levels with at most this many columns run in
-                                              one thread block (0: 64)                */
+                                              one thread block (0: 64); the coarsest
+                                              always does                             */
   int32_t mg_aggregate;                    /* multigrid aggregates of n x n columns (0: 2) */
   int32_t test_barrier_extra;              /* test hook, 0 in use: the persistent solve's
                                               grid barrier also waits for this many blocks
@@ -379,7 +380,8 @@ int nhw_profile_report(nhw_handle* h, char* buf, int32_t buflen);
 
 /* Device microseconds of one level-0 multigrid half-sweep, the largest
  * kernel of a non-hydrostatic step, on this handle's current operator (call
- * it after a step).  Events around single launches add several microseconds
+ * it after a step).  Grids of at most 4096 columns solve with half V-cycles in
+ * one launch instead (GMRES apart): there the figure is no part of a step.  Events around single launches add several microseconds
  * to each, so the launches are timed in bulk: a CUDA graph of `reps` rounds,
  * each a write of `flush_bytes` bytes (0: none; more than the 129 MB L2
  * evicts it) followed by the four level-0 half-sweeps of a V-cycle, minus a

@@ -1516,17 +1516,11 @@ struct OpVelBcB {
 // =========================================================================
 //   viscous flow with constant viscosities (IVTURB = IHTURB = 1)
 // =========================================================================
-// diffusion (src/nhwave.F:6785-7141): the explicit viscous terms of R2-R4,
-// one thread per interior cell, from the stage's starting DU/DV/DW and the
-// sigma slopes of the last sigma_transform (zero before the first one).
-// Cmu = Visc; CmuHt per cell (Cmut_min until eval_turb).  Each bracket
-// keeps the reference's evaluation order (bit-exact in the FP64 form).
 // DelxSc / DelySc and DelxSl / DelySl of the last sigma_transform (zero
 // before the first one), which OpDiffusion reads: formed once a column and
 // level, since each of that stencil's 30 uses costs two FP64 divisions
 // (515 x 30 x 15 FP32+IR: diffusion 677 us with the slopes in place, 60 + 19 for
-// the slopes).  The other quotients are divisions in both forms: multiplied by
-// reciprocals in FP32, OpDiffusion would take 23 us but round twice.
+// the slopes).
 struct OpViscSlopes {
   static constexpr const char* kName = "visc_slopes";
   template <class T>
@@ -1546,6 +1540,13 @@ struct OpViscSlopes {
     S.vsx[o] = cx; S.vsy[o] = cy; S.vlx[o] = lx; S.vly[o] = ly;
   }
 };
+// diffusion (src/nhwave.F:6785-7141): the explicit viscous terms of R2-R4,
+// one thread per interior cell, from the stage's starting DU/DV/DW and the
+// sigma slopes of the last sigma_transform (zero before the first one).
+// Cmu = Visc; CmuHt per cell (Cmut_min until eval_turb).  Each bracket
+// keeps the reference's evaluation order (bit-exact in the FP64 form), and its
+// quotients are divisions in both forms: multiplied by reciprocals in FP32 it
+// would take 23 us of 60 (515 x 30 x 15) but round twice.
 struct OpDiffusion {
   static constexpr const char* kName = "diffusion";
   template <class T>
@@ -3223,11 +3224,10 @@ struct OpProjection {
   }
 };
 // The same in the FP32+IR form: the pressure differences in FP64 (P is FP64),
-// each rounded once, and the rest in FP32
-// The same in the FP32+IR form, a thread walking kc levels of a column: the
-// column's factors are rounded to FP32 once, a level's horizontal pressure
-// differences serve the level below and above, 3 FP64 differences a cell
-// instead of 5, 7 conversions less (768 x 768 x 20: 398 -> @J us).
+// each rounded once, and the rest in FP32.  A thread walks kc levels of a
+// column: the column's factors are rounded to FP32 once, a level's horizontal
+// pressure differences serve the level below and above, 3 FP64 differences a
+// cell instead of 5, 7 conversions less (768 x 768 x 20: 398 -> 212 us).
 template <class T>
 __global__ void __launch_bounds__(128) k_projection32(Dev<T> S, int kc) {
   if (gated_off(S)) return;
@@ -3262,6 +3262,7 @@ __global__ void __launch_bounds__(128) k_projection32(Dev<T> S, int kc) {
   }
 }
 
+// SSP-RK combination, mask and Froude cap (src/nhwave.F:1227-1261)
 struct OpSSP {
   static constexpr const char* kName = "ssp_combine";
   int istep;

@@ -1967,7 +1967,9 @@ class Solver final : public SolverBase {
     prof_on = on != 0;
     return NHW_OK;
   }
-  // Device time of one level-0 half-sweep, the largest kernel of a step.
+  // Device time of one level-0 half-sweep, the largest kernel of a step on
+  // grids whose level 0 does not take the tiles; on those that it does
+  // (tiled()), the half-sweeps timed here are GMRES' and not BiCGSTAB's.
   // Events around single launches add several microseconds to each, so the
   // launches are timed in bulk: a CUDA graph of `reps` rounds, each a write
   // of `flush` bytes (evicting the L2) and then the four level-0 half-sweeps
