@@ -133,6 +133,28 @@ __device__ __forceinline__ double operator/(double a, const Quot<T>& q) {
   else return a / q.b;
 }
 
+// The same for divisors in the working precision R of a cell kernel.  FP32: the
+// reciprocal in two words, the quotient one product and one fused addition --
+// rounded once, but for 2^-23 of an ulp or so (Brisebarre, Muller and Raina,
+// "Accelerating correctly rounded floating-point division when the divisor is
+// known in advance", IEEE Trans. Comput. 53(8), 2004).
+template <class R>
+struct QuotR {
+  R b, hi, lo;
+};
+template <class R>
+__device__ __forceinline__ QuotR<R> over_r(R b) {
+  if constexpr (sizeof(R) == 4) {
+    const R hi = (R)1 / b;
+    return QuotR<R>{b, hi, hi * fmaf(-b, hi, (R)1)};
+  } else return QuotR<R>{b, (R)0, (R)0};
+}
+template <class R>
+__device__ __forceinline__ R operator/(R a, const QuotR<R>& q) {
+  if constexpr (sizeof(R) == 4) return fmaf(a, q.hi, a * q.lo);
+  else return a / q.b;
+}
+
 __device__ __forceinline__ int mirror(int i, int b, int e) {
   return i < b ? 2 * b - 1 - i : (i > e ? 2 * e + 1 - i : i);
 }
@@ -1519,7 +1541,7 @@ struct OpVelBcB {
 // DelxSc / DelySc and DelxSl / DelySl of the last sigma_transform (zero
 // before the first one), which OpDiffusion reads: formed once a column and
 // level, since each of that stencil's 30 uses costs two FP64 divisions
-// (515 x 30 x 15 FP32+IR: diffusion 677 us with the slopes in place, 60 + 19 for
+// (515 x 30 x 15 FP32+IR: diffusion 677 us with the slopes in place, 24 + 19 for
 // the slopes).
 struct OpViscSlopes {
   static constexpr const char* kName = "visc_slopes";
@@ -1544,9 +1566,9 @@ struct OpViscSlopes {
 // one thread per interior cell, from the stage's starting DU/DV/DW and the
 // sigma slopes of the last sigma_transform (zero before the first one).
 // Cmu = Visc; CmuHt per cell (Cmut_min until eval_turb).  Each bracket
-// keeps the reference's evaluation order (bit-exact in the FP64 form), and its
-// quotients are divisions in both forms: multiplied by reciprocals in FP32 it
-// would take 23 us of 60 (515 x 30 x 15) but round twice.
+// keeps the reference's evaluation order (bit-exact in the FP64 form); its
+// some 90 quotients a cell have eight divisors (FP32, 515 x 30 x 15: 60 us
+// divided, 24 us by QuotR).
 struct OpDiffusion {
   static constexpr const char* kName = "diffusion";
   template <class T>
@@ -1563,8 +1585,9 @@ struct OpDiffusion {
     const T* DV = S.DV;
     const T* DW = S.DW;
     auto F = [&](const T* a, int ii, int jj, int kk) -> R { return a[i3(S, ii, jj, kk)]; };
-    const R dx = (R)S.dx, dy = (R)S.dy;
-    const R cmu = (R)S.v_cmu, sch = (R)S.v_schmidt;
+    const QuotR<R> dx = over_r<R>((R)S.dx), dy = over_r<R>((R)S.dy);
+    const R cmu = (R)S.v_cmu;
+    const QuotR<R> sch = over_r<R>((R)S.v_schmidt);
     // CmuHt of a cell; face viscosity between two cells; cell viscosity
     auto H = [&](int ii, int jj, int kk) -> R { return (R)S.CmuHt[i3(S, ii, jj, kk)]; };
     auto nuF = [&](R ha, R hb) -> R { return (R)0.5 * (cmu + cmu) + (R)0.5 * (ha + hb) / sch; };
@@ -1577,10 +1600,11 @@ struct OpDiffusion {
     auto lv = [&](int n) { return S.lvv[n * S.Kloc + k]; };
     const double L1top = lv(kLvL1t), L2top = lv(kLvL2t), L1bot = lv(kLvL1b), L2bot = lv(kLvL2b);
     const R rck = (R)lv(kLvCk), rck1 = (R)lv(kLvCk1);
+    const QuotR<R> qck = over_r<R>(rck), qck1 = over_r<R>(rck1), qcc = over_r<R>(rck + rck1);
     const R ac = (R)lv(kLvAc), bc = (R)lv(kLvBc), gc = (R)lv(kLvGc);
     const R nuH_top = ((R)L1top * cmu + (R)L2top * cmu) + ((R)L1top * h0 + (R)L2top * H(i, j, k + 1)) / sch;
     const R nuH_bot = ((R)L1bot * cmu + (R)L2bot * cmu) + ((R)L1bot * H(i, j, k - 1) + (R)L2bot * h0) / sch;
-    const R Dc = (R)S.D[c], dsk = (R)S.dsig[k];
+    const QuotR<R> Dc = over_r<R>((R)S.D[c]), dsk = over_r<R>((R)S.dsig[k]);
     auto s3 = [&](const T* a, bool y, int ii, int jj) -> R {   // a F(k-1) Sc(k-1) + b .. + c ..
       auto sc = [&](int kk) { return y ? Scy(ii, jj, kk) : Scx(ii, jj, kk); };
       return ac * F(a, ii, jj, k - 1) * sc(k - 1) + bc * F(a, ii, jj, k) * sc(k) + gc * F(a, ii, jj, k + 1) * sc(k + 1);
@@ -1600,9 +1624,9 @@ struct OpDiffusion {
       const T* sl = y ? S.vly : S.vlx;
       const R st = sl[o + S.sz], sb = sl[o];
       const R Pq = nuH_top * st - nuH_bot * sb, Sq = nuH_top * st + nuH_bot * sb;
-      cA = Pq * ac / dsk + Sq / rck1 / (rck + rck1);
-      cB = Pq * bc / dsk - Sq / rck1 / rck;
-      cC = Pq * gc / dsk + Sq / rck / (rck + rck1);
+      cA = Pq * ac / dsk + Sq / qck1 / qcc;
+      cB = Pq * bc / dsk - Sq / qck1 / qck;
+      cC = Pq * gc / dsk + Sq / qck / qcc;
     };
     R xA, xB, xC, yA, yB, yC;
     vco(false, xA, xB, xC);

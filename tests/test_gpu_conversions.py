@@ -1,10 +1,14 @@
-"""GPU: the integer conversions between float and double against the hardware's.
+"""GPU: the arithmetic that replaces slower instructions, against those.
 
 ``widen`` and ``narrow`` (kernels.cuh) carry every FP32+IR step.  ``widen`` is
 compared over all floats.  ``narrow`` is compared over doubles of every
 exponent with the bit patterns at which rounding decides: zeros, halfway and
 one to either side of it, carries into the next exponent, both ends of the
 normal and subnormal floats, infinities and NaN, and over pseudo-random ones.
+
+``a / over_r(b)`` must be the quotient rounded once: half an ulp, and 2^-21 of
+one for the low word's two roundings (2^-24 of it each, and it is at most 2^-24
+of the quotient).
 """
 import ctypes
 import os
@@ -50,12 +54,26 @@ __global__ void k_narrow(unsigned long long* bad, int mode, unsigned long long n
     if (!same(narrow<float>(x), (float)x)) atomicAdd(bad, 1ull);
   }
 }
+// quotients of hashed operands from 2^-20 to 2^20, by divisors of the same range
+__global__ void k_quot(unsigned long long* bad, unsigned long long n) {
+  for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < n; i += gridDim.x * 256ull) {
+    unsigned long long h = 0x9e3779b97f4a7c15ull * (i + 1);
+    h ^= h >> 30; h *= 0xbf58476d1ce4e5b9ull; h ^= h >> 27; h *= 0x94d049bb133111ebull; h ^= h >> 31;
+    const unsigned e0 = 107 + (unsigned)(h >> 58) % 41, e1 = 107 + (unsigned)(h >> 52) % 41;
+    const float a = __uint_as_float(((unsigned)h & 0x807fffffu) | e0 << 23);
+    const float b = __uint_as_float(((unsigned)(h >> 24) & 0x7fffffu) | e1 << 23);
+    const double exact = (double)a / (double)b, q = (double)(a / over_r<float>(b));
+    const double ulp = ldexp(1.0, ilogb(exact) - 23);
+    if (!(fabs(q - exact) <= (0.5 + 0x1p-21) * ulp)) atomicAdd(bad, 1ull);
+  }
+}
 extern "C" long long mismatches(int what) {
   unsigned long long* bad = nullptr;
   unsigned long long h = ~0ull;
   if (cudaMalloc((void**)&bad, 8) != cudaSuccess || cudaMemset(bad, 0, 8) != cudaSuccess) return -1;
   if (what == 0) k_widen<<<152 * 8, 256>>>(bad);
-  else k_narrow<<<152 * 8, 256>>>(bad, what - 1, 1ull << 32);
+  else if (what < 3) k_narrow<<<152 * 8, 256>>>(bad, what - 1, 1ull << 32);
+  else k_quot<<<152 * 8, 256>>>(bad, 1ull << 28);
   if (cudaMemcpy(&h, bad, 8, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
   cudaFree(bad);
   return (long long)h;
@@ -77,6 +95,6 @@ def checker(tmp_path_factory):
     return lib
 
 
-@pytest.mark.parametrize("what", [0, 1, 2], ids=["widen_all", "narrow_edges", "narrow_random"])
+@pytest.mark.parametrize("what", [0, 1, 2, 3], ids=["widen_all", "narrow_edges", "narrow_random", "quotients"])
 def test_conversions_equal_the_instructions(what, checker):
     assert checker.mismatches(what) == 0
