@@ -203,7 +203,7 @@ struct TileB {
   __device__ __forceinline__ T operator()(int ic) const { return b[ic]; }
   __device__ __forceinline__ void put(int, T) const {}
 };
-// p = r + beta q, q = p - omega v of the last iteration (k_bicg_xr): p itself
+// p = r + beta q, q = p - omega v of the last iteration (k_bicg_xr_sl): p itself
 // cannot be both read by the neighbouring tiles and updated in place
 template <class T>
 struct TileInP {

@@ -82,7 +82,7 @@ extern "C" long long mismatches(int what) {
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def compiled(tmp_path_factory):
     from nhwave_gb300 import build
     d = tmp_path_factory.mktemp("conv")
     src, so = d / "conv.cu", d / "libconv.so"
@@ -96,5 +96,5 @@ def checker(tmp_path_factory):
 
 
 @pytest.mark.parametrize("what", [0, 1, 2, 3], ids=["widen_all", "narrow_edges", "narrow_random", "quotients"])
-def test_conversions_equal_the_instructions(what, checker):
-    assert checker.mismatches(what) == 0
+def test_conversions_equal_the_instructions(what, compiled):
+    assert compiled.mismatches(what) == 0
